@@ -1,5 +1,6 @@
 // Internal declarations shared by the host library (sb_api.cpp) and the CUDA kernels.
 #pragma once
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -129,6 +130,10 @@ cudaError_t launch_asb_local(float *x, float *y, int n, int R, int xp, float amp
                              float mts_dt, float detune, float kerr, cudaStream_t st);
 // Copy a dense host-layout J [n][n] (already on the device) into the padded [n][jp] FP32 layout.
 cudaError_t launch_pad_rows_f32(const float *src, float *dst, int n, int jp, cudaStream_t st);
+
+// Tensor map of a row-major FP32 matrix (rows x cols, pitch floats between rows; base and pitch
+// multiples of 16 bytes) read in unswizzled boxes of box_rows x box_cols, zero beyond its edges.
+bool encode_rows_f32(CUtensorMap *m, const float *base, int rows, int cols, int pitch, int box_cols, int box_rows);
 
 // ---------------------------------------------------------------------------------------------
 // Tensor-core (tcgen05) path. See sb_tc.cu.

@@ -328,6 +328,216 @@ __global__ void __launch_bounds__(kThreads) plain_step_kernel(PlainStep a) {
   }
 }
 
+// ---- many replicas: register tiles ----
+// With three or more replicas per row block the row-per-warp layout above is bound by shared-memory
+// loads of the replica vectors (one 16-byte load per 4 FMAs and replica). Here a warp keeps an 8-row x
+// 8-replica tile of partial sums: lane l sums the float4 groups g = l (mod 32) of K in increasing
+// order for all 64 pairs, 16 16-byte loads per 256 FMAs, and the 32 partials of a pair are then added in
+// the same butterfly order (16, 8, 4, 2, 1), each round halving the pairs a lane keeps, so a lane ends
+// with two finished fields and the bits equal the row-per-warp layout's. A CTA's 8 warps (4 row groups
+// x 2 replica groups) share 32 J rows and 16 replica rows, staged 128 floats of K at a time by 2-D TMA
+// (zero-filled past n and R) through a ring of four 24 KB stages; two CTAs share an SM. Staging the same
+// tiles with per-thread cp.async cost as many issue slots as half the FMAs.
+constexpr int kTileRows = 32, kTileReps = 16, kTileK = 128, kTileStages = 4;
+constexpr int kTileStageFloats = (kTileRows + kTileReps) * kTileK;
+constexpr size_t kTileSmem = (size_t)kTileStages * kTileStageFloats * sizeof(float);
+// A tile launch's arguments: the step's own and the tensor maps of J [n][jp] and of the replica
+// vectors [R][jp of pitch xp].
+template <typename Args>
+struct Tiled {
+  Args a;
+  CUtensorMap mj, mx;
+};
+
+// Fields of the warp's tile: on return f[0], f[1] are those of row row0 + 8 (warp & 3) + (lane >> 2) and
+// replicas r0 + 8 (warp >> 2) + 2 (lane & 3) + {0, 1}. Returns false (the whole CTA) when a bounded wait
+// gave up. J must not be written by the previous kernel of the stream: its first stages are requested
+// before grid_dep_wait.
+template <bool SIGN>
+__device__ __forceinline__ bool tile_field(const CUtensorMap *mj, const CUtensorMap *mx, int jp, int row0, int r0,
+                                           float *smem, float (&f)[2]) {
+  __shared__ __align__(8) uint64_t full[kTileStages], empty[kTileStages];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int nchunks = (jp + kTileK - 1) / kTileK;
+  auto issue_j = [&](int c) {
+    const int s = c % kTileStages;
+    ptx::mbar_arrive_expect_tx(&full[s], kTileStageFloats * 4u);  // boxes count their zero fill too
+    ptx::tma_load_2d(smem + s * kTileStageFloats, mj, c * kTileK, row0, &full[s]);
+  };
+  auto issue_x = [&](int c) {
+    const int s = c % kTileStages;
+    ptx::tma_load_2d(smem + s * kTileStageFloats + kTileRows * kTileK, mx, c * kTileK, r0, &full[s]);
+  };
+  const int pre = min(nchunks, kTileStages);
+  int issued = pre;  // chunks requested (thread 0)
+  if (tid == 0) {
+    for (int s = 0; s < kTileStages; ++s) {
+      ptx::mbar_init(&full[s], 1);
+      ptx::mbar_init(&empty[s], kThreads / 32);
+    }
+    ptx::fence_mbar_init();
+    for (int c = 0; c < pre; ++c) issue_j(c);
+  }
+  __syncthreads();
+  ptx::grid_dep_wait();
+  ptx::grid_dep_launch();
+  if (tid == 0) {
+    ptx::fence_proxy_async_global();  // the previous kernel's x, then the copies of it
+    for (int c = 0; c < pre; ++c) issue_x(c);
+  }
+  bool ok = true;
+  float acc[8][8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int r = 0; r < 8; ++r) acc[i][r] = 0.0f;
+  for (int c = 0; c < nchunks; ++c) {
+    const int s = c % kTileStages;
+    // refill the stage of chunk c - 2: every warp has had an iteration to leave it
+    const int cf = c + kTileStages - 2;
+    if (tid == 0 && c >= 2 && cf < nchunks) {
+      if (ptx::mbar_wait(&empty[cf % kTileStages], (uint32_t)((cf / kTileStages - 1) & 1))) {
+        issue_j(cf);
+        issue_x(cf);
+        issued = cf + 1;
+      }
+    }
+    if (!__all_sync(0xffffffffu, ptx::mbar_wait(&full[s], (uint32_t)((c / kTileStages) & 1)))) {
+      ok = false;
+      break;
+    }
+    const float4 *st = reinterpret_cast<const float4 *>(smem + s * kTileStageFloats);
+    const float4 *js = st + (warp & 3) * 8 * 32 + lane;
+    const float4 *xs = st + (kTileRows + (warp >> 2) * 8) * 32 + lane;
+    float4 jv[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) jv[i] = js[i * 32];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      float4 v = xs[r * 32];
+      if (SIGN) {
+        v.x = sgn(v.x);
+        v.y = sgn(v.y);
+        v.z = sgn(v.z);
+        v.w = sgn(v.w);
+      }
+      // the four products of a pair are one dependent chain: eight pairs in turn hide its latency
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[i][r] = __fmaf_rn(jv[i].x, v.x, acc[i][r]);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[i][r] = __fmaf_rn(jv[i].y, v.y, acc[i][r]);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[i][r] = __fmaf_rn(jv[i].z, v.z, acc[i][r]);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[i][r] = __fmaf_rn(jv[i].w, v.w, acc[i][r]);
+    }
+    __syncwarp();
+    if (lane == 0) ptx::mbar_arrive(&empty[s]);
+  }
+  if (!__syncthreads_and(ok ? 1 : 0)) {
+    // the copies requested last into each stage land before the CTA's shared memory goes away
+    if (tid == 0)
+      for (int c = max(0, issued - kTileStages); c < issued; ++c)
+        ptx::mbar_wait(&full[c % kTileStages], (uint32_t)((c / kTileStages) & 1));
+    return false;
+  }
+  // butterfly over the lanes' partials; pair p = 8 i + r: a lane keeps the half of its pairs that its
+  // bit of the round selects and receives the partner's sums of them
+  float v32[32], v16[16], v8[8], v4[4];
+  const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4, b1 = lane & 2, b0 = lane & 1;
+#pragma unroll
+  for (int p = 0; p < 32; ++p) {
+    const float lo = acc[p >> 3][p & 7], hi = acc[4 + (p >> 3)][p & 7];
+    v32[p] = (b4 ? hi : lo) + __shfl_xor_sync(0xffffffffu, b4 ? lo : hi, 16);
+  }
+#pragma unroll
+  for (int p = 0; p < 16; ++p) v16[p] = (b3 ? v32[16 + p] : v32[p]) + __shfl_xor_sync(0xffffffffu, b3 ? v32[p] : v32[16 + p], 8);
+#pragma unroll
+  for (int p = 0; p < 8; ++p) v8[p] = (b2 ? v16[8 + p] : v16[p]) + __shfl_xor_sync(0xffffffffu, b2 ? v16[p] : v16[8 + p], 4);
+#pragma unroll
+  for (int p = 0; p < 4; ++p) v4[p] = (b1 ? v8[4 + p] : v8[p]) + __shfl_xor_sync(0xffffffffu, b1 ? v8[p] : v8[4 + p], 2);
+#pragma unroll
+  for (int p = 0; p < 2; ++p) f[p] = (b0 ? v4[2 + p] : v4[p]) + __shfl_xor_sync(0xffffffffu, b0 ? v4[p] : v4[2 + p], 1);
+  return true;
+}
+
+template <int VARIANT>
+__global__ void __launch_bounds__(kThreads, 2) plain_tile_kernel(const __grid_constant__ Tiled<PlainStep> g) {
+  const PlainStep &a = g.a;
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ double red[kTileRows][kTileReps];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int row0 = blockIdx.x * kTileRows, r0 = blockIdx.y * kTileReps;
+  float f[2];
+  if (!tile_field<VARIANT == 2>(&g.mj, &g.mx, a.jp, row0, r0, reinterpret_cast<float *>(smem), f)) {
+    if (tid == 0) atomicOr(a.status, kErrWaitTimeout);
+    return;
+  }
+  const int w = 8 * (warp & 3) + (lane >> 2), i = row0 + w;
+#pragma unroll
+  for (int p = 0; p < 2; ++p) {
+    const int c = 8 * (warp >> 2) + 2 * (lane & 3) + p, r = r0 + c;
+    double e = 0.0;
+    if (i < a.n && r < a.R) {
+      const size_t k = (size_t)r * a.xp + i;
+      float x = a.x_in[k], y = a.y[k];
+      const float hv = a.h ? a.h[i] : 0.0f;
+      if (VARIANT == 0) {
+        y = __fmaf_rn(a.coeff, f[p], y);
+        if (a.do_local) asb_local(x, y, a.amp_next, a.m, a.mts_dt, a.detune, a.kerr);
+      } else {
+        const float s = sgn(x);
+        if (VARIANT == 2) e = -0.5 * (double)s * (double)f[p] - (double)hv * (double)s;
+        sb_update(f[p], hv, a.pump, a.c0, a.dt, a.dta0, x, y);
+      }
+      if (SB_BOUNDS(k < (size_t)a.R * a.xp, a.status)) {
+        a.x_out[k] = x;
+        a.y[k] = y;
+      }
+    }
+    if (VARIANT == 2 && a.energy) red[w][c] = e;
+  }
+  if (VARIANT == 2 && a.energy) {
+    __syncthreads();
+    if (tid < kTileReps && r0 + tid < a.R) {
+      double e = 0.0;
+      for (int q = 0; q < kTileRows; ++q) e += red[q][tid];
+      atomicAdd(a.energy + r0 + tid, e);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kThreads, 2) plain_tile_energy_kernel(const __grid_constant__ Tiled<PlainEnergy> g) {
+  const PlainEnergy &a = g.a;
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ double red[kTileRows][kTileReps];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int row0 = blockIdx.x * kTileRows, r0 = blockIdx.y * kTileReps;
+  float f[2];
+  if (!tile_field<true>(&g.mj, &g.mx, a.jp, row0, r0, reinterpret_cast<float *>(smem), f)) {
+    if (tid == 0) atomicOr(a.status, kErrWaitTimeout);
+    return;
+  }
+  const int w = 8 * (warp & 3) + (lane >> 2), i = row0 + w;
+#pragma unroll
+  for (int p = 0; p < 2; ++p) {
+    const int c = 8 * (warp >> 2) + 2 * (lane & 3) + p, r = r0 + c;
+    double e = 0.0;
+    if (i < a.n && r < a.R) {
+      const double s = sgn(a.x[(size_t)r * a.xp + i]);
+      const double hv = a.h ? (double)a.h[i] : 0.0;
+      e = -0.5 * s * (double)f[p] - hv * s;
+    }
+    red[w][c] = e;
+  }
+  __syncthreads();
+  if (tid < kTileReps && r0 + tid < a.R) {
+    double e = 0.0;
+    for (int q = 0; q < kTileRows; ++q) e += red[q][tid];
+    atomicAdd(a.energy + r0 + tid, e);
+  }
+}
+
 template <typename Acc, bool WIDE>
 __global__ void __launch_bounds__(kThreads) plain_energy_kernel(PlainEnergy a) {
   extern __shared__ __align__(128) unsigned char smem[];
@@ -383,6 +593,29 @@ __global__ void __launch_bounds__(kThreads) plain_energy_kernel(PlainEnergy a) {
 // sweep (the reference's sweeps inside a stage have no barrier between one warp's writes and
 // another's reads; for up to 32 spins, one warp, it computes exactly this).
 
+// The NMFA update of (sample r, spin i) from its field; draws the stage's pair on its first sweep.
+__device__ __forceinline__ void nmfa_element(const NmfaSweep &a, int i, int r, float f) {
+  const size_t k = (size_t)r * a.xp + i;
+  const size_t plane = (size_t)a.R * a.xp;
+  if (i >= a.n || r >= a.R || !SB_BOUNDS(k < plane, a.status)) return;
+  float z;
+  if (a.first) {
+    uint32_t wd[5];
+#pragma unroll
+    for (int q = 0; q < 5; ++q) wd[q] = a.rng[q * plane + k];
+    float z1;
+    sbm::nmfa_gauss(wd, a.noise, z, z1);
+#pragma unroll
+    for (int q = 0; q < 5; ++q) a.rng[q * plane + k] = wd[q];
+    a.z1[k] = z1;
+  } else {
+    z = a.z1[k];
+  }
+  const float st = sbm::nmfa_update(f, a.norm[i], z, a.beta, a.keep, a.mix, a.s_in[k]);
+  a.s_out[k] = st;
+  if (a.samples) a.samples[(size_t)r * a.n + i] = st > 0.0f ? 1 : -1;
+}
+
 template <bool WIDE>
 __global__ void __launch_bounds__(kThreads) nmfa_sweep_kernel(NmfaSweep a) {
   extern __shared__ __align__(128) unsigned char smem[];
@@ -418,28 +651,22 @@ __global__ void __launch_bounds__(kThreads) nmfa_sweep_kernel(NmfaSweep a) {
   }
   __syncthreads();
   const int w = tid % kRows, rr = tid / kRows;
-  if (rr < rb && w < rows) {
-    const int i = row0 + w, r = r0 + rr;
-    const size_t k = (size_t)r * a.xp + i;
-    const size_t plane = (size_t)a.R * a.xp;
-    if (!SB_BOUNDS(k < plane && i < a.n, a.status)) return;
-    float z;
-    if (a.first) {
-      uint32_t wd[5];
-#pragma unroll
-      for (int q = 0; q < 5; ++q) wd[q] = a.rng[q * plane + k];
-      float z1;
-      sbm::nmfa_gauss(wd, a.noise, z, z1);
-#pragma unroll
-      for (int q = 0; q < 5; ++q) a.rng[q * plane + k] = wd[q];
-      a.z1[k] = z1;
-    } else {
-      z = a.z1[k];
-    }
-    const float st = sbm::nmfa_update(fsh[w][rr], a.norm[i], z, a.beta, a.keep, a.mix, a.s_in[k]);
-    a.s_out[k] = st;
-    if (a.samples) a.samples[(size_t)r * a.n + i] = st > 0.0f ? 1 : -1;
+  if (rr < rb && w < rows) nmfa_element(a, row0 + w, r0 + rr, fsh[w][rr]);
+}
+
+__global__ void __launch_bounds__(kThreads, 2) nmfa_tile_kernel(const __grid_constant__ Tiled<NmfaSweep> g) {
+  const NmfaSweep &a = g.a;
+  extern __shared__ __align__(128) unsigned char smem[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int row0 = blockIdx.x * kTileRows, r0 = blockIdx.y * kTileReps;
+  float f[2];
+  if (!tile_field<false>(&g.mj, &g.mx, a.jp, row0, r0, reinterpret_cast<float *>(smem), f)) {
+    if (threadIdx.x == 0) atomicOr(a.status, kErrWaitTimeout);
+    return;
   }
+  const int i = row0 + 8 * (warp & 3) + (lane >> 2);
+#pragma unroll
+  for (int p = 0; p < 2; ++p) nmfa_element(a, i, r0 + 8 * (warp >> 2) + 2 * (lane & 3) + p, f[p]);
 }
 
 // norm[i] = -1 / sqrt(sum_j |J_ij|) (nmfa.cu:88-93) with the sum in double over j in index order and
@@ -810,17 +1037,22 @@ void set_smem_once(K kernel, size_t bytes) {
 struct PlainAttrInit {
   PlainAttrInit() {
     set_smem_once(plain_step_kernel<0, false>, kSmemBytes);
-    set_smem_once(plain_step_kernel<1, false>, kSmemBytes);
-    set_smem_once(plain_step_kernel<2, false>, kSmemBytes);
     set_smem_once(plain_step_kernel<0, true>, kWideSmem);
+    set_smem_once(plain_tile_kernel<0>, kTileSmem);
+    set_smem_once(plain_step_kernel<1, false>, kSmemBytes);
     set_smem_once(plain_step_kernel<1, true>, kWideSmem);
+    set_smem_once(plain_tile_kernel<1>, kTileSmem);
+    set_smem_once(plain_step_kernel<2, false>, kSmemBytes);
     set_smem_once(plain_step_kernel<2, true>, kWideSmem);
+    set_smem_once(plain_tile_kernel<2>, kTileSmem);
     set_smem_once(plain_energy_kernel<float, false>, kSmemBytes);
     set_smem_once(plain_energy_kernel<double, false>, kSmemBytes);
     set_smem_once(plain_energy_kernel<float, true>, kWideSmem);
+    set_smem_once(plain_tile_energy_kernel, kTileSmem);
     set_smem_once(plain_energy_kernel<double, true>, kWideSmem);
     set_smem_once(nmfa_sweep_kernel<false>, kSmemBytes);
     set_smem_once(nmfa_sweep_kernel<true>, kWideSmem);
+    set_smem_once(nmfa_tile_kernel, kTileSmem);
   }
 };
 
@@ -842,11 +1074,39 @@ int plain_stages(int jp, int rb) {
   return s < nchunks ? s : nchunks;
 }
 
-template <int V, bool WIDE>
-cudaError_t launch_step_variant(const PlainStep &a, dim3 grid, cudaStream_t st) {
+// The register-tile launch of `kernel` over n rows of J and R replica vectors x.
+// overlap: it may start during the previous kernel's tail (programmatic serialization).
+template <typename Args>
+cudaError_t launch_tiles(void (*kernel)(Tiled<Args>), const Args &a, const float *x, bool overlap, cudaStream_t st) {
+  Tiled<Args> t;
+  t.a = a;
+  if (!encode_rows_f32(&t.mj, a.J, a.n, a.jp, a.jp, kTileK, kTileRows) ||
+      !encode_rows_f32(&t.mx, x, a.R, a.jp, a.xp, kTileK, kTileReps))
+    return cudaErrorInvalidValue;
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = grid;
+  cfg.gridDim = dim3((unsigned)((a.n + kTileRows - 1) / kTileRows), (unsigned)((a.R + kTileReps - 1) / kTileReps));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = kTileSmem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = overlap ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, t);
+}
+
+// The row-per-warp layouts: `ring` for at most two replicas per CTA, else `wide` (which does not wait
+// in grid_dep_wait and so never overlaps the previous kernel).
+template <typename Args>
+cudaError_t launch_row_warps(void (*ring)(Args), void (*wide)(Args), const Args &a0, cudaStream_t st) {
+  Args a = a0;
+  const bool w = a.rb > 2;
+  a.stages = plain_stages(a.jp, a.rb);
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3((unsigned)((a.n + kRows - 1) / kRows), (unsigned)((a.R + a.rb - 1) / a.rb));
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = plain_smem(a.rb, a.stages);
   cfg.stream = st;
@@ -854,28 +1114,34 @@ cudaError_t launch_step_variant(const PlainStep &a, dim3 grid, cudaStream_t st) 
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = (a.overlap && !WIDE) ? 1 : 0;  // only the ring layout waits in grid_dep_wait
-  return cudaLaunchKernelEx(&cfg, plain_step_kernel<V, WIDE>, a);
+  cfg.numAttrs = (a.overlap && !w) ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, w ? wide : ring, a);
 }
+
+// Which shapes take the register tiles. A tile CTA covers 32 rows x 16 replicas whatever R is, so with
+// few replicas or rows it leaves SMs idle and lanes on padding. Measured, us per dSB step, row-per-warp
+// against tiles: n = 300 R = 6 4.9 / 5.2, R = 8 5.4 / 5.2; n = 1000 R = 6 7.8 / 7.9, R = 8 8.8 / 7.9;
+// n = 2048 R = 5 12.8 / 13.7, R = 8 15.5 / 13.6, R = 100 94 / 32; n = 4000 R = 3 25.0 / 26.2, R = 5
+// 29.9 / 26.0, R = 100 365 / 118.
+bool use_tiles(int n, int R) { return R >= 8 || (n >= 3000 && R >= 4); }
 
 cudaError_t launch_plain_step(const PlainStep &a0, cudaStream_t st) {
   plain_attrs();
   if (a0.rb < 1 || a0.rb > kMaxRB || a0.jp % 4 || a0.xp % 4 || a0.jp > a0.xp || a0.jp < 4)
     return cudaErrorInvalidValue;
-  PlainStep a = a0;
-  a.stages = plain_stages(a.jp, a.rb);
-  dim3 grid((a.n + kRows - 1) / kRows, (a.R + a.rb - 1) / a.rb);
-  const bool wide = a.rb > 2;
-  switch (a.variant) {
+  const bool tile = use_tiles(a0.n, a0.R), ov = a0.overlap != 0;
+  switch (a0.variant) {
     case 0:
-      return wide ? launch_step_variant<0, true>(a, grid, st) : launch_step_variant<0, false>(a, grid, st);
+      return tile ? launch_tiles(plain_tile_kernel<0>, a0, a0.x_in, ov, st)
+                  : launch_row_warps(plain_step_kernel<0, false>, plain_step_kernel<0, true>, a0, st);
     case 1:
-      return wide ? launch_step_variant<1, true>(a, grid, st) : launch_step_variant<1, false>(a, grid, st);
+      return tile ? launch_tiles(plain_tile_kernel<1>, a0, a0.x_in, ov, st)
+                  : launch_row_warps(plain_step_kernel<1, false>, plain_step_kernel<1, true>, a0, st);
     case 2:
-      return wide ? launch_step_variant<2, true>(a, grid, st) : launch_step_variant<2, false>(a, grid, st);
-    default:
-      return cudaErrorInvalidValue;
+      return tile ? launch_tiles(plain_tile_kernel<2>, a0, a0.x_in, ov, st)
+                  : launch_row_warps(plain_step_kernel<2, false>, plain_step_kernel<2, true>, a0, st);
   }
+  return cudaErrorInvalidValue;
 }
 
 int plain_persist_ctas(int n, int R, int jp) {
@@ -923,6 +1189,7 @@ cudaError_t launch_plain_energy(const PlainEnergy &a0, bool fp64, cudaStream_t s
   plain_attrs();
   if (a0.rb < 1 || a0.rb > kMaxRB || a0.jp % 4 || a0.xp % 4 || a0.jp > a0.xp || a0.jp < 4)
     return cudaErrorInvalidValue;
+  if (!fp64 && use_tiles(a0.n, a0.R)) return launch_tiles(plain_tile_energy_kernel, a0, a0.x, false, st);
   PlainEnergy a = a0;
   a.stages = plain_stages(a.jp, a.rb);
   dim3 grid((a.n + kRows - 1) / kRows, (a.R + a.rb - 1) / a.rb);
@@ -945,22 +1212,8 @@ cudaError_t launch_nmfa_sweep(const NmfaSweep &a0, cudaStream_t st) {
   plain_attrs();
   if (a0.rb < 1 || a0.rb > kMaxRB || a0.jp % 4 || a0.xp % 4 || a0.jp > a0.xp || a0.jp < 4)
     return cudaErrorInvalidValue;
-  NmfaSweep a = a0;
-  a.stages = plain_stages(a.jp, a.rb);
-  const bool wide = a.rb > 2;
-  cudaLaunchConfig_t cfg;
-  memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3((a.n + kRows - 1) / kRows, (a.R + a.rb - 1) / a.rb);
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = plain_smem(a.rb, a.stages);
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = (a.overlap && !wide) ? 1 : 0;
-  return wide ? cudaLaunchKernelEx(&cfg, nmfa_sweep_kernel<true>, a)
-              : cudaLaunchKernelEx(&cfg, nmfa_sweep_kernel<false>, a);
+  return use_tiles(a0.n, a0.R) ? launch_tiles(nmfa_tile_kernel, a0, a0.s_in, a0.overlap != 0, st)
+                               : launch_row_warps(nmfa_sweep_kernel<false>, nmfa_sweep_kernel<true>, a0, st);
 }
 
 cudaError_t launch_nmfa_norms(const float *J, int n, int jp, float *norm, bool integral, cudaStream_t st) {
