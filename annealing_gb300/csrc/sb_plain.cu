@@ -14,7 +14,7 @@
 //     before it touches x;
 //   * each warp forms its row's dot products with float4 shared-memory reads and a shuffle
 //     reduction; the fields then go through shared memory to consecutive threads, which apply the
-//     SB update (the aSB sub-steps in FP64 on one or two warps per CTA) and write x (ping-pong)
+//     SB update (the aSB sub-steps on one or two warps per CTA, sb_asb.cuh) and write x (ping-pong)
 //     and y (in place: every element has exactly one owner);
 //   * dSB also reduces -1/2 s_i f_i - h_i s_i per replica (block reduction + one atomic per
 //     replica), which is the energy of s(t) and costs nothing extra because f = J s(t).
@@ -23,6 +23,7 @@
 #include <stdint.h>
 #include <string.h>
 
+#include "sb_asb.cuh"
 #include "sb_internal.h"
 #include "sb_math.cuh"
 #include "sb_ptx.cuh"
@@ -55,20 +56,6 @@ __device__ __forceinline__ void sb_update(float f, float hv, float pump, float c
   if (fabsf(x) > 1.0f) {
     x = copysignf(1.0f, x);
     y = 0.0f;
-  }
-}
-
-// aSB local sub-steps (UpdateTwice, SB/CUDA_GPU/m2_opt.cu:66-71): the reference evaluates them in
-// double because its constants are double literals; explicit _rn ops keep the order fixed.
-__device__ __forceinline__ void asb_local(float &x, float &y, float amp, int m, float mts_dt,
-                                          float detune, float kerr) {
-  double dd = detune, dk = kerr, dh = mts_dt, da = amp;
-  for (int s = 0; s < m; ++s) {
-    x = (float)__dadd_rn((double)x, __dmul_rn(__dmul_rn(dd, (double)y), dh));
-    double lx = (double)x;
-    double x3 = __dmul_rn(__dmul_rn(__dmul_rn(dk, lx), lx), lx);
-    double lin = __dmul_rn(__dadd_rn(dd, -da), lx);
-    y = (float)__dadd_rn((double)y, -__dmul_rn(dh, __dadd_rn(x3, lin)));
   }
 }
 
@@ -288,9 +275,9 @@ __global__ void __launch_bounds__(kThreads) plain_step_kernel(PlainStep a) {
     return;
   }
   // The fields go through shared memory so that the update runs on consecutive threads (thread
-  // t: row t % kRows, replica t / kRows) instead of one lane in each row's warp: the aSB local
-  // sub-steps are FP64, and packing the CTA's elements into one or two warps issues that FP64
-  // work once per CTA instead of once per row.
+  // t: row t % kRows, replica t / kRows) instead of one lane in each row's warp: packing the CTA's
+  // elements into one or two warps issues the aSB local sub-steps (~140 operations each) once per CTA
+  // instead of once per row.
   if (lane == 0 && warp < rows) {
 #pragma unroll
     for (int rr = 0; rr < kMaxRB; ++rr)
@@ -306,7 +293,7 @@ __global__ void __launch_bounds__(kThreads) plain_step_kernel(PlainStep a) {
     const float hv = a.h ? a.h[i] : 0.0f;
     if (VARIANT == 0) {
       y = __fmaf_rn(a.coeff, f, y);
-      if (a.do_local) asb_local(x, y, a.amp_next, a.m, a.mts_dt, a.detune, a.kerr);
+      if (a.do_local) sbasb::local(x, y, a.amp_next, a.m, a.mts_dt, a.detune, a.kerr);
     } else {
       const float s = sgn(x);
       if (VARIANT == 2 && a.energy)
@@ -484,7 +471,7 @@ __global__ void __launch_bounds__(kThreads, 2) plain_tile_kernel(const __grid_co
       const float hv = a.h ? a.h[i] : 0.0f;
       if (VARIANT == 0) {
         y = __fmaf_rn(a.coeff, f[p], y);
-        if (a.do_local) asb_local(x, y, a.amp_next, a.m, a.mts_dt, a.detune, a.kerr);
+        if (a.do_local) sbasb::local(x, y, a.amp_next, a.m, a.mts_dt, a.detune, a.kerr);
       } else {
         const float s = sgn(x);
         if (VARIANT == 2) e = -0.5 * (double)s * (double)f[p] - (double)hv * (double)s;
@@ -763,8 +750,11 @@ __global__ void init_reference_kernel(float *x, float *y, int n, int R, int xp) 
     }
     const float qx = __fmul_rn(__uint2float_rn(u[0]), 2.3283064365386963e-10f);
     const float qy = __fmul_rn(__uint2float_rn(u[1]), 2.3283064365386963e-10f);
-    x[(size_t)r * xp + i] = __double2float_rn(__ddiv_rn((double)qx, 10.0));
-    y[(size_t)r * xp + i] = __double2float_rn(__ddiv_rn((double)qy, 10.0));
+    // the reference divides by 10.0 in double and rounds to float; a quotient of two floats rounded to
+    // 53 >= 2 24 + 2 bits and then to 24 is the float quotient (double rounding is innocuous), so one
+    // FP32 division gives its bits. The FP64 divisions, 2 R in a row per thread, took 70 us at R = 100.
+    x[(size_t)r * xp + i] = __fdiv_rn(qx, 10.0f);
+    y[(size_t)r * xp + i] = __fdiv_rn(qy, 10.0f);
   }
 }
 
@@ -775,7 +765,7 @@ __global__ void asb_local_kernel(float *x, float *y, int n, int R, int xp, float
        k += (size_t)gridDim.x * blockDim.x) {
     const size_t r = k / n, i = k % n, idx = r * xp + i;
     float lx = x[idx], ly = y[idx];
-    asb_local(lx, ly, amp, m, mts_dt, detune, kerr);
+    sbasb::local(lx, ly, amp, m, mts_dt, detune, kerr);
     x[idx] = lx;
     y[idx] = ly;
   }
@@ -827,7 +817,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1) plain_persist_kernel(Plain
   constexpr bool kSigns = VARIANT == 2;
   __shared__ __align__(16) float xs[kPersistMaxJp];  // x(t) of every spin (dSB: its sign, +-1)
   __shared__ uint32_t sout[kPersistRows];
-  __shared__ float sx[kPersistRows], sy[kPersistRows];  // aSB: the rows' x, y for the FP64 sub-steps
+  __shared__ float sx[kPersistRows], sy[kPersistRows];  // aSB: the rows' x, y for the local sub-steps
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int c = blockIdx.x, r = blockIdx.y, G = gridDim.x;
   const int row = c * kPersistRows + warp;
@@ -990,9 +980,9 @@ __global__ void __launch_bounds__(kPersistThreads, 1) plain_persist_kernel(Plain
     }
     if constexpr (VARIANT == 0) {
       if (t + 1 < a.steps) {
-        // aSB: the next step's FP64 local sub-steps (none after the last) for the CTA's 16 rows in
-        // 16 lanes of one warp, where one lane per row warp would issue 16 times the FP64 warp
-        // instructions (FP64 is scarce on this part); rows past n run on x = y = 0 and stay 0
+        // aSB: the next step's local sub-steps (none after the last) for the CTA's 16 rows in 16 lanes
+        // of one warp, where one lane per row warp would issue them 16 times; rows past n run on
+        // x = y = 0 and stay 0
         if (lane == 0) {
           sx[warp] = x;
           sy[warp] = y;
@@ -1000,7 +990,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1) plain_persist_kernel(Plain
         __syncthreads();
         if (warp == 0 && lane < kPersistRows) {
           float lx = sx[lane], ly = sy[lane];
-          asb_local(lx, ly, __fdiv_rn((float)(t + 1), (float)a.steps), a.m, a.mts_dt, a.detune, a.kerr);
+          sbasb::local(lx, ly, __fdiv_rn((float)(t + 1), (float)a.steps), a.m, a.mts_dt, a.detune, a.kerr);
           sx[lane] = lx;
           sy[lane] = ly;
         }
