@@ -18,6 +18,8 @@
 #include "sb_grouped.cuh"
 #include "sb_grouped.h"
 #include "sb_host.h"
+#include "sb_run.cuh"
+#include "sb_run.h"
 
 namespace sbk {
 namespace {
@@ -126,6 +128,13 @@ bool encode_operand(int op, CUtensorMap *m, void *base, int Kp, int kbytes, uint
                         : encode_fp8(m, base, (uint64_t)kbytes, rows, box_rows);
 }
 
+// The V maps of an instance for its current buffers and replica tile.
+bool encode_v(GHost &g, int nr) {
+  for (int b = 0; b < 2; ++b)
+    if (!encode_operand(g.op, &g.desc.tmB[b], g.v[b], g.Kp, g.kbytes, (uint64_t)g.Rp, (uint32_t)nr)) return false;
+  return true;
+}
+
 template <int NR, int OP>
 const void *gk(int emode) {
   return emode == kEmodeEnergy ? reinterpret_cast<const void *>(&grouped_kernel<NR, grouped_stages<NR>(), kEmodeEnergy, OP>)
@@ -135,6 +144,48 @@ const void *gk(int emode) {
 template <int NR>
 const void *gk_op(int op, int emode) {
   return op == kGopE2m1 ? gk<NR, kGopE2m1>(emode) : (op == kGopE2m3 ? gk<NR, kGopE2m3>(emode) : gk<NR, kGopFp8>(emode));
+}
+
+// Couplings a wave may hold: they should stay in the 129 MB L2 beside the signs and the other traffic.
+constexpr int64_t kWaveBytes = 80ll << 20;
+// Steps of one launch (a step's tag has 32 bits).
+constexpr int kWaveSteps = 1 << 20;
+
+// V of every instance at its step tick - t0, from x: one block per item (128 spins x nr replicas).
+__global__ void g_signs_items_kernel(const GInst *insts, const RunItem *items, int nr, int op, int tick) {
+  const RunItem w = items[blockIdx.x];
+  const GInst *in = insts + w.inst;
+  uint8_t *v = in->v[(tick - in->t0) & 1];
+  const int n = in->n, xp = in->xp, kb = in->kbytes, rows = min(nr, in->R - w.r0);
+  if (op == kGopE2m3) {
+    for (int k = threadIdx.x; k < rows * 8; k += blockDim.x) {
+      const int r = w.r0 + k / 8, s0 = w.m0 + 16 * (k % 8);
+      if (s0 >= n) continue;
+      uint32_t word[3] = {0u, 0u, 0u};
+      for (int i = 0; i < 16 && s0 + i < n; ++i) {
+        const uint32_t code = in->x[(size_t)r * xp + s0 + i] > 0.0f ? 0x18u : 0x38u;
+        const int bit = 6 * i;
+        word[bit >> 5] |= code << (bit & 31);
+        if ((bit & 31) > 26) word[(bit >> 5) + 1] |= code >> (32 - (bit & 31));
+      }
+      uint32_t *dst = reinterpret_cast<uint32_t *>(v + (size_t)r * kb + s0 / 16 * 12);
+      for (int i = 0; i < 3; ++i) dst[i] = word[i];
+    }
+    return;
+  }
+  const int per = op == kGopE2m1 ? 64 : 128;  // bytes of a replica's 128 signs
+  for (int k = threadIdx.x; k < rows * per; k += blockDim.x) {
+    const int r = w.r0 + k / per, b = k % per;
+    const float *x = in->x + (size_t)r * xp;
+    if (op == kGopE2m1) {
+      const int i = w.m0 + 2 * b;
+      const uint32_t lo = i < n ? (x[i] > 0.0f ? kE2m1Plus : kE2m1Minus) : 0u;
+      const uint32_t hi = i + 1 < n ? (x[i + 1] > 0.0f ? kE2m1Plus : kE2m1Minus) : 0u;
+      v[(size_t)r * kb + w.m0 / 2 + b] = (uint8_t)(lo | (hi << 4));
+    } else if (w.m0 + b < n) {
+      v[(size_t)r * kb + w.m0 + b] = x[w.m0 + b] > 0.0f ? (uint8_t)0x38 : (uint8_t)0xB8;
+    }
+  }
 }
 
 bool grouped_kernel_for(int nr, int emode, int op, const void **k, size_t *smem) {
@@ -338,6 +389,15 @@ void Grouped::clear() {
   cudaFree(d_sub_items);
   d_sub_items = nullptr;
   cap_sub = 0;
+  cudaFree(d_run);
+  cudaFree(d_rest);
+  cudaFree(d_ll);
+  d_run = nullptr;
+  d_rest = nullptr;
+  d_ll = nullptr;
+  n_run = n_rest = 0;
+  cap_run = cap_rest = cap_ll = 0;
+  waves.clear();
   if (graph) cudaGraphExecDestroy(graph);
   d_insts = nullptr;
   d_items = nullptr;
@@ -427,9 +487,7 @@ sb_status Grouped::prepare(GHost &g, const sb_problem *p, const sb_params *prm, 
   if ((e = cudaMemsetAsync(g.v[1], 0, vb, st)) != cudaSuccess) return fail("memset");
   if ((e = cudaMemsetAsync(g.x, 0, xs, st)) != cudaSuccess) return fail("memset");
   if ((e = cudaMemsetAsync(g.y, 0, xs, st)) != cudaSuccess) return fail("memset");
-  if (!encode_operand(op, &g.desc.tmA, g.a, g.Kp, g.kbytes, (uint64_t)g.Np, kBM) ||
-      !encode_operand(op, &g.desc.tmB[0], g.v[0], g.Kp, g.kbytes, (uint64_t)g.Rp, (uint32_t)nr) ||
-      !encode_operand(op, &g.desc.tmB[1], g.v[1], g.Kp, g.kbytes, (uint64_t)g.Rp, (uint32_t)nr)) {
+  if (!encode_operand(op, &g.desc.tmA, g.a, g.Kp, g.kbytes, (uint64_t)g.Np, kBM) || !encode_v(g, nr)) {
     e = cudaErrorInvalidValue;
     return fail("cuTensorMapEncodeTiled");
   }
@@ -477,7 +535,9 @@ sb_status Grouped::add(const sb_problem *p, const sb_params *prm, uint64_t seed,
 }
 
 
-sb_status Grouped::init_state(GHost &g, uint64_t seed, std::string &err) { return init_state_on(g, seed, st, err); }
+sb_status Grouped::init_state(GHost &g, uint64_t seed, std::string &err) {
+  return init_state_on(g, seed, st, err);
+}
 
 sb_status Grouped::init_state_on(GHost &g, uint64_t seed, cudaStream_t st, std::string &err) {
   cudaError_t e = launch_init_uniform(g.x, g.y, g.n, g.R, g.xp, seed, st);
@@ -514,8 +574,7 @@ sb_status Grouped::retile(int new_nr, std::string &err) {
     }
     cudaMemsetAsync(g.v[0], 0, vb, st);
     cudaMemsetAsync(g.v[1], 0, vb, st);
-    if (!encode_operand(g.op, &g.desc.tmB[0], g.v[0], g.Kp, g.kbytes, (uint64_t)g.Rp, (uint32_t)nr) ||
-        !encode_operand(g.op, &g.desc.tmB[1], g.v[1], g.Kp, g.kbytes, (uint64_t)g.Rp, (uint32_t)nr)) {
+    if (!encode_v(g, nr)) {
       err = "cuTensorMapEncodeTiled";
       return SB_ERR_CUDA;
     }
@@ -586,6 +645,7 @@ sb_status Grouped::sync_tables(std::string &err) {
     err = std::string("synchronize: ") + cudaGetErrorString(e);
     return SB_ERR_CUDA;
   }
+  if (sb_status s = build_waves(err); s != SB_OK) return s;
   if (graph) {
     cudaGraphExecDestroy(graph);
     graph = nullptr;
@@ -594,7 +654,109 @@ sb_status Grouped::sync_tables(std::string &err) {
   return SB_OK;
 }
 
-cudaError_t Grouped::launch(int tick, int emode) { return launch_items(d_items, n_items, tick, emode); }
+namespace {
+// Device array `p` of at least `count` elements (contents not kept).
+template <typename T>
+bool reserve(T *&p, size_t &cap, size_t count) {
+  if (cap >= count) return true;
+  cudaFree(p);
+  p = nullptr;
+  cap = std::max(count, 2 * cap);
+  if (cudaMalloc((void **)&p, cap * sizeof(T)) == cudaSuccess) return true;
+  p = nullptr;
+  cap = 0;
+  return false;
+}
+}  // namespace
+
+// Deals the resident instances into waves, largest first: as many as fit the CTAs' slots and kWaveBytes
+// of couplings (at least one instance). Like-sized instances share a wave, so its CTAs carry like work.
+sb_status Grouped::build_waves(std::string &err) {
+  waves.clear();
+  const int sms = device_sms(), most = run_slots(nr) * sms;
+  std::vector<int> by_size(insts.size());
+  for (size_t i = 0; i < insts.size(); ++i) by_size[i] = (int)i;
+  std::stable_sort(by_size.begin(), by_size.end(), [&](int a, int b) { return insts[a].Kp > insts[b].Kp; });
+  std::vector<RunItem> run;
+  std::vector<GItem> rest;
+  int64_t bytes = 0;
+  size_t ll = 0;
+  for (int i : by_size) {
+    const GHost &g = insts[i];
+    const int mt = g.Np / kBM, rt = g.Rp / nr, kc = grouped_kchunks(g.Kp, g.op);
+    const size_t words = (size_t)2 * 4 * mt * nr;  // of one replica tile
+    if ((int64_t)mt * rt > most) {
+      for (int m = 0; m < mt; ++m)
+        for (int r = 0; r < rt; ++r) rest.push_back(GItem{i, m * kBM, r * nr, kc});
+      continue;
+    }
+    const int64_t ab = (int64_t)g.Np * g.kbytes;
+    if (waves.empty() || waves.back().count + mt * rt > most || bytes + ab > kWaveBytes) {
+      waves.push_back(Wave{(int)run.size(), 0, 0, kc <= kResChunks});
+      bytes = 0;
+    }
+    Wave &w = waves.back();
+    for (int m = 0; m < mt; ++m)
+      for (int r = 0; r < rt; ++r) run.push_back(RunItem{i, m * kBM, r * nr, kc, mt, (uint32_t)(w.ll + r * words)});
+    w.count += mt * rt;
+    w.ll += rt * words;
+    w.res = w.res && w.count <= sms;
+    bytes += ab;
+    ll = std::max(ll, w.ll);
+  }
+  n_run = (int)run.size();
+  n_rest = (int)rest.size();
+  if (!reserve(d_run, cap_run, run.size()) || !reserve(d_rest, cap_rest, rest.size()) || !reserve(d_ll, cap_ll, ll)) {
+    waves.clear();
+    n_run = n_rest = 0;
+    err = "cudaMalloc(wave tables)";
+    return SB_ERR_OOM;
+  }
+  if ((!run.empty() &&
+       cudaMemcpyAsync(d_run, run.data(), run.size() * sizeof(RunItem), cudaMemcpyHostToDevice, st) != cudaSuccess) ||
+      (!rest.empty() &&
+       cudaMemcpyAsync(d_rest, rest.data(), rest.size() * sizeof(GItem), cudaMemcpyHostToDevice, st) != cudaSuccess) ||
+      cudaStreamSynchronize(st) != cudaSuccess) {
+    err = "upload wave tables";
+    return SB_ERR_CUDA;
+  }
+  return SB_OK;
+}
+
+cudaError_t Grouped::run_wave(const Wave &w, int tick0, int count) {
+  RunArgs a;
+  memset(&a, 0, sizeof(a));
+  a.insts = d_insts;
+  a.items = d_run + w.first;
+  a.ll = d_ll;
+  a.status = d_status;
+  a.n_items = w.count;
+  a.skip_item = a.skip_step = -1;
+  a.wait_cycles = ptx::kWaitCycles;
+  v_stale = true;
+  for (int s0 = 0; s0 < count; s0 += kWaveSteps) {
+    a.tick0 = tick0 + s0;
+    a.count = std::min(kWaveSteps, count - s0);
+    cudaError_t e = cudaMemsetAsync(d_ll, 0, w.ll * sizeof(unsigned long long), st);
+    if (e == cudaSuccess) e = launch_run(nr, op, w.res, a, std::min(w.count, device_sms()), st);
+    if (e != cudaSuccess) return e;
+    ++launches;
+  }
+  return cudaSuccess;
+}
+
+cudaError_t Grouped::refresh_v(int tick) {
+  if (!v_stale || n_run == 0) return cudaSuccess;
+  v_stale = false;
+  g_signs_items_kernel<<<n_run, 256, 0, st>>>(d_insts, d_run, nr, op, tick);
+  ++launches;
+  return cudaGetLastError();
+}
+
+cudaError_t Grouped::launch(int tick, int emode) {
+  cudaError_t e = refresh_v(tick);
+  return e == cudaSuccess ? launch_items(d_items, n_items, tick, emode) : e;
+}
 
 cudaError_t Grouped::launch_items(const GItem *items_ptr, int count, int tick, int emode) {
   const void *k = nullptr;
@@ -623,6 +785,13 @@ cudaError_t Grouped::launch_items(const GItem *items_ptr, int count, int tick, i
 
 cudaError_t Grouped::run_steps(int tick0, int count, bool use_graph) {
   if (count <= 0) return cudaSuccess;
+  if (count > 1 && !waves.empty()) {
+    for (const Wave &w : waves)
+      if (cudaError_t e = run_wave(w, tick0, count); e != cudaSuccess) return e;
+    for (int s = 0; s < count && n_rest > 0; ++s)
+      if (cudaError_t e = launch_items(d_rest, n_rest, tick0 + s, kEmodeStep); e != cudaSuccess) return e;
+    return cudaSuccess;
+  }
   if (!use_graph) {
     for (int s = 0; s < count; ++s) {
       cudaError_t e = launch(tick0 + s, kEmodeStep);
@@ -691,6 +860,7 @@ cudaError_t Grouped::energy_pass_for(const std::vector<int> &idx, int tick) {
   }
   cudaError_t e = cudaMemcpyAsync(d_sub_items, items.data(), items.size() * sizeof(GItem), cudaMemcpyHostToDevice, st);
   if (e != cudaSuccess) return e;
+  if ((e = refresh_v(tick)) != cudaSuccess) return e;
   e = launch_items(d_sub_items, (int)items.size(), tick, kEmodeEnergy);
   if (e != cudaSuccess) return e;
   return cudaStreamSynchronize(st);  // `items` is a host temporary

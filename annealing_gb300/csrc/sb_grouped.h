@@ -46,6 +46,8 @@ int64_t grouped_instance_bytes(int n, int R, int steps, int nr, int op = kGopFp8
 // K chunks (128 bytes of shared memory each) of an instance's operand rows
 inline int grouped_kchunks(int Kp, int op) { return op == kGopE2m1 ? Kp / 256 : Kp / 128; }
 
+struct RunItem;  // sb_run.cuh
+
 struct GHost {
   int tag = 0;                  // caller's index / ticket
   const sb_problem *prob = nullptr;
@@ -91,8 +93,12 @@ class Grouped {
   void clear();
   // Re-uploads the instance / item tables after add / remove (synchronous).
   sb_status sync_tables(std::string &err);
-  // Steps ticks [tick0, tick0 + count) for every resident instance (a CUDA graph when use_graph).
+  // Steps ticks [tick0, tick0 + count) for every resident instance. Two steps or more run wave by wave,
+  // a wave's steps in one launch (sb_run.cuh); a single step, and instances with more items than
+  // a wave holds, take one launch per step (a CUDA graph of them when use_graph).
   cudaError_t run_steps(int tick0, int count, bool use_graph);
+  // whether some instance does not fit a wave (valid after sync_tables)
+  bool has_rest() const { return n_rest > 0; }
   // Energies of every resident instance's current spins (instances must be at step t = tick - t0).
   cudaError_t energy_pass(int tick);
   // The same for a subset of resident instances (indices into insts).
@@ -124,6 +130,23 @@ class Grouped {
  private:
   cudaError_t launch(int tick, int emode);
   cudaError_t launch_items(const GItem *items, int count, int tick, int emode);
+  // Instances whose couplings share L2 and whose items fit the SMs (slots per CTA), run together.
+  struct Wave {
+    int first, count;  // its items in d_run
+    size_t ll;         // 8-byte words of its sign exchange
+    bool res;          // J rows resident in shared memory
+  };
+  sb_status build_waves(std::string &err);
+  cudaError_t run_wave(const Wave &w, int tick0, int count);
+  // V(tick) from x for every instance of a wave: the multi-step launches exchange signs of their own
+  cudaError_t refresh_v(int tick);
+  std::vector<Wave> waves;
+  RunItem *d_run = nullptr;          // items of every wave
+  GItem *d_rest = nullptr;           // items of the instances that fit no wave
+  unsigned long long *d_ll = nullptr;  // exchange words of one wave
+  int n_run = 0, n_rest = 0;
+  size_t cap_run = 0, cap_rest = 0, cap_ll = 0;
+  bool v_stale = false;              // the V buffers lag x (a wave has run since)
   GItem *d_sub_items = nullptr;
   int cap_sub = 0;
   void free_instance(GHost &g);

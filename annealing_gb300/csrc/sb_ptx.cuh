@@ -45,6 +45,30 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
   return ok != 0;
 }
 
+// Whether the phase has completed, without waiting.
+__device__ __forceinline__ bool mbar_test(uint64_t *bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
+// True in one lane of a converged warp. tcgen05.mma and the TMA copies take their descriptors,
+// addresses and barriers from uniform registers. In a loop that one lane runs alone (if (lane == 0))
+// the compiler moves every operand there anew for each instruction, ~215 clocks per four MMAs on top of
+// the 193 they take (M = 128, N = 64); in a loop that the whole warp runs, with the issue alone under
+// elect_one, they stay there: measured 49 clocks per MMA issued (against 102), 48 without any wait.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
+
 // Bounded wait without the sleep back-off, for short hand-offs on the critical path.
 __device__ __forceinline__ bool mbar_wait_spin(uint64_t *bar, uint32_t parity, long long limit = kWaitCycles) {
   if (mbar_try_wait(bar, parity)) return true;

@@ -39,8 +39,11 @@
 #include <cmath>
 #include <mutex>
 #include <string>
+#include <vector>
 
 #include "sb_host.h"
+#include "sb_run.cuh"
+#include "sb_run.h"
 #include "sb_tc_fp4.cuh"
 #include "sb_tc_kernel.cuh"
 
@@ -213,6 +216,14 @@ struct TcEngine {
   bool pair = false;  // E2M1 kernel in CTA pairs (clusters of two, launched with that attribute)
   float jscale = 1.0f, jinv = 1.0f;  // FP16 hi + lo: the coupling scale (a power of two) and its inverse
   int flag_stride = 1;  // words between consecutive units' step flags
+  // E2M1 solves without a trace run in the multi-step kernel with tagged sign words (sb_run.cuh)
+  int run_nr = 0, run_grid = 0;  // its replica tile (0: not used) and CTAs
+  GInst *d_inst = nullptr;       // the one instance
+  GInst h_inst;                  // what d_inst holds
+  RunItem *d_items = nullptr;
+  unsigned long long *d_ll = nullptr;
+  size_t ll_words = 0;
+  int n_items = 0;
 };
 
 namespace {
@@ -362,6 +373,61 @@ const char *bind(TcEngine *e, cudaError_t *ce) {
 }  // namespace
 
 namespace {
+// Replica tile of the multi-step kernel for n spins x R replicas, and how its items share CTAs (per_cta
+// items of one spin tile each, its J rows resident): the smallest tile whose items have an SM each, since a
+// step is bound by its dependent chain and a smaller tile shortens every part of it; else two 64-replica
+// items per CTA. Measured, us per step: (N, R) = (300, 1000) 1.85 with 32-replica items, 2.45 with 64;
+// (1111, 300) 2.34 / 3.16; (2000, 256) 2.64 / 3.55; (2000, 512) 3.42 with 64; (2000, 1024) 4.16 with two of
+// 64. The kernel that exchanges operands (sb_tc_fp4.cuh) took 4.43, 6.49, 6.28, 6.27 and 6.20.
+bool run_shape(int n, int R, int sms, int *nr, int *per_cta) {
+  if (kp_for(kTcFp4, n) / 256 > kResChunks) return false;
+  const int mt = (n + kBM - 1) / kBM, t32 = (R + 31) / 32, t64 = (R + 63) / 64;
+  *per_cta = 1;
+  if (mt * t32 <= sms) {
+    *nr = 32;
+  } else if (mt * t64 <= sms) {
+    *nr = 64;
+  } else if (mt * ((t64 + 1) / 2) <= sms) {
+    *nr = 64;
+    *per_cta = 2;
+  } else {
+    return false;
+  }
+  return true;
+}
+
+// Items, exchange words and instance slot of the multi-step kernel; buffers of the engine's own.
+sb_status run_create(TcEngine *e, cudaStream_t st, cudaError_t *ce) {
+  int nr = 0, per = 0;
+  if (e->pair || e->s.variant != 2 || !run_shape(e->s.n, e->s.R, sm_count(), &nr, &per)) return SB_OK;
+  const int mt = (e->s.n + kBM - 1) / kBM, rt = (e->s.R + nr - 1) / nr, cta_r = (rt + per - 1) / per;
+  const size_t words = (size_t)2 * 4 * mt * nr;
+  std::vector<RunItem> items;
+  // CTA b: spin tile b % mt, replica tiles per (b / mt) .. ; slot j of CTA b is item j grid + b. Tiles missing
+  // from the last CTAs come last.
+  const int grid = mt * cta_r;
+  for (int j = 0; j < per; ++j)
+    for (int b = 0; b < grid; ++b) {
+      const int r = per * (b / mt) + j;
+      if (r < rt) items.push_back(RunItem{0, (b % mt) * kBM, r * nr, e->Kp / 256, mt, (uint32_t)(r * words)});
+    }
+  e->ll_words = words * rt;
+  e->n_items = (int)items.size();
+  if ((*ce = cudaMalloc(&e->d_inst, sizeof(GInst))) != cudaSuccess ||
+      (*ce = cudaMalloc(&e->d_items, items.size() * sizeof(RunItem))) != cudaSuccess ||
+      (*ce = cudaMalloc(&e->d_ll, e->ll_words * sizeof(unsigned long long))) != cudaSuccess ||
+      (*ce = cudaMemcpyAsync(e->d_items, items.data(), items.size() * sizeof(RunItem), cudaMemcpyHostToDevice, st)) !=
+          cudaSuccess ||
+      (*ce = cudaStreamSynchronize(st)) != cudaSuccess)
+    return SB_ERR_CUDA;
+  memset(&e->h_inst, 0xFF, sizeof(GInst));  // nothing uploaded yet
+  e->run_nr = nr;
+  e->run_grid = grid;
+  return SB_OK;
+}
+}  // namespace
+
+namespace {
 // The CTA-pair E2M1 kernel runs this dSB shape when asked for (SB_TC_PAIR=1): the 128-replica
 // tile, its units (spin tiles rounded up to an even count) on distinct SMs, every pair co-resident
 // as a cluster of two. It is bit-identical to the single-CTA kernel and measured slower on the
@@ -409,7 +475,7 @@ int64_t tc_footprint(const TcSetup &s) {
   if (s.dtype == kTcFp4) {
     const int64_t Np = (s.n + 2 * kBM - 1) / (2 * kBM) * (2 * kBM), Kb = kp_for(kTcFp4, s.n) / 2;
     const int64_t Rp = (s.R + 127) / 128 * 128;
-    return Np * Kb + 2 * Rp * Kb + 4096;
+    return Np * Kb + 2 * Rp * Kb + Np * Rp / 2 + 65536;  // + the multi-step kernel's exchange words and items
   }
   const int elem = s.dtype == kTcFp8 ? 1 : 2;
   const int64_t Np = (s.n + kBM - 1) / kBM * kBM, Kp = (s.n + 127) / 128 * 128;
@@ -466,6 +532,7 @@ sb_status tc_create(TcEngine **out, const TcSetup &s, const float *dJ, int jp, s
   if ((ce = tc_reload(e, dJ, jp, st)) != cudaSuccess) return fail("convert_j_kernel", ce);
   const char *what = bind(e, &ce);
   if (what) return fail(what, ce);
+  if (s.dtype == kTcFp4 && run_create(e, st, &ce) != SB_OK) return fail("multi-step kernel tables", ce);
   *out = e;
   return SB_OK;
 }
@@ -477,6 +544,9 @@ void tc_destroy(TcEngine *e) {
   for (int b = 0; b < 2; ++b)
     for (int pp = 0; pp < 2; ++pp) cudaFree(e->v[b][pp]);
   cudaFree(e->flags);
+  cudaFree(e->d_inst);
+  cudaFree(e->d_items);
+  cudaFree(e->d_ll);
   delete e;
 }
 
@@ -551,6 +621,51 @@ static cudaError_t launch(TcEngine *e, int emode, const TcArgs &a, cudaStream_t 
   return cudaLaunchKernelExC(&cfg, e->kernel[emode], params);
 }
 
+// All steps of an E2M1 solve in the multi-step kernel, then V(steps) for the energy pass.
+static cudaError_t run_multi(TcEngine *e, const TcArgs &a, cudaStream_t st) {
+  GInst in;
+  memset(&in, 0, sizeof(in));
+  in.tmA = e->args.tmA[0];
+  in.x = a.x;
+  in.y = a.y;
+  in.h = a.h;
+  in.pumps = a.pumps;
+  in.n = e->s.n;
+  in.Kp = e->Kp;
+  in.R = e->s.R;
+  in.Rp = e->Rp;
+  in.xp = e->s.xp;
+  in.c0 = a.c0;
+  in.dt = a.dt;
+  in.dta0 = a.dta0;
+  in.kbytes = e->Kp / 2;
+  cudaError_t ce;
+  if (memcmp(&in, &e->h_inst, sizeof(in)) != 0) {
+    if ((ce = cudaMemcpyAsync(e->d_inst, &in, sizeof(in), cudaMemcpyHostToDevice, st)) != cudaSuccess ||
+        (ce = cudaStreamSynchronize(st)) != cudaSuccess)  // `in` is a host temporary
+      return ce;
+    memcpy(&e->h_inst, &in, sizeof(in));
+  }
+  if ((ce = cudaMemsetAsync(e->d_ll, 0, e->ll_words * sizeof(unsigned long long), st)) != cudaSuccess) return ce;
+  RunArgs r;
+  memset(&r, 0, sizeof(r));
+  r.insts = e->d_inst;
+  r.items = e->d_items;
+  r.ll = e->d_ll;
+  r.status = a.status;
+  r.n_items = e->n_items;
+  r.tick0 = a.t0;
+  r.count = a.steps;
+  r.skip_item = a.skip_unit;
+  r.skip_step = a.skip_step;
+  r.wait_cycles = a.wait_cycles;
+  if ((ce = launch_run(e->run_nr, kGopE2m1, true, r, e->run_grid, st)) != cudaSuccess) return ce;
+  const int Kb = e->Kp / 2;
+  prepare_v_fp4_kernel<<<grid_1d((size_t)e->s.R * Kb), 256, 0, st>>>(a.x, e->s.n, e->s.R, e->s.xp,
+                                                                     e->v[a.steps & 1][0], Kb);
+  return cudaGetLastError();
+}
+
 cudaError_t tc_run(TcEngine *e, int steps, const float *pumps, float *x, float *y, const float *h, float c0,
                    float dt, float dta0, double *energy_trace, uint32_t *status, cudaStream_t st) {
   if (steps <= 0) return cudaSuccess;
@@ -567,6 +682,7 @@ cudaError_t tc_run(TcEngine *e, int steps, const float *pumps, float *x, float *
   a.c0 = c0;
   a.dt = dt;
   a.dta0 = dta0;
+  if (e->run_nr > 0 && !energy_trace) return run_multi(e, a, st);
   cudaError_t ce = cudaMemsetAsync(e->flags, 0, flag_bytes(e), st);
   if (ce != cudaSuccess) return ce;
   return launch(e, energy_trace ? kEmodeStepTrace : kEmodeStep, a, st);
