@@ -560,6 +560,8 @@ sb_status plan_run(sb_plan *pl, uint64_t seed, sb_result *res, std::string &err)
   ++launches;
   std::vector<double> e_final((size_t)R);
   uint32_t status = 0;
+  sbh::touch_pages(res->final_x, (size_t)R * n * sizeof(float));
+  sbh::touch_pages(res->final_y, (size_t)R * n * sizeof(float));
   SB_CUDA(cudaMemcpyAsync(e_final.data(), final_slot, (size_t)R * sizeof(double),
                           cudaMemcpyDeviceToHost, st));
   SB_CUDA(cudaMemcpyAsync(&status, pl->dstatus, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));

@@ -294,6 +294,10 @@ sb_status run(sb_batch *b, uint64_t seed, sb_result *res, std::string &err) {
       inst[bk.members[j]] = &bk.g->insts[j];
       inst_op[bk.members[j]] = bk.g->op;
     }
+  for (size_t k = 0; k < count; ++k) {
+    sbh::touch_pages(res[k].final_x, (size_t)inst[k]->R * inst[k]->n * sizeof(float));
+    sbh::touch_pages(res[k].final_y, (size_t)inst[k]->R * inst[k]->n * sizeof(float));
+  }
   std::vector<std::vector<double>> energies(count);
   std::vector<uint32_t> status(b->buckets.size(), 0);
   for (size_t k = 0; k < count && e == cudaSuccess; ++k) {

@@ -300,6 +300,8 @@ sb_status nmfa_run(sb_ctx *ctx, const sb_problem *prob, const sb_nmfa_params *pr
     ++launches;
   }
   NM_CUDA(cudaEventRecord(c->ev1, st));
+  if (samples32) sbh::touch_pages(samp, (size_t)R * n * sizeof(int32_t));
+  if (res) sbh::touch_pages(res->states, (size_t)R * n * sizeof(float));
   NM_CUDA(cudaMemcpyAsync(samp, c->dsamp, (size_t)R * n * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
   NM_CUDA(cudaMemcpyAsync(hen.data(), c->den, hen.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
   if (res && res->states)
