@@ -96,61 +96,70 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   }
 
   if (warp == 0) {
-    if (lane == 0) {
-      // ---------------- TMA producer ----------------
-      uint32_t g = 0;
-      for (int it = blockIdx.x; it < n_items && ok; it += gridDim.x) {
-        const GItem w = items[it];
-        const GInst *in = insts + w.inst;
-        const int buf = (tick - in->t0) & 1;
-        for (int kc = 0; kc < w.kchunks; ++kc, ++g) {
-          const int s = g % STAGES;
-          const uint32_t use = g / STAGES;
-          if (use > 0 && !ptx::mbar_wait(&empty_bar[s], (use - 1) & 1)) {
-            ok = false;
-            break;
-          }
-          uint8_t *st = smem + s * kStage;
-          ptx::mbar_arrive_expect_tx(&full_bar[s], kTx);
-          ptx::tma_load_2d(st, &in->tmA, kc * kChunkBytes, w.m0, &full_bar[s]);
-          ptx::tma_load_2d(st + kATile, &in->tmB[buf], kc * kChunkBytes, w.r0, &full_bar[s]);
-        }
-      }
-    }
-  } else if (warp == 1) {
-    if (lane == 0) {
-      // ---------------- MMA issuer ----------------
-      uint32_t g = 0;
-      int li = 0;
-      for (int it = blockIdx.x; it < n_items && ok; it += gridDim.x, ++li) {
-        const int kchunks = items[it].kchunks;
-        const int ab = li & 1;
-        const uint32_t t_acc = tmem + ab * NR;
-        if (li >= 2 && !ptx::mbar_wait(&acce_bar[ab], (uint32_t)((li >> 1) - 1) & 1)) {
+    // ---------------- TMA producer (the whole warp; elect_one issues) ----------------
+    uint32_t g = 0;
+    for (int it = blockIdx.x; it < n_items && ok; it += gridDim.x) {
+      const GItem w = items[it];
+      const GInst *in = insts + w.inst;
+      const CUtensorMap *ma = &in->tmA, *mv = &in->tmB[(tick - in->t0) & 1];
+      for (int kc = 0; kc < w.kchunks; ++kc, ++g) {
+        const int s = g % STAGES;
+        const uint32_t use = g / STAGES;
+        if (use > 0 && !__all_sync(0xffffffffu, ptx::mbar_wait(&empty_bar[s], (use - 1) & 1))) {
           ok = false;
           break;
         }
-        ptx::tc_fence_after();
-        for (int kc = 0; kc < kchunks; ++kc, ++g) {
-          const int s = g % STAGES;
-          const uint32_t use = g / STAGES;
-          if (!ptx::mbar_wait(&full_bar[s], use & 1)) {
-            ok = false;
-            break;
-          }
-          ptx::tc_fence_after();
-          const uint32_t sa = ptx::smem_u32(smem + s * kStage);
+        if (ptx::elect_one()) {
+          uint8_t *st = smem + s * kStage;
+          ptx::mbar_arrive_expect_tx(&full_bar[s], kTx);
+          ptx::tma_load_2d(st, ma, kc * kChunkBytes, w.m0, &full_bar[s]);
+          ptx::tma_load_2d(st + kATile, mv, kc * kChunkBytes, w.r0, &full_bar[s]);
+        }
+        __syncwarp();
+      }
+    }
+  } else if (warp == 1) {
+    // ---------------- MMA issuer (the whole warp; elect_one issues) ----------------
+    int s = 0, li = 0;
+    uint32_t ph = 0;
+    bool have = false;  // stage s is known to be full
+    // a stage's descriptors differ from stage 0's in the address field (units of 16 bytes) alone
+    const uint64_t ad0 = ptx::smem_desc_sw128(ptx::smem_u32(smem)), bd0 = ptx::smem_desc_sw128(ptx::smem_u32(smem) + kATile);
+    for (int it = blockIdx.x; it < n_items && ok; it += gridDim.x, ++li) {
+      const int kchunks = items[it].kchunks;
+      const int ab = li & 1;
+      const uint32_t t_acc = tmem + ab * NR;
+      if (li >= 2 && !__all_sync(0xffffffffu, ptx::mbar_wait(&acce_bar[ab], (uint32_t)((li >> 1) - 1) & 1))) {
+        ok = false;
+        break;
+      }
+      ptx::tc_fence_after();
+      for (int kc = 0; kc < kchunks; ++kc) {
+        if (!have && !__all_sync(0xffffffffu, ptx::mbar_wait(&full_bar[s], ph))) {
+          ok = false;
+          break;
+        }
+        const int cur = s;
+        if (++s == STAGES) {
+          s = 0;
+          ph ^= 1;
+        }
+        const bool next = ptx::mbar_test(&full_bar[s], ph);  // looked at while the MMAs below issue
+        if (ptx::elect_one()) {
+          const uint64_t off = (uint64_t)(cur * (kStage / 16));
 #pragma unroll
           for (int k = 0; k < C::kMmaPerChunk; ++k) {
-            const uint64_t ad = ptx::smem_desc_sw128(sa + k * 32), bd = ptx::smem_desc_sw128(sa + kATile + k * 32);
+            const uint64_t ad = ad0 + off + 2 * k, bd = bd0 + off + 2 * k;
             if constexpr (FP4)
               ptx::mma_mxf4(t_acc, ad, bd, kIdesc, tmem + kSf, tmem + kSf + 16, (kc > 0 || k > 0) ? 1u : 0u);
             else
               ptx::mma_f8(t_acc, ad, bd, kIdesc, (kc > 0 || k > 0) ? 1u : 0u);
           }
-          ptx::mma_commit(&empty_bar[s]);
+          ptx::mma_commit(&empty_bar[cur]);
+          if (kc + 1 == kchunks) ptx::mma_commit(&accf_bar[ab]);
         }
-        ptx::mma_commit(&accf_bar[ab]);
+        __syncwarp();
+        have = __all_sync(0xffffffffu, next);
       }
     }
   } else {

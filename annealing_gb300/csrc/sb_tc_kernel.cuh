@@ -296,12 +296,27 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_sb_kernel(const __grid_const
   const int nseg = kSeg ? (p.k_chunks + p.seg_chunks - 1) / p.seg_chunks : 1;
 
   if (warp == 0) {
-    // ---------------- TMA producer (lane 0 issues; the warp polls the column's flags) ----------------
+    // ---------------- TMA producer (the whole warp; elect_one issues) ----------------
     // Every lane runs the same loop and meets the others only at warp-collective points, so a
     // lane that gives up on a wait never strands the rest.
-    uint32_t g = 0;  // chunks issued so far (the MMA lane counts identically)
+    uint32_t g = 0;  // chunks issued so far (the MMA warp counts identically)
     int pre = 0;     // chunks of the coming step whose J part is already in flight
-    uint32_t armed = 0;  // stage uses whose barrier lane 0 has armed (loads in flight or landed)
+    uint32_t armed = 0;  // stage uses whose barrier is armed (loads in flight or landed)
+    // arms chunk gg's stage and starts its J tiles (K offset kx, elements); false when the stage was not freed
+    auto load_j = [&](uint32_t gg, int kx) -> bool {
+      const int s = gg % STAGES;
+      const uint32_t use = gg / STAGES;
+      if (use > 0 && !__all_sync(0xffffffffu, ptx::mbar_wait(&empty_bar[s], (use - 1) & 1, p.wait_cycles))) return false;
+      if (ptx::elect_one()) {
+        ptx::mbar_arrive_expect_tx(&full_bar[s], kTx);
+#pragma unroll
+        for (int a = 0; a < C::kAParts; ++a)
+          ptx::tma_load_2d(smem + s * kStage + a * kATile, &p.tmA[a], kx, m0, &full_bar[s]);
+      }
+      __syncwarp();
+      armed = gg + 1;
+      return true;
+    };
     for (int ls = 0; ls < nsteps && ok; ++ls) {
       const int buf = (p.buf0 + ls) & 1;
       int ready = ls == 0 ? p.n_mtiles : 0;  // units of this column known to have published V(ls)
@@ -315,50 +330,22 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_sb_kernel(const __grid_const
           ready = ready + 32 < p.n_mtiles ? ready + 32 : p.n_mtiles;
           ptx::fence_proxy_async_global();
         }
-        if (lane == 0 && ok) {
+        if (ok && kc >= pre) ok = load_j(g, kx);
+        if (!ok) break;
+        if (ptx::elect_one()) {
           const int s = g % STAGES;
-          const uint32_t use = g / STAGES;
-          uint8_t *st = smem + s * kStage;
-          bool issue = true;
-          if (kc >= pre) {
-            if (use > 0 && !ptx::mbar_wait(&empty_bar[s], (use - 1) & 1, p.wait_cycles)) {
-              ok = false;
-              issue = false;
-            } else {
-              ptx::mbar_arrive_expect_tx(&full_bar[s], kTx);
-              for (int a = 0; a < C::kAParts; ++a)
-                ptx::tma_load_2d(st + a * kATile, &p.tmA[a], kx, m0, &full_bar[s]);
-              armed = g + 1;
-            }
-          }
-          if (issue)
-            for (int b = 0; b < C::kBParts; ++b)
-              ptx::tma_load_2d(st + C::kAParts * kATile + b * kBTile, &p.tmB[buf][b], kx, r0, &full_bar[s]);
+#pragma unroll
+          for (int b = 0; b < C::kBParts; ++b)
+            ptx::tma_load_2d(smem + s * kStage + C::kAParts * kATile + b * kBTile, &p.tmB[buf][b], kx, r0, &full_bar[s]);
         }
-        ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+        __syncwarp();
       }
       // J does not change between steps: start the next step's first J tiles now.
       pre = 0;
-      if (lane == 0 && ok && ls + 1 < nsteps) {
+      if (ok && ls + 1 < nsteps) {
         const int npre = p.k_chunks < STAGES ? p.k_chunks : STAGES;
-        for (int kc = 0; kc < npre; ++kc) {
-          const uint32_t gg = g + kc;
-          const int s = gg % STAGES;
-          const uint32_t use = gg / STAGES;
-          if (use > 0 && !ptx::mbar_wait(&empty_bar[s], (use - 1) & 1, p.wait_cycles)) {
-            ok = false;
-            break;
-          }
-          ptx::mbar_arrive_expect_tx(&full_bar[s], kTx);
-          for (int a = 0; a < C::kAParts; ++a)
-            ptx::tma_load_2d(smem + s * kStage + a * kATile, &p.tmA[a], kc * (kChunkBytes / C::kElem), m0,
-                             &full_bar[s]);
-          armed = gg + 1;
-          ++pre;
-        }
+        while (pre < npre && (ok = load_j(g + pre, pre * (kChunkBytes / C::kElem)))) ++pre;
       }
-      pre = __shfl_sync(0xffffffffu, pre, 0);
-      ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
     }
     if (!ok && lane == 0) {
       // a wait gave up: let the copies this CTA started land before it exits (each stage's last
@@ -368,31 +355,47 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_sb_kernel(const __grid_const
         if (armed > (uint32_t)s) ptx::mbar_wait(&full_bar[s], ((armed - 1 - s) / STAGES) & 1, p.wait_cycles);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      // ---------------- MMA issuer ----------------
-      uint32_t g = 0;
-      uint32_t gs = 0;  // split operands: segments issued
-      for (int ls = 0; ls < nsteps && ok; ++ls) {
-        const int ab = ls & 1;
-        if constexpr (!kSeg) {
-          if (ls >= 2 && !ptx::mbar_wait(&acce_bar[ab], (uint32_t)((ls >> 1) - 1) & 1, p.wait_cycles)) { ok = false; break; }
+    // ---------------- MMA issuer (the whole warp; elect_one issues) ----------------
+    int s = 0;
+    uint32_t ph = 0;
+    uint32_t gs = 0;    // split operands: segments issued
+    bool have = false;  // stage s is known to be full
+    // a stage's descriptors differ from stage 0's in the address field (units of 16 bytes) alone
+    const uint64_t ad0 = ptx::smem_desc_sw128(ptx::smem_u32(smem));
+    const uint64_t bd0 = ptx::smem_desc_sw128(ptx::smem_u32(smem) + C::kAParts * kATile);
+    for (int ls = 0; ls < nsteps && ok; ++ls) {
+      const int ab = ls & 1;
+      if constexpr (!kSeg) {
+        if (ls >= 2 && !__all_sync(0xffffffffu, ptx::mbar_wait(&acce_bar[ab], (uint32_t)((ls >> 1) - 1) & 1, p.wait_cycles))) {
+          ok = false;
+          break;
+        }
+        ptx::tc_fence_after();
+      }
+      int kin = 0;  // chunk index inside the current segment
+      for (int kc = 0; kc < p.k_chunks; ++kc) {
+        const uint32_t t_acc = tmem + (kSeg ? 0 : ab) * NR;
+        if (kSeg && kin == 0) {
+          // the segment block is free once the epilogue has loaded the previous segment
+          if (gs >= 1 && !__all_sync(0xffffffffu, ptx::mbar_wait_spin(&acce_bar[0], (uint32_t)(gs - 1) & 1, p.wait_cycles))) {
+            ok = false;
+            break;
+          }
           ptx::tc_fence_after();
         }
-        int kin = 0;  // chunk index inside the current segment
-        for (int kc = 0; kc < p.k_chunks; ++kc, ++g) {
-          const uint32_t t_acc = tmem + (kSeg ? 0 : ab) * NR;
-          if (kSeg && kin == 0) {
-            // the segment block is free once the epilogue has loaded the previous segment
-            if (gs >= 1 && !ptx::mbar_wait_spin(&acce_bar[0], (uint32_t)(gs - 1) & 1, p.wait_cycles)) { ok = false; break; }
-            ptx::tc_fence_after();
-          }
-          const int s = g % STAGES;
-          const uint32_t use = g / STAGES;
-          if (!ptx::mbar_wait(&full_bar[s], use & 1, p.wait_cycles)) { ok = false; break; }
-          ptx::tc_fence_after();
-          const uint32_t sa = ptx::smem_u32(smem + s * kStage);
-          const uint32_t sb = sa + C::kAParts * kATile;
-          int prod = 0;
+        if (!have && !__all_sync(0xffffffffu, ptx::mbar_wait(&full_bar[s], ph, p.wait_cycles))) {
+          ok = false;
+          break;
+        }
+        const int cur = s;
+        if (++s == STAGES) {
+          s = 0;
+          ph ^= 1;
+        }
+        const bool next = ptx::mbar_test(&full_bar[s], ph);  // looked at while the MMAs below issue
+        const bool seg_end = kSeg && (kin + 1 == p.seg_chunks || kc + 1 == p.k_chunks);
+        if (ptx::elect_one()) {
+          const uint64_t off = (uint64_t)(cur * (kStage / 16));
 #pragma unroll
           for (int a = 0; a < C::kAParts; ++a) {
 #pragma unroll
@@ -400,34 +403,31 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_sb_kernel(const __grid_const
               if (a + b > 1) continue;  // lo * lo is below the FP32 accumulator's resolution
 #pragma unroll
               for (int k = 0; k < C::kMmaPerChunk; ++k) {
-                const uint64_t ad = ptx::smem_desc_sw128(sa + a * kATile + k * 32);
-                const uint64_t bd = ptx::smem_desc_sw128(sb + b * kBTile + k * 32);
-                const uint32_t acc = ((kSeg ? kin : kc) > 0 || prod > 0 || k > 0) ? 1u : 0u;
+                const uint64_t ad = ad0 + off + a * (kATile / 16) + 2 * k, bd = bd0 + off + b * (kBTile / 16) + 2 * k;
+                const uint32_t acc = ((kSeg ? kin : kc) > 0 || a + b > 0 || k > 0) ? 1u : 0u;
                 if constexpr (DT == kTcFp8)
                   ptx::mma_f8(t_acc, ad, bd, kIdesc, acc);
                 else
                   ptx::mma_f16(t_acc, ad, bd, kIdesc, acc);
               }
-              ++prod;
             }
           }
-          ptx::mma_commit(&empty_bar[s]);
-          if constexpr (kSeg) {
-            if (++kin == p.seg_chunks || kc + 1 == p.k_chunks) {
-              ptx::mma_commit(&accf_bar[0]);
-              ++gs;
-              kin = 0;
-            }
-          }
+          ptx::mma_commit(&empty_bar[cur]);
+          if (kSeg ? seg_end : kc + 1 == p.k_chunks) ptx::mma_commit(&accf_bar[kSeg ? 0 : ab]);
         }
-        if (!ok) break;
-        if constexpr (!kSeg) ptx::mma_commit(&accf_bar[ab]);
+        __syncwarp();
+        have = __all_sync(0xffffffffu, next);
+        if constexpr (kSeg) {
+          kin = seg_end ? 0 : kin + 1;
+          gs += seg_end ? 1u : 0u;
+        }
       }
-      if (!ok) {
-        // a wait gave up: the MMAs already issued finish before TMEM is freed
-        ptx::mma_commit(&drain_bar);
-        ptx::mbar_wait(&drain_bar, 0, p.wait_cycles);
-      }
+    }
+    if (!ok) {
+      // a wait gave up: the MMAs already issued finish before TMEM is freed
+      if (ptx::elect_one()) ptx::mma_commit(&drain_bar);
+      __syncwarp();
+      ptx::mbar_wait(&drain_bar, 0, p.wait_cycles);
     }
   } else {
     // ---------------- epilogue: 8 warps, two per TMEM lane quadrant ----------------
