@@ -135,6 +135,10 @@ cudaError_t launch_pad_rows_f32(const float *src, float *dst, int n, int jp, cud
 // multiples of 16 bytes) read in unswizzled boxes of box_rows x box_cols, zero beyond its edges.
 bool encode_rows_f32(CUtensorMap *m, const float *base, int rows, int cols, int pitch, int box_cols, int box_rows);
 
+// Tensor map of rows x row_bytes operand bytes (row_bytes a multiple of 128) read in 128-byte x box_rows boxes
+// with the 128-byte swizzle.
+bool encode_operand_bytes(CUtensorMap *m, void *base, uint64_t row_bytes, uint64_t rows, uint32_t box_rows);
+
 // ---------------------------------------------------------------------------------------------
 // Tensor-core (tcgen05) path. See sb_tc.cu.
 enum TcDtype : int { kTcFp8 = 1, kTcBf16 = 2, kTcBf16Split = 3, kTcFp4 = 4, kTcFp16Split = 5 };

@@ -324,6 +324,10 @@ __global__ void __launch_bounds__(kSqaMaxWarps * 32, 1) sqa_kernel(const __grid_
     for (int k = tid; k < M * W; k += blockDim.x) p.spins[(size_t)r * M * W + k] = sp[(k / W) * SPS + k % W];
 }
 
+}  // namespace
+#include "sb_sqa_tc.cuh"
+namespace {
+
 // Initial slices as bits [R][M][W]. Reference mode (pre_calculate.cu:38-51, :186-191, :213): spin i
 // keeps one xorshift32 state seeded with i; replica r takes calls r M + 1 .. (r + 1) M for its
 // slices and keeps the state after them as the spin's random word. Hash mode: one counter hash per
@@ -333,7 +337,7 @@ __global__ void sqa_init_kernel(uint32_t *spins, uint32_t *rnd, int n, int W, in
   const int i = blockIdx.x * blockDim.x + threadIdx.x;  // grid covers W * 32 threads
   const bool in = i < n;
   uint32_t st = (uint32_t)i;
-  for (int r = 0; r < R; ++r) {
+  for (int r = blockIdx.y; r < R; r += gridDim.y) {  // reference mode: one block row, the calls are in sequence
     for (int m = 0; m < M; ++m) {
       bool neg;
       if (mode == 0) {
@@ -354,29 +358,66 @@ __global__ void sqa_init_kernel(uint32_t *spins, uint32_t *rnd, int n, int W, in
   }
 }
 
-// Bit-plane rows of J ([n][n] FP32 integers, |J| < 2^P) into [n][RW]: per 32-coupling word the sign
-// word then the P magnitude words, the row's sum of |J| after them; one thread per word.
-__global__ void sqa_rows_kernel(const float *J, int n, int W, int P, int RW, uint32_t *rows) {
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (t >= (long long)n * W) return;
-  const int i = (int)(t / W), w = (int)(t % W);
-  uint32_t sign = 0, mag[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  int abs_sum = 0;
+// The couplings in the forms the kernels read, one thread per output piece of J ([n][n] FP32 integers,
+// |J| < 2^P):
+//   rows [n][RW]: per 32-coupling word the sign word then the P magnitude words, the row's sum of |J| after them;
+//   and, when op is not null (|J| <= 4, n >= 128), for sqa_tc_kernel
+//   op [n + 128][Kp / 2]: packed E2M1, row n + k repeating row k, nibble 8 k + i of a 32-column group holding its
+//   column 4 i + k;
+//   window [n][2][window_words(P)]: planes (sign, magnitudes) of J[i][(i - 32 h - b - 1) mod n] at bit b of word h.
+__global__ void sqa_setup_kernel(const float *J, int n, int W, int P, int RW, uint32_t *rows, uint8_t *op, int Kp,
+                                 uint32_t *window) {
+  long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (t < (long long)n * W) {
+    const int i = (int)(t / W), w = (int)(t % W);
+    uint32_t sign = 0, mag[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    int abs_sum = 0;
+    for (int b = 0; b < 32; ++b) {
+      const int j = w * 32 + b;
+      if (j >= n || j == i) continue;
+      const int v = (int)J[(size_t)i * n + j];
+      const int a = v < 0 ? -v : v;
+      if (v < 0) sign |= 1u << b;
+      for (int k = 0; k < P; ++k)
+        if ((a >> k) & 1) mag[k] |= 1u << b;
+      abs_sum += a;
+    }
+    uint32_t *row = rows + (size_t)i * RW;
+    row[(size_t)w * (P + 1)] = sign;
+    for (int k = 0; k < P; ++k) row[(size_t)w * (P + 1) + k + 1] = mag[k];
+    // the row's sum of |J| (warps of one row reduce through an atomic; the word starts at 0)
+    atomicAdd(&row[(P + 1) * W], (uint32_t)abs_sum);
+    return;
+  }
+  if (!op) return;
+  t -= (long long)n * W;
+  const int groups = Kp / 32;
+  if (t < (long long)(n + 128) * groups) {
+    const int i = (int)(t / groups) % n, g = (int)(t % groups);
+    uint32_t word[4] = {0u, 0u, 0u, 0u};
+    for (int b = 0; b < 32; ++b) {
+      const int j = 32 * g + b;
+      if (j >= n || j == i) continue;
+      const uint32_t code = sbk::tck::e2m1_code(J[(size_t)i * n + j]) & 0xFu;
+      word[b & 3] |= code << (4 * (b >> 2));
+    }
+    reinterpret_cast<uint4 *>(op)[t] = make_uint4(word[0], word[1], word[2], word[3]);
+    return;
+  }
+  t -= (long long)(n + 128) * groups;
+  if (t >= 2ll * n) return;
+  const int i = (int)(t >> 1), half = (int)(t & 1);
+  uint32_t plane[4] = {0u, 0u, 0u, 0u};  // |J| <= 4: at most three magnitude planes
   for (int b = 0; b < 32; ++b) {
-    const int j = w * 32 + b;
-    if (j >= n || j == i) continue;
+    int j = i - (32 * half + b) - 1;
+    if (j < 0) j += n;
     const int v = (int)J[(size_t)i * n + j];
     const int a = v < 0 ? -v : v;
-    if (v < 0) sign |= 1u << b;
+    if (v < 0) plane[0] |= 1u << b;
     for (int k = 0; k < P; ++k)
-      if ((a >> k) & 1) mag[k] |= 1u << b;
-    abs_sum += a;
+      if ((a >> k) & 1) plane[k + 1] |= 1u << b;
   }
-  uint32_t *row = rows + (size_t)i * RW;
-  row[(size_t)w * (P + 1)] = sign;
-  for (int k = 0; k < P; ++k) row[(size_t)w * (P + 1) + k + 1] = mag[k];
-  // the row's sum of |J| (warps of one row reduce through an atomic; the word starts at 0)
-  atomicAdd(&row[(P + 1) * W], (uint32_t)abs_sum);
+  for (int k = 0; k <= P; ++k) window[(size_t)t * sqatc::window_words(P) + k] = plane[k];
 }
 
 // The kernel for P magnitude planes (|J| < 2^P, P <= 7).
@@ -391,6 +432,22 @@ const void *sqa_kernel_for(int P) {
     default: return reinterpret_cast<const void *>(&sqa_kernel<7>);
   }
 }
+
+// The tensor-core kernel for M slices and P planes.
+template <int NS>
+const void *sqa_tc_kernel_ns(int P) {
+  return P == 1   ? reinterpret_cast<const void *>(&sqatc::sqa_tc_kernel<NS, 1>)
+         : P == 2 ? reinterpret_cast<const void *>(&sqatc::sqa_tc_kernel<NS, 2>)
+                  : reinterpret_cast<const void *>(&sqatc::sqa_tc_kernel<NS, 3>);
+}
+const void *sqa_tc_kernel_for(int M, int P) { return M <= 32 ? sqa_tc_kernel_ns<32>(P) : sqa_tc_kernel_ns<64>(P); }
+template <int NS>
+size_t sqa_tc_smem_ns(int M, int P, int SPS) {
+  return P == 1   ? sqatc::Layout<NS, 1>::bytes(M, SPS)
+         : P == 2 ? sqatc::Layout<NS, 2>::bytes(M, SPS)
+                  : sqatc::Layout<NS, 3>::bytes(M, SPS);
+}
+size_t sqa_tc_smem(int M, int P, int SPS) { return M <= 32 ? sqa_tc_smem_ns<32>(M, P, SPS) : sqa_tc_smem_ns<64>(M, P, SPS); }
 
 // cudaLaunchKernel argument array for a kernel taking one SqaArgs by value
 void **args_of(SqaArgs &a) {
@@ -461,6 +518,14 @@ extern "C" sb_status sb_sqa_solve(sb_ctx *ctx, const sb_problem *prob, const sb_
   const int RS = RW + ((16 - RW % 32) + 32) % 32;
   const int SPS = W + (((P == 1 ? 16 : 8) - W % 32) + 32) % 32;
   const size_t sp_words = (size_t)M * SPS;
+  // |J| <= 4, M <= 64: the tensor-core kernel, whose fields fit 16 bits and whose rows of a block are distinct
+  // (n >= 128). Faster wherever it runs, ms of 6 annealing steps against sqa_kernel: n = 150, M = R = 4 0.17 / 0.65;
+  // n = 500, M = 16, R = 64 0.51 / 2.06; n = 1000, M = 64, R = 304 1.6 / 8.7; n = 4096, M = 64, R = 4 6.2 / 26.5,
+  // R = 304 7.5 / 37.8; n = 2000, M = 64, R = 304, |J| <= 3 3.6 / 21.9; n = 6000, M = 64, R = 304 22 / 102.
+  const int tc_sps = W + 1, tc_kp = (n + 255) / 256 * 256;  // W is a multiple of four: odd
+  const size_t tc_smem = sqa_tc_smem(M, P, tc_sps);
+  const bool use_tc = prob->max_abs_j <= 4 && M <= 64 && n >= 128 && (long long)n * prob->max_abs_j <= 32767 &&
+                      tc_smem <= kSqaSmemBudget;
   // ring slots: the M rows of one iteration plus up to kSqaAhead rows ahead; the deepest ring that
   // lets two CTAs (two replicas) share an SM, else the deepest that fits one
   int S = 0;
@@ -469,12 +534,14 @@ extern "C" sb_status sb_sqa_solve(sb_ctx *ctx, const sb_problem *prob, const sb_
       const size_t bytes = (size_t)(M + d) * RS * 4 + sp_words * 4 + thr_words * 4 + (size_t)(M + d) * 8;
       if (bytes <= budget) S = M + d;
     }
-  if (S == 0) return fail(ctx, SB_ERR_UNSUPPORTED, "sb_sqa_solve: trotter x n too large for one CTA's shared memory");
+  if (S == 0 && !use_tc) return fail(ctx, SB_ERR_UNSUPPORTED, "sb_sqa_solve: trotter x n too large for one CTA's shared memory");
   const size_t smem = (size_t)S * RS * 4 + sp_words * 4 + thr_words * 4 + (size_t)S * 8;
   const int threads = 32 * ((M + kSqaSlicesPerWarp - 1) / kSqaSlicesPerWarp);
   cudaStream_t st = ctx->stream;
   cudaError_t e;
   float *dJ = nullptr, *dbeta = nullptr, *djp = nullptr;
+  uint32_t *dwindow = nullptr;
+  uint8_t *dop = nullptr;
   uint32_t *drows = nullptr, *dspins = nullptr, *drnd = nullptr, *dstatus = nullptr;
   int64_t *den = nullptr;
   const size_t en_count = prm->trace ? (size_t)R * steps : (size_t)R;
@@ -492,11 +559,16 @@ extern "C" sb_status sb_sqa_solve(sb_ctx *ctx, const sb_problem *prob, const sb_
     where = #call;                    \
     goto cleanup;                     \
   }
-  SQ_CUDA(cudaFuncSetAttribute(sqa_kernel_for(P), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  SQ_CUDA(cudaFuncSetAttribute(use_tc ? sqa_tc_kernel_for(M, P) : sqa_kernel_for(P),
+                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(use_tc ? tc_smem : smem)));
   SQ_CUDA(cudaEventCreate(&ev0));
   SQ_CUDA(cudaEventCreate(&ev1));
   SQ_CUDA(cudaMallocAsync((void **)&dJ, (size_t)n * n * sizeof(float), st));
   SQ_CUDA(cudaMallocAsync((void **)&drows, (size_t)n * RW * sizeof(uint32_t), st));
+  if (use_tc) {
+    SQ_CUDA(cudaMallocAsync((void **)&dop, (size_t)(n + 128) * tc_kp / 2, st));
+    SQ_CUDA(cudaMallocAsync((void **)&dwindow, (size_t)n * 2 * sqatc::window_words(P) * sizeof(uint32_t), st));
+  }
   SQ_CUDA(cudaMallocAsync((void **)&dspins, (size_t)R * spin_words * sizeof(uint32_t), st));
   if (prm->rng_mode == SB_SQA_RNG_REFERENCE) SQ_CUDA(cudaMallocAsync((void **)&drnd, (size_t)R * n * sizeof(uint32_t), st));
   SQ_CUDA(cudaMallocAsync((void **)&dbeta, (size_t)steps * sizeof(float), st));
@@ -510,33 +582,64 @@ extern "C" sb_status sb_sqa_solve(sb_ctx *ctx, const sb_problem *prob, const sb_
   SQ_CUDA(cudaMemsetAsync(dstatus, 0, sizeof(uint32_t), st));
   SQ_CUDA(cudaEventRecord(ev0, st));
   {
-    const long long nt = (long long)n * W;
-    sqa_rows_kernel<<<(unsigned)((nt + 255) / 256), 256, 0, st>>>(dJ, n, W, P, RW, drows);
+    const long long nt = (long long)n * W + (use_tc ? (long long)(n + 128) * (tc_kp / 32) + 2ll * n : 0);
+    sqa_setup_kernel<<<(unsigned)((nt + 255) / 256), 256, 0, st>>>(dJ, n, W, P, RW, drows, dop, tc_kp, dwindow);
     SQ_CUDA(cudaGetLastError());
-    sqa_init_kernel<<<(W * 32 + 127) / 128, 128, 0, st>>>(dspins, drnd, n, W, M, R,
-                                                          prm->rng_mode == SB_SQA_RNG_REFERENCE ? 0 : 1, prm->seed);
+    const bool ref_rng = prm->rng_mode == SB_SQA_RNG_REFERENCE;
+    sqa_init_kernel<<<dim3((W * 32 + 127) / 128, ref_rng ? 1 : std::min(R, 65535)), 128, 0, st>>>(
+        dspins, drnd, n, W, M, R, ref_rng ? 0 : 1, prm->seed);
     SQ_CUDA(cudaGetLastError());
-    SqaArgs a;
-    a.rows = drows;
-    a.spins = dspins;
-    a.rnd = drnd;
-    a.beta = dbeta;
-    a.jperp = djp;
-    a.energy = den;
-    a.status = dstatus;
-    a.seed = prm->seed;
-    a.n = n;
-    a.W = W;
-    a.P = P;
-    a.RW = RW;
-    a.M = M;
-    a.steps = steps;
-    a.S = S;
-    a.RS = RS;
-    a.SPS = SPS;
-    a.trace = prm->trace ? 1 : 0;
-    SQ_CUDA(cudaLaunchKernel(sqa_kernel_for(P), dim3((unsigned)R), dim3((unsigned)threads), args_of(a), smem, st));
-    SQ_CUDA(cudaGetLastError());
+    if (use_tc) {
+      sqatc::Args a;
+      memset(&a, 0, sizeof(a));
+      if (!sbk::encode_operand_bytes(&a.tmJ, dop, (uint64_t)tc_kp / 2, (uint64_t)n + 128, 128)) {
+        out = SB_ERR_CUDA;
+        ctx->last_error = "sb_sqa_solve: cuTensorMapEncodeTiled";
+        goto cleanup_noerr;
+      }
+      a.rows = drows;
+      a.window = dwindow;
+      a.spins = dspins;
+      a.rnd = drnd;
+      a.beta = dbeta;
+      a.jperp = djp;
+      a.energy = den;
+      a.status = dstatus;
+      a.seed = prm->seed;
+      a.n = n;
+      a.W = W;
+      a.RW = RW;
+      a.M = M;
+      a.steps = steps;
+      a.trace = prm->trace ? 1 : 0;
+      a.chunks = tc_kp / 256;
+      a.SPS = tc_sps;
+      void *args[] = {&a};
+      SQ_CUDA(cudaLaunchKernel(sqa_tc_kernel_for(M, P), dim3((unsigned)R), dim3(sqatc::kThreads), args, tc_smem, st));
+      SQ_CUDA(cudaGetLastError());
+    } else {
+      SqaArgs a;
+      a.rows = drows;
+      a.spins = dspins;
+      a.rnd = drnd;
+      a.beta = dbeta;
+      a.jperp = djp;
+      a.energy = den;
+      a.status = dstatus;
+      a.seed = prm->seed;
+      a.n = n;
+      a.W = W;
+      a.P = P;
+      a.RW = RW;
+      a.M = M;
+      a.steps = steps;
+      a.S = S;
+      a.RS = RS;
+      a.SPS = SPS;
+      a.trace = prm->trace ? 1 : 0;
+      SQ_CUDA(cudaLaunchKernel(sqa_kernel_for(P), dim3((unsigned)R), dim3((unsigned)threads), args_of(a), smem, st));
+      SQ_CUDA(cudaGetLastError());
+    }
   }
   SQ_CUDA(cudaEventRecord(ev1, st));
   SQ_CUDA(cudaMemcpyAsync(hen.data(), den, en_count * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
@@ -589,6 +692,8 @@ cleanup:
 cleanup_noerr:
   cudaFreeAsync(dJ, st);
   cudaFreeAsync(drows, st);
+  if (dop) cudaFreeAsync(dop, st);
+  if (dwindow) cudaFreeAsync(dwindow, st);
   cudaFreeAsync(dspins, st);
   if (drnd) cudaFreeAsync(drnd, st);
   cudaFreeAsync(dbeta, st);

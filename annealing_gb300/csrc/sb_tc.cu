@@ -203,6 +203,10 @@ bool encode_rows_f32(CUtensorMap *m, const float *base, int rows, int cols, int 
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+bool encode_operand_bytes(CUtensorMap *m, void *base, uint64_t row_bytes, uint64_t rows, uint32_t box_rows) {
+  return encode_2d(m, base, 1, row_bytes, rows, box_rows);
+}
+
 struct TcEngine {
   TcSetup s{};
   int nr = 128, Np = 0, Kp = 0, Rp = 0, n_mtiles = 0, n_rtiles = 0, units = 0;
