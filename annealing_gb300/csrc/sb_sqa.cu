@@ -433,21 +433,40 @@ const void *sqa_kernel_for(int P) {
   }
 }
 
-// The tensor-core kernel for M slices and P planes.
-template <int NS>
-const void *sqa_tc_kernel_ns(int P) {
-  return P == 1   ? reinterpret_cast<const void *>(&sqatc::sqa_tc_kernel<NS, 1>)
-         : P == 2 ? reinterpret_cast<const void *>(&sqatc::sqa_tc_kernel<NS, 2>)
-                  : reinterpret_cast<const void *>(&sqatc::sqa_tc_kernel<NS, 3>);
+// The tensor-core kernel for M slices and P planes, its J stages (0: its spins leave no room for two), the replicas
+// of a CTA and its shared memory.
+struct SqaTc {
+  const void *kernel;
+  int jstages, nrep;
+  size_t smem;
+};
+template <int NS, int P, int NREP>
+SqaTc sqa_tc(int M, int SPS, size_t budget) {
+  using L = sqatc::Layout<NS, P, NREP>;
+  const size_t fixed = L::bytes(M, SPS, 0);
+  int js = 0;
+  if (fixed + 2 * sbk::tck::kFp4ATile <= budget)
+    js = std::min<int>(sqatc::kMaxJStages, (int)((budget - fixed) / sbk::tck::kFp4ATile));
+  return SqaTc{reinterpret_cast<const void *>(&sqatc::sqa_tc_kernel<NS, P, NREP>), js, NREP, L::bytes(M, SPS, js)};
 }
-const void *sqa_tc_kernel_for(int M, int P) { return M <= 32 ? sqa_tc_kernel_ns<32>(P) : sqa_tc_kernel_ns<64>(P); }
-template <int NS>
-size_t sqa_tc_smem_ns(int M, int P, int SPS) {
-  return P == 1   ? sqatc::Layout<NS, 1>::bytes(M, SPS)
-         : P == 2 ? sqatc::Layout<NS, 2>::bytes(M, SPS)
-                  : sqatc::Layout<NS, 3>::bytes(M, SPS);
+template <int NS, int NREP>
+SqaTc sqa_tc_planes(int M, int P, int SPS, size_t budget) {
+  return P == 1   ? sqa_tc<NS, 1, NREP>(M, SPS, budget)
+         : P == 2 ? sqa_tc<NS, 2, NREP>(M, SPS, budget)
+                  : sqa_tc<NS, 3, NREP>(M, SPS, budget);
 }
-size_t sqa_tc_smem(int M, int P, int SPS) { return M <= 32 ? sqa_tc_smem_ns<32>(M, P, SPS) : sqa_tc_smem_ns<64>(M, P, SPS); }
+// More replicas than SMs: two CTAs to an SM, or, where their shared memory leaves fewer than three J stages, two
+// replicas to a CTA; else an SM for each.
+SqaTc sqa_tc_for(int M, int P, int SPS, int R, int sms) {
+  if (R > sms) {
+    const size_t half = kSqaSmemHalf - 1024;  // less the static part, 1.4 KB
+    const SqaTc pair = M <= 32 ? sqa_tc_planes<32, 1>(M, P, SPS, half) : sqa_tc_planes<64, 1>(M, P, SPS, half);
+    if (pair.jstages >= 3) return pair;
+    const SqaTc two = M <= 32 ? sqa_tc_planes<32, 2>(M, P, SPS, kSqaSmemBudget) : sqa_tc_planes<64, 2>(M, P, SPS, kSqaSmemBudget);
+    if (two.jstages > 0) return two;
+  }
+  return M <= 32 ? sqa_tc_planes<32, 1>(M, P, SPS, kSqaSmemBudget) : sqa_tc_planes<64, 1>(M, P, SPS, kSqaSmemBudget);
+}
 
 // cudaLaunchKernel argument array for a kernel taking one SqaArgs by value
 void **args_of(SqaArgs &a) {
@@ -519,13 +538,15 @@ extern "C" sb_status sb_sqa_solve(sb_ctx *ctx, const sb_problem *prob, const sb_
   const int SPS = W + (((P == 1 ? 16 : 8) - W % 32) + 32) % 32;
   const size_t sp_words = (size_t)M * SPS;
   // |J| <= 4, M <= 64: the tensor-core kernel, whose fields fit 16 bits and whose rows of a block are distinct
-  // (n >= 128). Faster wherever it runs, ms of 6 annealing steps against sqa_kernel: n = 150, M = R = 4 0.17 / 0.65;
-  // n = 500, M = 16, R = 64 0.51 / 2.06; n = 1000, M = 64, R = 304 1.6 / 8.7; n = 4096, M = 64, R = 4 6.2 / 26.5,
-  // R = 304 7.5 / 37.8; n = 2000, M = 64, R = 304, |J| <= 3 3.6 / 21.9; n = 6000, M = 64, R = 304 22 / 102.
+  // (n >= 128). Faster wherever it runs, ms of 6 annealing steps against sqa_kernel: n = 150, M = R = 4 0.14 / 0.65;
+  // n = 500, M = 16, R = 64 0.41 / 2.06; n = 1000, M = 64, R = 304 1.5 / 8.7; n = 4096, M = 64, R = 4 6.3 / 26.5,
+  // R = 304 7.7 / 37.8; n = 2000, M = 64, R = 304, |J| <= 3 3.4 / 21.9; n = 6000, M = 64, R = 304 13.2 / 102.
   const int tc_sps = W + 1, tc_kp = (n + 255) / 256 * 256;  // W is a multiple of four: odd
-  const size_t tc_smem = sqa_tc_smem(M, P, tc_sps);
+  int sms = 1;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+  const SqaTc tc = sqa_tc_for(M, P, tc_sps, R, sms);
   const bool use_tc = prob->max_abs_j <= 4 && M <= 64 && n >= 128 && (long long)n * prob->max_abs_j <= 32767 &&
-                      tc_smem <= kSqaSmemBudget;
+                      tc.jstages > 0;
   // ring slots: the M rows of one iteration plus up to kSqaAhead rows ahead; the deepest ring that
   // lets two CTAs (two replicas) share an SM, else the deepest that fits one
   int S = 0;
@@ -559,8 +580,8 @@ extern "C" sb_status sb_sqa_solve(sb_ctx *ctx, const sb_problem *prob, const sb_
     where = #call;                    \
     goto cleanup;                     \
   }
-  SQ_CUDA(cudaFuncSetAttribute(use_tc ? sqa_tc_kernel_for(M, P) : sqa_kernel_for(P),
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(use_tc ? tc_smem : smem)));
+  SQ_CUDA(cudaFuncSetAttribute(use_tc ? tc.kernel : sqa_kernel_for(P),
+                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(use_tc ? tc.smem : smem)));
   SQ_CUDA(cudaEventCreate(&ev0));
   SQ_CUDA(cudaEventCreate(&ev1));
   SQ_CUDA(cudaMallocAsync((void **)&dJ, (size_t)n * n * sizeof(float), st));
@@ -614,8 +635,10 @@ extern "C" sb_status sb_sqa_solve(sb_ctx *ctx, const sb_problem *prob, const sb_
       a.trace = prm->trace ? 1 : 0;
       a.chunks = tc_kp / 256;
       a.SPS = tc_sps;
+      a.R = R;
+      a.jstages = tc.jstages;
       void *args[] = {&a};
-      SQ_CUDA(cudaLaunchKernel(sqa_tc_kernel_for(M, P), dim3((unsigned)R), dim3(sqatc::kThreads), args, tc_smem, st));
+      SQ_CUDA(cudaLaunchKernel(tc.kernel, dim3((unsigned)((R + tc.nrep - 1) / tc.nrep)), dim3((unsigned)sqatc::threads(tc.nrep)), args, tc.smem, st));
       SQ_CUDA(cudaGetLastError());
     } else {
       SqaArgs a;

@@ -49,6 +49,11 @@ def _couplings(n, kind):
     (257, 65, 1, 2, "pm1"),       # above the rule: more slices than a tile holds
     (300, 40, 5, 2, "er5"),       # above the rule: |J| = 5
     (520, 48, 2, 2, "er4"),
+    # more replicas than SMs: two per thread block, the last one alone
+    (128, 64, 153, 2, "er4"),
+    (130, 1, 301, 2, "pm1"),
+    (161, 32, 153, 2, "er3"),
+    (161, 33, 154, 2, "pm1"),
 ])
 def test_blocks_match_the_oracle(ctx, n, M, R, steps, kind, mode):
     _check(ctx, _couplings(n, kind), M, R, steps, mode)
