@@ -303,7 +303,7 @@ sb_status plan_create(sb_ctx *ctx, const sb_problem *p, const sb_params *prm, sb
     const bool want = !(env && env[0] == '0');
     const int ctas = want ? sbk::plain_persist_ctas(pl->n, pl->R, pl->jp) : 0;
     if (ctas > 0) {
-      pl->words_bytes = (size_t)2 * ctas * 128;  // one 128-byte line per CTA's word
+      pl->words_bytes = (size_t)2 * ctas * 128;  // at most one 128-byte line per CTA
       PLAN_ALLOC(pl->dwords, pl->words_bytes);
     }
   }

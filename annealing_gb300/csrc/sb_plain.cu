@@ -792,9 +792,12 @@ int grid_for(size_t total) {
 // (PlainPersist). Warp w of CTA (c, r) owns row i = 16 c + w of replica r: its J row sits in the
 // lanes' registers (lane L: float4 groups g = L + 32 k, k < kPersistGroups, the order dot_chunk
 // sums in), its x, y in registers too. A dSB step needs sign(x(t)) of every spin; CTA c's 16 signs
-// travel in one 64-bit word
-// (tag t + 1 << 32 | bit w = x_i <= 0) at words[t & 1][r][c]: the tag is the flag, so one L2 round
-// trip per step moves all the data; the thread that polls a word writes its 16 signs into shared
+// travel in one 32-bit word
+// (low 16 bits of t + 1 << 16 | bit w = x_i <= 0) at words[t & 1][r][c]: the tag is the flag, so one L2
+// round trip per step moves all the data (a word holds tag t - 1 until then, 0 at first: 16 bits tell them
+// apart); a replica's words lie side by side, so a warp polls 32 of them with one 128-byte request (us per step,
+// against a 64-bit word in a line of its own: n = 500 1.26 -> 1.06, n = 1000 1.40 -> 1.20, n = 2000
+// 1.63 -> 1.41); the thread that polls a word writes its 16 signs into shared
 // memory as +-1.0, so the field sums the same products as the bSB / aSB form, which exchanges x
 // itself as sixteen tagged words per CTA. A CTA rewrites parity t & 1 with step t + 2 only after
 // every CTA has published step t + 1, which each did after reading all of step t's words.
@@ -806,13 +809,21 @@ __device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long
   asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
 }
+__device__ __forceinline__ uint32_t ld_relaxed_u32(const uint32_t *p) {
+  uint32_t v;
+  asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_relaxed_u32(uint32_t *p, uint32_t v) {
+  asm volatile("st.relaxed.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
 __device__ __forceinline__ void st_relaxed_u64(unsigned long long *p, unsigned long long v) {
   asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
 template <int VARIANT>
 __global__ void __launch_bounds__(kPersistThreads, 1) plain_persist_kernel(PlainPersist a) {
-  // dSB exchanges signs: one word per CTA (tag << 32 | 16 sign bits). bSB / aSB exchange x: the 16
+  // dSB exchanges signs: one word per CTA (tag << 16 | 16 sign bits). bSB / aSB exchange x: the 16
   // words of a CTA's line are its rows' (tag << 32 | bits of x), one written by each warp.
   constexpr bool kSigns = VARIANT == 2;
   __shared__ __align__(16) float xs[kPersistMaxJp];  // x(t) of every spin (dSB: its sign, +-1)
@@ -855,11 +866,13 @@ __global__ void __launch_bounds__(kPersistThreads, 1) plain_persist_kernel(Plain
       for (int q = 0; q < 5; ++q) wd[q] = a.rng[q * plane + k_xy];
     }
   }
-  // one 128-byte line per CTA: its store(s) and the other CTAs' polls share no line with any other
-  // CTA's words
+  // x: one 128-byte line per CTA
   constexpr int kLine = 16;                                       // words per line
   unsigned long long *wr = a.words + (size_t)r * G * kLine;      // parity 0 of replica r
   const size_t par = (size_t)a.R * G * kLine;                     // parity stride
+  // dSB: the replica's words side by side
+  const int gp = (G + 31) & ~31;
+  auto signs = [&](int t) { return reinterpret_cast<uint32_t *>(a.words) + ((size_t)(t & 1) * a.R + r) * gp; };
   // rows past n publish x = 0 (sign -1), as the per-step kernel reads padding spins
   auto publish = [&](int t) {  // x(t) or its signs, with tag t + 1
     const unsigned long long tag = (unsigned long long)(uint32_t)(t + 1) << 32;
@@ -869,24 +882,25 @@ __global__ void __launch_bounds__(kPersistThreads, 1) plain_persist_kernel(Plain
       __syncthreads();
       if (warp == 0) {
         const uint32_t b = __ballot_sync(0xffffffffu, lane < kPersistRows && sout[lane] != 0u);
-        if (lane == 0) st_relaxed_u64(line, tag | b);
+        if (lane == 0) st_relaxed_u32(signs(t) + c, ((uint32_t)(t + 1) << 16) | b);
       }
     } else {
       if (lane == 0) st_relaxed_u64(line + warp, tag | __float_as_uint(have ? x : 0.0f));
       __syncthreads();
     }
   };
-  // one word with tag t + 1 into v: a first load, then bounded polling; false when it gave up
-  auto poll = [&](const unsigned long long *src, int t, unsigned long long &v) -> bool {
-    v = ld_relaxed_u64(src);
-    if ((uint32_t)(v >> 32) == (uint32_t)(t + 1)) return true;
+  // one word of signs with tag t + 1 into v: a first load, then bounded polling; false when it gave up
+  auto poll = [&](const uint32_t *src, int t, uint32_t &v) -> bool {
+    const uint32_t want = (uint32_t)(t + 1) & 0xFFFFu;
+    v = ld_relaxed_u32(src);
+    if (v >> 16 == want) return true;
     const long long t0 = clock64();
     int spins = 0;
     do {
       if (++spins > 8) __nanosleep(32);
-      v = ld_relaxed_u64(src);
+      v = ld_relaxed_u32(src);
       if (clock64() - t0 > ptx::kWaitCycles) return false;
-    } while ((uint32_t)(v >> 32) != (uint32_t)(t + 1));
+    } while (v >> 16 != want);
     return true;
   };
   // x(t) of every spin into xs (dSB: the signs as +-1.0); false when a wait gave up
@@ -894,10 +908,8 @@ __global__ void __launch_bounds__(kPersistThreads, 1) plain_persist_kernel(Plain
     if constexpr (kSigns) {
       // thread q < G polls CTA q's word and writes its 16 signs (bit w set: spin 16 q + w is -1)
       if (tid >= G) return true;
-      const unsigned long long *src = wr + (size_t)(t & 1) * par + (size_t)tid * kLine;
-      unsigned long long v;
-      if (!poll(src, t, v)) return false;
-      const uint32_t b = (uint32_t)v;
+      uint32_t b;
+      if (!poll(signs(t) + tid, t, b)) return false;
       float4 *dst = reinterpret_cast<float4 *>(xs) + 4 * tid;
 #pragma unroll
       for (int k = 0; k < 4; ++k)
