@@ -54,6 +54,8 @@ struct sb_plan {
   // plain FP32 SB that fits one cooperative launch: the exchange lines of PlainPersist
   unsigned long long *dwords = nullptr;
   size_t words_bytes = 0;
+  uint32_t *dplanes = nullptr;  // dSB with small integer couplings: their bit planes, and how many magnitudes
+  int planes = 0;               // they have (0: the couplings uploaded are not such)
   float *dxk = nullptr;    // [kTopK][xp] rows of the best candidates (real-valued J)
   double *dek = nullptr;   // [kTopK] their FP64 energies
   // compact copy of integer couplings for the host re-check, built on a background thread while
@@ -204,6 +206,8 @@ void plan_free_device(sb_plan *pl) {
   cudaFree(pl->dxk);
   cudaFree(pl->dek);
   cudaFree(pl->dwords);
+  cudaFree(pl->dplanes);
+  pl->dplanes = nullptr;
   pl->dwords = nullptr;
   pl->dpump = nullptr;
   pl->dxk = nullptr;
@@ -217,6 +221,9 @@ void plan_free_device(sb_plan *pl) {
   pl->dstatus = nullptr;
   pl->ev0 = pl->ev1 = nullptr;
 }
+
+// The plain FP32 steps of a solve run in one launch.
+bool one_launch(const sb_plan *pl) { return pl->planes || pl->dwords; }
 
 bool needs_trace(const sb_params &p) { return p.trace || p.trace_all; }
 
@@ -239,6 +246,10 @@ sb_status upload_problem(sb_plan *pl, const sb_problem *p, std::string &err) {
       sb_status ts = sbk::tc_create(&pl->tc, s, pl->dJ, pl->jp, err, st);
       if (ts != SB_OK) return ts;
     }
+  }
+  if (pl->dplanes) {
+    pl->planes = p->integer_valued ? sbk::sign_planes(n, pl->R, p->max_abs_j) : 0;
+    if (pl->planes) SB_CUDA(sbk::launch_sign_planes(pl->dJ, n, pl->jp, pl->planes, pl->dplanes, st));
   }
   pl->copies.reset();
   pl->prob = p;
@@ -301,6 +312,9 @@ sb_status plan_create(sb_ctx *ctx, const sb_problem *p, const sb_params *prm, sb
   if (mode == SB_FIELD_FP32 && !needs_trace(*prm) && prm->steps > 0) {
     const char *env = getenv("SB_PLAIN_PERSIST");
     const bool want = !(env && env[0] == '0');
+    // dSB with couplings up to 3 or 7: no exchange through L2 at all (sb_signs.cuh)
+    if (want && prm->variant == SB_DSB && p->integer_valued && sbk::sign_planes(pl->n, pl->R, p->max_abs_j))
+      PLAN_ALLOC(pl->dplanes, sbk::sign_plane_bytes(pl->n));
     const int ctas = want ? sbk::plain_persist_ctas(pl->n, pl->R, pl->jp) : 0;
     if (ctas > 0) {
       pl->words_bytes = (size_t)2 * ctas * 128;  // at most one 128-byte line per CTA
@@ -372,6 +386,34 @@ cudaError_t enqueue_loop(sb_plan *pl, cudaStream_t st, std::vector<cudaEvent_t> 
       if (evs) cudaEventRecord((*evs)[0], st);
       cudaError_t e = sbk::tc_run(pl->tc, p.steps, pl->dpump, pl->dx[0], pl->dy, pl->dh, pl->c0, p.dt,
                                   pl->dta0, tr ? pl->denergy : nullptr, pl->dstatus, st);
+      if (e != cudaSuccess) return e;
+      if (evs) cudaEventRecord((*evs)[1], st);
+      nl = 1;
+    }
+    if (launches) *launches = nl;
+    return cudaSuccess;
+  }
+  if (pl->planes) {
+    if (p.steps > 0) {
+      sbk::SignSolve a;
+      memset(&a, 0, sizeof(a));
+      a.n = pl->n;
+      a.R = R;
+      a.xp = pl->xp;
+      a.words = (pl->n + 31) / 32;
+      a.planes = pl->dplanes;
+      a.h = pl->dh;
+      a.x_in = pl->dx[0];
+      a.x_out = pl->dx[p.steps & 1];
+      a.y = pl->dy;
+      a.pumps = pl->dpump;
+      a.c0 = pl->c0;
+      a.dt = p.dt;
+      a.dta0 = pl->dta0;
+      a.steps = p.steps;
+      a.status = pl->dstatus;
+      if (evs) cudaEventRecord((*evs)[0], st);
+      const cudaError_t e = sbk::launch_signs(a, pl->planes, st);
       if (e != cudaSuccess) return e;
       if (evs) cudaEventRecord((*evs)[1], st);
       nl = 1;
@@ -504,7 +546,7 @@ sb_status plan_run(sb_plan *pl, uint64_t seed, sb_result *res, std::string &err)
   }
   double kernel_ms = 0.0;
   if (p.profile) {
-    const int nmeas = (pl->mode == SB_FIELD_TC || pl->dwords) ? (p.steps > 0 ? 1 : 0) : p.steps;
+    const int nmeas = (pl->mode == SB_FIELD_TC || one_launch(pl)) ? (p.steps > 0 ? 1 : 0) : p.steps;
     std::vector<cudaEvent_t> evs((size_t)2 * (nmeas > 0 ? nmeas : 1));
     for (auto &ev : evs) SB_CUDA(cudaEventCreate(&ev));
     int64_t nl = 0;
@@ -522,7 +564,7 @@ sb_status plan_run(sb_plan *pl, uint64_t seed, sb_result *res, std::string &err)
     }
     if (nmeas > 0) kernel_ms /= nmeas;
     launches += nl;
-  } else if (p.steps > 0 && (pl->mode == SB_FIELD_TC || pl->dwords)) {
+  } else if (p.steps > 0 && (pl->mode == SB_FIELD_TC || one_launch(pl))) {
     int64_t nl = 0;
     SB_CUDA(enqueue_loop(pl, st, nullptr, &nl));
     launches += nl;
@@ -660,7 +702,7 @@ sb_status plan_run(sb_plan *pl, uint64_t seed, sb_result *res, std::string &err)
   }
   res->device_ms = dev_ms;
   res->kernel_ms_avg = kernel_ms;
-  res->steps_per_launch = (pl->mode == SB_FIELD_TC || pl->dwords) ? p.steps : 1;
+  res->steps_per_launch = (pl->mode == SB_FIELD_TC || one_launch(pl)) ? p.steps : 1;
   res->kernel_launches = launches;
   res->total_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_start).count();
   res->spin_updates_per_s =

@@ -81,6 +81,26 @@ constexpr int kPersistMaxJp = 2048;
 int plain_persist_ctas(int n, int R, int jp);
 cudaError_t launch_plain_persist(const PlainPersist &a, cudaStream_t st);
 
+// Plain FP32 dSB with small integer couplings, the whole solve in one launch of independent clusters (sb_signs.cuh).
+struct SignSolve {
+  int n, R, xp, words;        // words = ceil(n / 32)
+  const uint32_t *planes;     // [P + 1][words][n] from launch_sign_planes
+  const float *h;             // [n] or null
+  const float *x_in;          // x(0) [R][xp]
+  float *x_out, *y;           // x(steps), y in place
+  const float *pumps;         // [steps] a0 - a(t)
+  float c0, dt, dta0;
+  int steps;
+  uint32_t *status;
+};
+constexpr int kSignsMaxN = 2048;
+constexpr int kSignsOneCta = 512;  // spins of the one-CTA form with one magnitude plane
+// Magnitude planes of the one-launch sign kernel for couplings up to max_abs_j, or 0 when it does not take the shape.
+int sign_planes(int n, int R, int max_abs_j);
+size_t sign_plane_bytes(int n);  // for any couplings that n allows
+cudaError_t launch_sign_planes(const float *J, int n, int jp, int P, uint32_t *planes, cudaStream_t st);
+cudaError_t launch_signs(const SignSolve &a, int P, cudaStream_t st);
+
 struct PlainEnergy {
   int n, R, jp, xp, rb;
   const float *J, *h;

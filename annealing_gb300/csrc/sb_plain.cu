@@ -1029,6 +1029,8 @@ __global__ void __launch_bounds__(kPersistThreads, 1) plain_persist_kernel(Plain
   }
 }
 
+#include "sb_signs.cuh"
+
 }  // namespace
 
 template <typename K>
@@ -1185,6 +1187,66 @@ cudaError_t launch_plain_persist(const PlainPersist &a, cudaStream_t st) {
     case 3: return cudaLaunchKernelEx(&cfg, plain_persist_kernel<3>, a);
   }
   return cudaErrorInvalidValue;
+}
+
+namespace {
+const void *signs_kernel_for(int n, int P) {
+  return P == 1 ? signs::kernel_for<1>(n) : P == 2 ? signs::kernel_for<2>(n) : signs::kernel_for<3>(n);
+}
+// Launch shape for R solves of n spins.
+void signs_config(int n, int R, int P, cudaLaunchConfig_t &cfg, cudaLaunchAttribute &attr) {
+  memset(&cfg, 0, sizeof(cfg));
+  memset(&attr, 0, sizeof(attr));
+  const bool one = signs::one_cta(n, P);
+  const int C = one ? 1 : (n + signs::kClusterRows - 1) / signs::kClusterRows;
+  cfg.gridDim = dim3((unsigned)C, (unsigned)R);
+  cfg.blockDim = dim3((unsigned)(one ? (n + 31) / 32 * 32 : signs::kClusterRows));
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = (unsigned)C;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = one ? 0 : 1;
+}
+}  // namespace
+
+int sign_planes(int n, int R, int max_abs_j) {
+  if (n < 1 || n > kSignsMaxN || R < 1 || R > 65535 || max_abs_j > 7) return 0;
+  const int P = max_abs_j <= 1 ? 1 : max_abs_j <= 3 ? 2 : 3;
+  const void *k = signs_kernel_for(n, P);
+  if (!k) return 0;  // more planes than registers hold
+  if (signs::one_cta(n, P)) return P;
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute attr;
+  signs_config(n, R, P, cfg, attr);
+  int clusters = 0;  // more than eight CTAs to a cluster need the attribute, and SMs of one GPC free for them
+  if (cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&clusters, k, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return clusters > 0 ? P : 0;
+}
+
+size_t sign_plane_bytes(int n) {
+  const size_t words = (size_t)(n + 31) / 32;
+  return (words <= 32 ? 4 : 2) * words * n * sizeof(uint32_t);
+}
+
+cudaError_t launch_sign_planes(const float *J, int n, int jp, int P, uint32_t *planes, cudaStream_t st) {
+  const int words = (n + 31) / 32;
+  const long long threads = 32ll * n * words;
+  signs::sign_planes_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(J, n, jp, words, P, planes);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_signs(const SignSolve &a, int P, cudaStream_t st) {
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute attr;
+  signs_config(a.n, a.R, P, cfg, attr);
+  cfg.stream = st;
+  SignSolve v = a;
+  void *args[] = {&v};
+  return cudaLaunchKernelExC(&cfg, signs_kernel_for(a.n, P), args);
 }
 
 cudaError_t launch_plain_energy(const PlainEnergy &a0, bool fp64, cudaStream_t st) {
