@@ -53,8 +53,8 @@ namespace sbk {
 // in its own translation unit (sb_tc_fp8.cu, sb_tc_bf16.cu, sb_tc_split.cu).
 bool tc_kernel_fp8(int variant, int nr, int emode, const void **k, size_t *smem);
 bool tc_kernel_bf16(int variant, int nr, int emode, const void **k, size_t *smem);
-bool tc_kernel_split(int variant, int nr, int emode, const void **k, size_t *smem);
-bool tc_kernel_split16(int variant, int nr, int emode, const void **k, size_t *smem);
+bool tc_kernel_split(int variant, int nr, int emode, const void **k, size_t *smem, bool pair = false);
+bool tc_kernel_split16(int variant, int nr, int emode, const void **k, size_t *smem, bool pair = false);
 bool tc_kernel_fp4(int variant, int nr, int emode, int k_chunks, const void **k, size_t *smem, bool pair = false);
 
 namespace {
@@ -217,7 +217,8 @@ struct TcEngine {
   const void *kernel[3] = {nullptr, nullptr, nullptr};  // by epilogue mode
   size_t smem = 0;
   int threads = kTcThreads;
-  bool pair = false;  // E2M1 kernel in CTA pairs (clusters of two, launched with that attribute)
+  bool pair = false;  // kernel in CTA pairs (clusters of two, launched with that attribute)
+  CUtensorMap tmE;    // V operand buffer 0, part 0, whole replica tiles (the energy contraction)
   float jscale = 1.0f, jinv = 1.0f;  // FP16 hi + lo: the coupling scale (a power of two) and its inverse
   int flag_stride = 1;  // words between consecutive units' step flags
   // E2M1 solves without a trace run in the multi-step kernel with tagged sign words (sb_run.cuh)
@@ -236,18 +237,18 @@ namespace {
 int kp_for(int dt, int n) { return dt == kTcFp4 ? (n + 255) / 256 * 256 : (n + 127) / 128 * 128; }
 
 bool pick(TcEngine *e, int dt, int variant, int nr, int n, bool pair = false) {
-  size_t smem = 0;
   for (int m = 0; m < 3; ++m) {
+    size_t smem = 0;
     const void *k = nullptr;
     bool ok;
     if (dt == kTcFp4) ok = tc_kernel_fp4(variant, nr, m, kp_for(dt, n) / 256, &k, &smem, pair);
     else if (dt == kTcFp8) ok = tc_kernel_fp8(variant, nr, m, &k, &smem);
     else if (dt == kTcBf16) ok = tc_kernel_bf16(variant, nr, m, &k, &smem);
-    else if (dt == kTcFp16Split) ok = tc_kernel_split16(variant, nr, m, &k, &smem);
-    else ok = tc_kernel_split(variant, nr, m, &k, &smem);
+    else if (dt == kTcFp16Split) ok = tc_kernel_split16(variant, nr, m, &k, &smem, pair);
+    else ok = tc_kernel_split(variant, nr, m, &k, &smem, pair);
     e->kernel[m] = ok ? k : nullptr;
+    if (ok) e->smem = smem;
   }
-  e->smem = smem;
   return e->kernel[kEmodeStep] != nullptr;
 }
 
@@ -338,6 +339,7 @@ const char *bind(TcEngine *e, cudaError_t *ce) {
         return "cuTensorMapEncodeTiled(V)";
       g.v[b][pp] = e->v[b][pp];
     }
+  if (!encode_2d(&e->tmE, e->v[0][0], elem, rowe, (uint64_t)e->Rp, vrows)) return "cuTensorMapEncodeTiled(V)";
   // the unit's V tile: 128 spins = 128 elements, or 64 bytes of E2M1 pairs
   for (int b = 0; b < 2; ++b)
     if (!encode_2d(&g.tmS[b], e->v[b][0], elem, rowe, (uint64_t)e->Rp, vrows, true, fp4 ? kBM / 2 : kBM))
@@ -432,25 +434,35 @@ sb_status run_create(TcEngine *e, cudaStream_t st, cudaError_t *ce) {
 }  // namespace
 
 namespace {
-// The CTA-pair E2M1 kernel runs this dSB shape when asked for (SB_TC_PAIR=1): the 128-replica
-// tile, its units (spin tiles rounded up to an even count) on distinct SMs, every pair co-resident
-// as a cluster of two. It is bit-identical to the single-CTA kernel and measured slower on the
-// batched dSB workload, so the single-CTA kernel is the default.
+// The CTA-pair kernels: the 128-replica tile, units on distinct SMs, every pair co-resident as a cluster of two.
+// SB_TC_PAIR=0 / 1 decides, else:
+//   * E2M1 dSB (spin tiles rounded up to an even count): never; bit-identical to the single-CTA kernel and measured
+//     slower on the batched dSB workload.
+//   * bSB with BF16 hi + lo operands from six spin tiles on, an even count of them (so the operands take no more
+//     memory). Bit-identical to the single-CTA kernel, us per step against it: n = 500 R = 100 13.1 / 12.4,
+//     n = 1000 R = 128 16.4 / 17.2, n = 2000 R = 256 24.8 / 27.4, n = 4096 42.9 / 51.9, n = 8192 95 / 114. FP16
+//     hi + lo segments are too short (two chunks): n = 1000 20.4 / 18.5, n = 8192 132 / 121.
 bool pair_fits(const TcSetup &s, int nr, int sms) {
-  if (s.dtype != kTcFp4 || s.variant != 2 || nr != 128) return false;
+  const bool fp4 = s.dtype == kTcFp4 && s.variant == 2, split = tc_split(s.dtype) && s.variant == 1;
+  if (!(fp4 || split) || nr != 128) return false;
+  const int tiles = (s.n + kBM - 1) / kBM;
   const char *v = getenv("SB_TC_PAIR");
-  if (!v || v[0] != '1') return false;
-  const int mt = (s.n + 2 * kBM - 1) / (2 * kBM) * 2;
+  if (v ? v[0] != '1' : fp4 || s.dtype == kTcFp16Split || tiles < 6) return false;
+  if (split && tiles % 2 != 0) return false;
+  const int mt = (tiles + 1) / 2 * 2;
   const int units = mt * ((s.R + nr - 1) / nr);
   if (units > sms) return false;
   const void *k = nullptr;
   size_t smem = 0;
-  if (!tc_kernel_fp4(2, nr, kEmodeStep, kp_for(kTcFp4, s.n) / 256, &k, &smem, true)) return false;
+  const bool have = fp4                        ? tc_kernel_fp4(2, nr, kEmodeStep, kp_for(kTcFp4, s.n) / 256, &k, &smem, true)
+                    : s.dtype == kTcFp16Split ? tc_kernel_split16(1, nr, kEmodeStep, &k, &smem, true)
+                                              : tc_kernel_split(1, nr, kEmodeStep, &k, &smem, true);
+  if (!have) return false;
   if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return false;
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3((unsigned)units);
-  cfg.blockDim = dim3((unsigned)kFp4Threads);
+  cfg.blockDim = dim3((unsigned)(fp4 ? kFp4Threads : kTcThreads));
   cfg.dynamicSmemBytes = smem;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -733,6 +745,7 @@ cudaError_t tc_energy_signs(TcEngine *e, const float *x, const float *h, double 
                                                                       e->Kp, e->s.dtype, 2, 1.0f);
   if ((ce = cudaGetLastError()) != cudaSuccess) return ce;
   TcArgs a = e->args;
+  a.tmB[0][0] = e->tmE;
   a.x = const_cast<float *>(x);
   a.y = nullptr;
   a.h = h;

@@ -217,17 +217,24 @@ __device__ __forceinline__ bool wait_flag(const uint32_t *flag, uint32_t target,
 // flags[rt][chunk's unit] >= t before loading that chunk. Those same flags also order the reuse of
 // the ping-pong operand buffer (a unit overwrites V(t+1)'s buffer only after consuming all of V(t),
 // i.e. after every reader of V(t-1)'s chunk finished its step t-1 contraction).
-template <int DT, int VARIANT, int NR, int STAGES, int EMODE>
+// PAIR (a cluster of two CTAs, spin tiles 2 k and 2 k + 1; split bSB, 128 replicas): one M = 256 MMA works both
+// tiles' rows against the replicas, of which each CTA stages half, so a chunk costs a CTA's shared memory 48 KB of
+// copies and 72 KB of operand reads instead of 64 and 96. The first CTA (rank 0) issues the MMAs and owns the
+// barriers that both CTAs' copies (full_bar) and epilogues (acce_bar) complete; its commits arrive on both CTAs'
+// barriers. Both CTAs meet at a cluster barrier before freeing tensor memory and exiting.
+template <int DT, int VARIANT, int NR, int STAGES, int EMODE, bool PAIR = false>
 __global__ void __launch_bounds__(kTcThreads, 1) tc_sb_kernel(const __grid_constant__ TcArgs p) {
   using C = Cfg<DT, VARIANT>;
   constexpr int kATile = kBM * kChunkBytes;  // bytes per A part per stage
-  constexpr int kBTile = NR * kChunkBytes;   // bytes per B part per stage
+  constexpr int kBRows = PAIR ? NR / 2 : NR; // replicas staged by this CTA
+  constexpr int kBTile = kBRows * kChunkBytes;  // bytes per B part per stage
+  static_assert(!PAIR || (C::kBParts == 2 && VARIANT == 1 && NR == 128 && EMODE == kEmodeStep), "the pair form");
   constexpr int kStage = C::kAParts * kATile + C::kBParts * kBTile;
   // Single-part operands (FP8 / BF16 signs) leave the epilogue through a shared-memory tile and one
   // TMA store per unit per step; split operands are stored element by element.
   constexpr bool kStageV = C::kBParts == 1;
   constexpr int kVRow = kBM * C::kElem;      // bytes of one replica row of the unit's V tile
-  constexpr uint32_t kTx = (uint32_t)kStage;
+  constexpr uint32_t kTx = (uint32_t)(PAIR ? 2 * kStage : kStage);  // both CTAs' copies
   // NMFA draws stage k+1's noise pair ahead, in the idle time after stage k's sweeps publish (the
   // first chunk of a thread's columns after the first sweep, the rest after the second), when three
   // more column blocks fit TMEM (z0, and z1 alternating between y and y1 by stage parity);
@@ -235,14 +242,16 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_sb_kernel(const __grid_const
   constexpr bool kNoiseAhead = VARIANT == 3 && 6 * NR <= 512;
   constexpr int kUsedCols = kNoiseAhead ? 6 * NR : 4 * NR;
   constexpr uint32_t kCols = kUsedCols <= 32 ? 32 : (kUsedCols <= 64 ? 64 : (kUsedCols <= 128 ? 128 : (kUsedCols <= 256 ? 256 : 512)));
-  constexpr uint32_t kIdesc = make_idesc(DT, kBM, NR);
+  constexpr uint32_t kIdesc = make_idesc(DT, PAIR ? 2 * kBM : kBM, NR);
   constexpr int kHalf = NR / 2;               // columns per epilogue warp
   // Split couplings (BF16 hi + lo, real-valued J): the tensor core rounds the sum of each MMA into
   // its FP32 accumulator toward zero, a bias that grows with the number of MMAs one accumulator
   // takes and with its magnitude. So the contraction over K runs in segments of p.seg_chunks chunks,
-  // each into a fresh accumulator (column block 0), and the epilogue warps, idle during the
-  // contraction, load each finished segment (the MMA lane waits only for that load) and add it into
-  // a running FP32 sum (round to nearest; column block 1). x and y keep blocks 2 and 3.
+  // each into a fresh accumulator, and the epilogue warps, idle during the contraction, load each finished
+  // segment and add it into a running FP32 sum (round to nearest). x and y keep column blocks 2 and 3. One CTA
+  // is bound by its shared memory: the segments take block 0 (the MMA warp waits only for its load) and the sum
+  // block 1. A pair is not, and waited for those loads 18 % of a step at eight chunks a segment: its segments take
+  // blocks 0 and 1 in turn and the sum stays in registers (in one CTA that order cost 5 to 9 % at small sizes).
   constexpr bool kSeg = tc_split(DT);
   // FP16 hi + lo: the accumulated field is scaled back by an exact power of two
   const float fscale = DT == kTcFp16Split ? (C::kBParts == 2 ? p.jinv / p.xscale : p.jinv) : 1.0f;
@@ -263,6 +272,15 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_sb_kernel(const __grid_const
   const int nsteps = kEOnly ? 1 : p.steps;
   uint32_t *col_flags = p.flags + (size_t)rt * p.n_mtiles * p.flag_stride;
   bool ok = true;
+  const uint32_t crank = PAIR ? ptx::cluster_rank() : 0u;  // 0: the pair's MMA issuer
+  const bool issuer = crank == 0;
+  // a wait on a barrier that the peer's arrivals or copies may complete
+  auto wait = [&](uint64_t *bar, uint32_t parity) {
+    return PAIR ? ptx::mbar_wait_cluster(bar, parity, p.wait_cycles) : ptx::mbar_wait(bar, parity, p.wait_cycles);
+  };
+  auto wait_spin = [&](uint64_t *bar, uint32_t parity) {
+    return PAIR ? ptx::mbar_wait_cluster_spin(bar, parity, p.wait_cycles) : ptx::mbar_wait_spin(bar, parity, p.wait_cycles);
+  };
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -271,7 +289,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_sb_kernel(const __grid_const
     }
     for (int b = 0; b < 2; ++b) {
       ptx::mbar_init(&accf_bar[b], 1);
-      ptx::mbar_init(&acce_bar[b], kEpiWarps);
+      ptx::mbar_init(&acce_bar[b], PAIR ? 2 * kEpiWarps : kEpiWarps);
     }
     ptx::mbar_init(&drain_bar, 1);
     ptx::fence_mbar_init();
@@ -282,17 +300,25 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_sb_kernel(const __grid_const
     }
   }
   if (warp == 1) {
-    ptx::tmem_alloc(&tmem_base_sh, kCols);
-    ptx::tmem_relinquish();
+    if constexpr (PAIR) {
+      ptx::tmem_alloc_pair(&tmem_base_sh, kCols);
+      ptx::tmem_relinquish_pair();
+    } else {
+      ptx::tmem_alloc(&tmem_base_sh, kCols);
+      ptx::tmem_relinquish();
+    }
   }
   ptx::tc_fence_before();
-  __syncthreads();
+  if constexpr (PAIR)
+    ptx::cluster_sync();  // both CTAs' barriers initialised
+  else
+    __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem = tmem_base_sh;
   // columns: accumulators [0, NR) and [NR, 2NR), x [2NR, 3NR), y [3NR, 4NR); NMFA with the noise
   // drawn ahead: z0 [4NR, 5NR), y1 [5NR, 6NR) (stage k's z1 in y for even k, in y1 for odd k)
   const uint32_t t_x = tmem + 2 * NR, t_y = tmem + 3 * NR, t_z0 = tmem + 4 * NR, t_y1 = tmem + 5 * NR;
-  const uint32_t t_sum = tmem + NR;  // split operands: the running sum of the segments
+  const uint32_t t_sum = tmem + NR;  // split operands, one CTA: the running sum of the segments
   const int nseg = kSeg ? (p.k_chunks + p.seg_chunks - 1) / p.seg_chunks : 1;
 
   if (warp == 0) {
@@ -306,12 +332,16 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_sb_kernel(const __grid_const
     auto load_j = [&](uint32_t gg, int kx) -> bool {
       const int s = gg % STAGES;
       const uint32_t use = gg / STAGES;
-      if (use > 0 && !__all_sync(0xffffffffu, ptx::mbar_wait(&empty_bar[s], (use - 1) & 1, p.wait_cycles))) return false;
+      if (use > 0 && !__all_sync(0xffffffffu, wait(&empty_bar[s], (use - 1) & 1))) return false;
       if (ptx::elect_one()) {
-        ptx::mbar_arrive_expect_tx(&full_bar[s], kTx);
+        if (issuer) ptx::mbar_arrive_expect_tx(&full_bar[s], kTx);
 #pragma unroll
-        for (int a = 0; a < C::kAParts; ++a)
-          ptx::tma_load_2d(smem + s * kStage + a * kATile, &p.tmA[a], kx, m0, &full_bar[s]);
+        for (int a = 0; a < C::kAParts; ++a) {
+          if constexpr (PAIR)
+            ptx::tma_load_2d_pair(smem + s * kStage + a * kATile, &p.tmA[a], kx, m0, ptx::mapa(ptx::smem_u32(&full_bar[s]), 0));
+          else
+            ptx::tma_load_2d(smem + s * kStage + a * kATile, &p.tmA[a], kx, m0, &full_bar[s]);
+        }
       }
       __syncwarp();
       armed = gg + 1;
@@ -335,8 +365,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_sb_kernel(const __grid_const
         if (ptx::elect_one()) {
           const int s = g % STAGES;
 #pragma unroll
-          for (int b = 0; b < C::kBParts; ++b)
-            ptx::tma_load_2d(smem + s * kStage + C::kAParts * kATile + b * kBTile, &p.tmB[buf][b], kx, r0, &full_bar[s]);
+          for (int b = 0; b < C::kBParts; ++b) {
+            uint8_t *dst = smem + s * kStage + C::kAParts * kATile + b * kBTile;
+            if constexpr (PAIR)
+              ptx::tma_load_2d_pair(dst, &p.tmB[buf][b], kx, r0 + (int)crank * kBRows,
+                                    ptx::mapa(ptx::smem_u32(&full_bar[s]), 0));
+            else
+              ptx::tma_load_2d(dst, &p.tmB[buf][b], kx, r0, &full_bar[s]);
+          }
         }
         __syncwarp();
       }
@@ -351,11 +387,18 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_sb_kernel(const __grid_const
       // a wait gave up: let the copies this CTA started land before it exits (each stage's last
       // armed use; a use whose J part alone was started never completes its phase, and the
       // bounded wait then outlasts those loads)
-      for (int s = 0; s < STAGES; ++s)
-        if (armed > (uint32_t)s) ptx::mbar_wait(&full_bar[s], ((armed - 1 - s) / STAGES) & 1, p.wait_cycles);
+      if constexpr (PAIR) {
+        // this CTA's copies complete barriers of the issuer, which the second CTA cannot wait on: a bounded
+        // pause far longer than any copy, then the issuer's own bounded waits
+        const long long t0 = clock64();
+        while (clock64() - t0 < (p.wait_cycles < 2000000LL ? p.wait_cycles : 2000000LL)) __nanosleep(1000);
+      }
+      if (issuer)
+        for (int s = 0; s < STAGES; ++s)
+          if (armed > (uint32_t)s) wait(&full_bar[s], ((armed - 1 - s) / STAGES) & 1);
     }
   } else if (warp == 1) {
-    // ---------------- MMA issuer (the whole warp; elect_one issues) ----------------
+    // ---------------- MMA issuer (the whole warp; elect_one issues; a pair's first CTA) ----------------
     int s = 0;
     uint32_t ph = 0;
     uint32_t gs = 0;    // split operands: segments issued
@@ -363,7 +406,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_sb_kernel(const __grid_const
     // a stage's descriptors differ from stage 0's in the address field (units of 16 bytes) alone
     const uint64_t ad0 = ptx::smem_desc_sw128(ptx::smem_u32(smem));
     const uint64_t bd0 = ptx::smem_desc_sw128(ptx::smem_u32(smem) + C::kAParts * kATile);
-    for (int ls = 0; ls < nsteps && ok; ++ls) {
+    for (int ls = 0; ls < nsteps && ok && issuer; ++ls) {
       const int ab = ls & 1;
       if constexpr (!kSeg) {
         if (ls >= 2 && !__all_sync(0xffffffffu, ptx::mbar_wait(&acce_bar[ab], (uint32_t)((ls >> 1) - 1) & 1, p.wait_cycles))) {
@@ -374,16 +417,18 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_sb_kernel(const __grid_const
       }
       int kin = 0;  // chunk index inside the current segment
       for (int kc = 0; kc < p.k_chunks; ++kc) {
-        const uint32_t t_acc = tmem + (kSeg ? 0 : ab) * NR;
+        const uint32_t t_acc = tmem + (PAIR ? (gs & 1) : kSeg ? 0 : ab) * NR;
         if (kSeg && kin == 0) {
-          // the segment block is free once the epilogue has loaded the previous segment
-          if (gs >= 1 && !__all_sync(0xffffffffu, ptx::mbar_wait_spin(&acce_bar[0], (uint32_t)(gs - 1) & 1, p.wait_cycles))) {
+          // the segment's block is free once the epilogue has loaded the segment before it there
+          const bool freed = PAIR ? gs < 2 || wait_spin(&acce_bar[gs & 1], ((gs >> 1) - 1) & 1)
+                                  : gs < 1 || wait_spin(&acce_bar[0], (gs - 1) & 1);
+          if (!__all_sync(0xffffffffu, freed)) {
             ok = false;
             break;
           }
           ptx::tc_fence_after();
         }
-        if (!have && !__all_sync(0xffffffffu, ptx::mbar_wait(&full_bar[s], ph, p.wait_cycles))) {
+        if (!have && !__all_sync(0xffffffffu, wait(&full_bar[s], ph))) {
           ok = false;
           break;
         }
@@ -392,7 +437,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_sb_kernel(const __grid_const
           s = 0;
           ph ^= 1;
         }
-        const bool next = ptx::mbar_test(&full_bar[s], ph);  // looked at while the MMAs below issue
+        // looked at while the MMAs below issue
+        const bool next = PAIR ? ptx::mbar_test_cluster(&full_bar[s], ph) : ptx::mbar_test(&full_bar[s], ph);
         const bool seg_end = kSeg && (kin + 1 == p.seg_chunks || kc + 1 == p.k_chunks);
         if (ptx::elect_one()) {
           const uint64_t off = (uint64_t)(cur * (kStage / 16));
@@ -405,15 +451,23 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_sb_kernel(const __grid_const
               for (int k = 0; k < C::kMmaPerChunk; ++k) {
                 const uint64_t ad = ad0 + off + a * (kATile / 16) + 2 * k, bd = bd0 + off + b * (kBTile / 16) + 2 * k;
                 const uint32_t acc = ((kSeg ? kin : kc) > 0 || a + b > 0 || k > 0) ? 1u : 0u;
-                if constexpr (DT == kTcFp8)
+                if constexpr (PAIR)
+                  ptx::mma_f16_pair(t_acc, ad, bd, kIdesc, acc);
+                else if constexpr (DT == kTcFp8)
                   ptx::mma_f8(t_acc, ad, bd, kIdesc, acc);
                 else
                   ptx::mma_f16(t_acc, ad, bd, kIdesc, acc);
               }
             }
           }
-          ptx::mma_commit(&empty_bar[cur]);
-          if (kSeg ? seg_end : kc + 1 == p.k_chunks) ptx::mma_commit(&accf_bar[kSeg ? 0 : ab]);
+          auto commit = [&](uint64_t *bar) {
+            if constexpr (PAIR)
+              ptx::mma_commit_pair(bar);
+            else
+              ptx::mma_commit(bar);
+          };
+          commit(&empty_bar[cur]);
+          if (kSeg ? seg_end : kc + 1 == p.k_chunks) commit(&accf_bar[PAIR ? (gs & 1) : kSeg ? 0 : ab]);
         }
         __syncwarp();
         have = __all_sync(0xffffffffu, next);
@@ -423,7 +477,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_sb_kernel(const __grid_const
         }
       }
     }
-    if (!ok) {
+    if constexpr (PAIR) {
+      // both CTAs wait on drain_bar before freeing tensor memory: the MMAs issued are done
+      if (issuer) {
+        if (ptx::elect_one()) ptx::mma_commit_pair(&drain_bar);
+        __syncwarp();
+        wait(&drain_bar, 0);
+      }
+    } else if (!ok) {
       // a wait gave up: the MMAs already issued finish before TMEM is freed
       if (ptx::elect_one()) ptx::mma_commit(&drain_bar);
       __syncwarp();
@@ -498,7 +559,58 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_sb_kernel(const __grid_const
     for (int ls = 0; ls < nsteps; ++ls) {
       const int t = p.t0 + ls;
       const int buf = (p.buf0 + ls) & 1;
-      if constexpr (kSeg) {
+      auto release = [&](uint32_t blk) {  // the accumulator block may be overwritten
+        ptx::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          if constexpr (PAIR)
+            ptx::mbar_arrive_cluster(ptx::mapa(ptx::smem_u32(&acce_bar[blk]), 0));
+          else
+            ptx::mbar_arrive(&acce_bar[blk]);
+        }
+      };
+      uint32_t ab = ls & 1;  // accumulator block holding the field
+      if constexpr (PAIR) {
+        // every segment: load it (then the MMA warp may start the next but one into the same block) and add it
+        // into the sum, which goes back into the last one's block; a single segment stays where it is
+        float sum[kHalf];
+        bool seg_ok = true;
+        for (int sg = 0; sg < nseg; ++sg, ++gs) {
+          ab = gs & 1;
+          const bool got_s = wait_spin(&accf_bar[ab], (gs >> 1) & 1);
+          if (!epi_all(got_s)) { seg_ok = false; break; }
+          ptx::tc_fence_after();
+          if (nseg == 1) continue;
+          constexpr int kLoad = kHalf < 32 ? kHalf : 32;  // columns in flight
+#pragma unroll
+          for (int h = 0; h < kHalf; h += kLoad) {
+            uint32_t va[kLoad];
+#pragma unroll
+            for (int i = 0; i < kLoad / 16; ++i)
+              ptx::tmem_ld16(tmem + ab * NR + lane_off + c_lo + h + 16 * i, *reinterpret_cast<uint32_t(*)[16]>(va + 16 * i));
+            ptx::tmem_ld_wait();
+            if (h + kLoad == kHalf && sg + 1 < nseg) release(ab);
+            if (sg == 0) {
+#pragma unroll
+              for (int j = 0; j < kLoad; ++j) sum[h + j] = __uint_as_float(va[j]);
+            } else {
+#pragma unroll
+              for (int j = 0; j < kLoad; ++j) sum[h + j] = __fadd_rn(sum[h + j], __uint_as_float(va[j]));
+            }
+          }
+        }
+        if (!seg_ok) { ok = false; break; }
+        if (nseg > 1) {
+#pragma unroll
+          for (int h = 0; h < kHalf; h += 16) {
+            uint32_t vs[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) vs[j] = __float_as_uint(sum[h + j]);
+            ptx::tmem_st16(tmem + ab * NR + lane_off + c_lo + h, vs);
+          }
+          ptx::tmem_st_wait();
+        }
+      } else if constexpr (kSeg) {
         // every segment, the step's last too: load it (then the MMA lane may start the next one into
         // the same block, the next step's first included) and add it into the sum, which is the field
         bool seg_ok = true;
@@ -538,8 +650,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_sb_kernel(const __grid_const
         }
         if (!seg_ok) { ok = false; break; }
       }
-      const int ab = ls & 1;
-      const uint32_t t_acc = kSeg ? t_sum : tmem + ab * NR;
+      const uint32_t t_acc = kSeg && !PAIR ? t_sum : tmem + ab * NR;
       if constexpr (!kSeg) {
         const bool got = ptx::mbar_wait(&accf_bar[ab], (uint32_t)(ls >> 1) & 1, p.wait_cycles);
         if (!epi_all(got)) { ok = false; break; }
@@ -632,10 +743,12 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_sb_kernel(const __grid_const
         }
       }
       if constexpr (!kEOnly) ptx::tmem_st_wait();
-      // the accumulator may be overwritten from here on (split operands: released by the folds)
-      ptx::tc_fence_before();
-      __syncwarp();
-      if (!kSeg && lane == 0) ptx::mbar_arrive(&acce_bar[ab]);
+      if constexpr (PAIR || !kSeg) {
+        release(ab);
+      } else {
+        ptx::tc_fence_before();
+        __syncwarp();
+      }
       // publish this unit's V(t+1) chunk to the replica column
       if constexpr (kStageV && !kEOnly) ptx::fence_proxy_async_shared();  // tile writes -> TMA store
       epi_sync();
@@ -693,9 +806,19 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_sb_kernel(const __grid_const
   if (!ok) atomicOr(p.status, kErrWaitTimeout);
   ptx::tc_fence_before();
   __syncthreads();
+  if constexpr (PAIR) {
+    // the second CTA: the issuer's MMAs write its tensor memory and read its shared memory; its own work done,
+    // it waits for their completion (the issuer's last commit)
+    if (!issuer && warp == 1 && lane == 0 && !wait(&drain_bar, 0)) atomicOr(p.status, kErrWaitTimeout);
+    __syncwarp();
+    ptx::cluster_sync();  // neither CTA leaves while the other may still touch its memory
+  }
   if (warp == 1) {
     ptx::tc_fence_after();
-    ptx::tmem_dealloc(tmem, kCols);
+    if constexpr (PAIR)
+      ptx::tmem_dealloc_pair(tmem, kCols);
+    else
+      ptx::tmem_dealloc(tmem, kCols);
   }
 }
 
@@ -705,17 +828,29 @@ constexpr int tc_vtile_bytes() {
   return Cfg<DT, VARIANT>::kBParts == 1 ? NR * kBM * Cfg<DT, VARIANT>::kElem : 0;
 }
 
-template <int DT, int VARIANT, int NR>
+template <int DT, int VARIANT, int NR, bool PAIR = false>
+constexpr int tc_stage_bytes() {
+  return Cfg<DT, VARIANT>::kAParts * kBM * kChunkBytes + Cfg<DT, VARIANT>::kBParts * (PAIR ? NR / 2 : NR) * kChunkBytes;
+}
+
+template <int DT, int VARIANT, int NR, bool PAIR = false>
 constexpr int tc_stages() {
-  constexpr int kStage = Cfg<DT, VARIANT>::kAParts * kBM * kChunkBytes + Cfg<DT, VARIANT>::kBParts * NR * kChunkBytes;
+  constexpr int kStage = tc_stage_bytes<DT, VARIANT, NR, PAIR>();
   constexpr int kBudget = 216 * 1024 - tc_vtile_bytes<DT, VARIANT, NR>();
   return kBudget / kStage > 8 ? 8 : kBudget / kStage;
 }
 
-template <int DT, int VARIANT, int NR>
+template <int DT, int VARIANT, int NR, bool PAIR = false>
 constexpr size_t tc_smem() {
-  constexpr int kStage = Cfg<DT, VARIANT>::kAParts * kBM * kChunkBytes + Cfg<DT, VARIANT>::kBParts * NR * kChunkBytes;
-  return (size_t)tc_stages<DT, VARIANT, NR>() * kStage + tc_vtile_bytes<DT, VARIANT, NR>() + 1024;
+  constexpr int kStage = tc_stage_bytes<DT, VARIANT, NR, PAIR>();
+  return (size_t)tc_stages<DT, VARIANT, NR, PAIR>() * kStage + tc_vtile_bytes<DT, VARIANT, NR>() + 1024;
+}
+
+// The pair form of a split bSB step.
+template <int DT>
+inline void tc_lookup_pair(const void **k, size_t *smem) {
+  *smem = tc_smem<DT, 1, 128, true>();
+  *k = reinterpret_cast<const void *>(&tc_sb_kernel<DT, 1, 128, tc_stages<DT, 1, 128, true>(), kEmodeStep, true>);
 }
 
 // Kernel for one epilogue mode; MODES is the bit set of modes compiled in.
