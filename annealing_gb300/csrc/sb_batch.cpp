@@ -49,11 +49,10 @@ std::map<std::string, std::pair<int, int>> g_tune_cache;
 
 // instance k of the batch starts from seed + k, whichever bucket holds it
 sb_status init_all(sb_bucket &bk, uint64_t seed, std::string &err) {
-  for (size_t j = 0; j < bk.g->insts.size(); ++j) {
-    sb_status s = bk.g->init_state(bk.g->insts[j], seed + (uint64_t)bk.members[j], err);
-    if (s != SB_OK) return s;
-  }
-  return SB_OK;
+  const cudaError_t e = bk.g->init_states(seed);
+  if (e == cudaSuccess) return SB_OK;
+  err = std::string("initial state: ") + cudaGetErrorString(e);
+  return SB_ERR_CUDA;
 }
 
 // Instances too large for a wave take one launch per step: times a few steps of each (replica tile, item
@@ -298,13 +297,10 @@ sb_status run(sb_batch *b, uint64_t seed, sb_result *res, std::string &err) {
     sbh::touch_pages(res[k].final_x, (size_t)inst[k]->R * inst[k]->n * sizeof(float));
     sbh::touch_pages(res[k].final_y, (size_t)inst[k]->R * inst[k]->n * sizeof(float));
   }
-  std::vector<std::vector<double>> energies(count);
+  // every instance's energies, best replica and its spins, one copy per bucket
+  std::vector<std::vector<uint8_t>> packed(b->buckets.size());
   std::vector<uint32_t> status(b->buckets.size(), 0);
-  for (size_t k = 0; k < count && e == cudaSuccess; ++k) {
-    energies[k].resize(inst[k]->R);
-    e = cudaMemcpyAsync(energies[k].data(), inst[k]->energy, (size_t)inst[k]->R * sizeof(double),
-                        cudaMemcpyDeviceToHost, st);
-  }
+  for (size_t i = 0; i < b->buckets.size() && e == cudaSuccess; ++i) e = b->buckets[i].g->results(packed[i]);
   for (size_t i = 0; i < b->buckets.size() && e == cudaSuccess; ++i)
     e = cudaMemcpyAsync(&status[i], b->buckets[i].g->d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -320,16 +316,22 @@ sb_status run(sb_batch *b, uint64_t seed, sb_result *res, std::string &err) {
   }
   float dev_ms = 0;
   cudaEventElapsedTime(&dev_ms, b->ev0, b->ev1);
-  // best replica of each instance, its spins, optional full state
+  std::vector<const double *> energies(count);
   std::vector<int> best(count, 0);
-  std::vector<std::vector<float>> xb(count);
+  std::vector<const int8_t *> spins(count);
+  for (size_t i = 0; i < b->buckets.size(); ++i)
+    for (size_t j = 0; j < b->buckets[i].members.size(); ++j) {
+      const size_t k = (size_t)b->buckets[i].members[j];
+      const uint8_t *p = packed[i].data() + inst[k]->out;
+      energies[k] = reinterpret_cast<const double *>(p);
+      int64_t r;
+      memcpy(&r, p + 8 * (size_t)inst[k]->R, sizeof(r));
+      best[k] = (int)r;
+      spins[k] = reinterpret_cast<const int8_t *>(p) + 8 * ((size_t)inst[k]->R + 1);
+    }
+  // optional full state
   for (size_t k = 0; k < count; ++k) {
     const auto &gi = *inst[k];
-    for (int r = 1; r < gi.R; ++r)
-      if (energies[k][r] < energies[k][best[k]]) best[k] = r;
-    xb[k].resize(gi.n);
-    e = cudaMemcpyAsync(xb[k].data(), gi.x + (size_t)best[k] * gi.xp, (size_t)gi.n * sizeof(float),
-                        cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess && res[k].final_x)
       e = cudaMemcpy2DAsync(res[k].final_x, (size_t)gi.n * 4, gi.x, (size_t)gi.xp * 4, (size_t)gi.n * 4, (size_t)gi.R,
                             cudaMemcpyDeviceToHost, st);
@@ -346,16 +348,12 @@ sb_status run(sb_batch *b, uint64_t seed, sb_result *res, std::string &err) {
   // exact host re-check of every returned spin vector, spread over the host cores
   std::vector<int64_t> e64(count, 0);
   std::vector<int> okv(count, 0);
-  std::vector<std::vector<int8_t>> spins(count);
   const unsigned nth = std::max(1u, std::min(std::thread::hardware_concurrency(), (unsigned)count));
   std::vector<std::thread> th;
   for (unsigned w = 0; w < nth; ++w)
     th.emplace_back([&, w] {
       for (size_t k = w; k < count; k += nth) {
-        const auto &gi = *inst[k];
-        spins[k].resize(gi.n);
-        for (int i = 0; i < gi.n; ++i) spins[k][i] = xb[k][i] > 0.0f ? 1 : -1;
-        if (b->copies->energy(k, spins[k].data(), &e64[k], 1) == SB_OK)
+        if (b->copies->energy(k, spins[k], &e64[k], 1) == SB_OK)
           okv[k] = (double)e64[k] == energies[k][best[k]] ? 1 : 0;
       }
     });
@@ -368,8 +366,8 @@ sb_status run(sb_batch *b, uint64_t seed, sb_result *res, std::string &err) {
   for (auto &bk : b->buckets) launches += bk.g->launches;
   for (size_t k = 0; k < count; ++k) {
     sb_result &r = res[k];
-    if (r.best_spins) memcpy(r.best_spins, spins[k].data(), spins[k].size());
-    if (r.replica_energies) memcpy(r.replica_energies, energies[k].data(), energies[k].size() * sizeof(double));
+    if (r.best_spins) memcpy(r.best_spins, spins[k], (size_t)inst[k]->n);
+    if (r.replica_energies) memcpy(r.replica_energies, energies[k], (size_t)inst[k]->R * sizeof(double));
     r.best_energy = energies[k][best[k]];
     r.best_energy_i64 = e64[k];
     r.best_replica = best[k];
@@ -380,7 +378,7 @@ sb_status run(sb_batch *b, uint64_t seed, sb_result *res, std::string &err) {
     r.device_ms = dev_ms;
     r.kernel_ms_avg = kernel_ms;
     r.steps_per_launch = 1;
-    r.kernel_launches = launches + 2 * (int64_t)count;  // + init and sign kernels per instance
+    r.kernel_launches = launches;
     r.total_ms = total_ms;
     r.spin_updates_per_s = dev_ms > 0 ? updates / (dev_ms * 1e-3) : 0.0;
   }

@@ -18,6 +18,7 @@
 #include "sb_grouped.cuh"
 #include "sb_grouped.h"
 #include "sb_host.h"
+#include "sb_init.cuh"
 #include "sb_run.cuh"
 #include "sb_run.h"
 
@@ -151,15 +152,12 @@ constexpr int64_t kWaveBytes = 80ll << 20;
 // Steps of one launch (a step's tag has 32 bits).
 constexpr int kWaveSteps = 1 << 20;
 
-// V of every instance at its step tick - t0, from x: one block per item (128 spins x nr replicas).
-__global__ void g_signs_items_kernel(const GInst *insts, const RunItem *items, int nr, int op, int tick) {
-  const RunItem w = items[blockIdx.x];
-  const GInst *in = insts + w.inst;
-  uint8_t *v = in->v[(tick - in->t0) & 1];
-  const int n = in->n, xp = in->xp, kb = in->kbytes, rows = min(nr, in->R - w.r0);
+// The signs of an item's x (128 spins x nr replicas) into its instance's V buffer v, by a block.
+__device__ __forceinline__ void signs_of_item(const GInst *in, uint8_t *v, int m0, int r0, int nr, int op) {
+  const int n = in->n, xp = in->xp, kb = in->kbytes, rows = min(nr, in->R - r0);
   if (op == kGopE2m3) {
     for (int k = threadIdx.x; k < rows * 8; k += blockDim.x) {
-      const int r = w.r0 + k / 8, s0 = w.m0 + 16 * (k % 8);
+      const int r = r0 + k / 8, s0 = m0 + 16 * (k % 8);
       if (s0 >= n) continue;
       uint32_t word[3] = {0u, 0u, 0u};
       for (int i = 0; i < 16 && s0 + i < n; ++i) {
@@ -175,17 +173,78 @@ __global__ void g_signs_items_kernel(const GInst *insts, const RunItem *items, i
   }
   const int per = op == kGopE2m1 ? 64 : 128;  // bytes of a replica's 128 signs
   for (int k = threadIdx.x; k < rows * per; k += blockDim.x) {
-    const int r = w.r0 + k / per, b = k % per;
+    const int r = r0 + k / per, b = k % per;
     const float *x = in->x + (size_t)r * xp;
     if (op == kGopE2m1) {
-      const int i = w.m0 + 2 * b;
+      const int i = m0 + 2 * b;
       const uint32_t lo = i < n ? (x[i] > 0.0f ? kE2m1Plus : kE2m1Minus) : 0u;
       const uint32_t hi = i + 1 < n ? (x[i + 1] > 0.0f ? kE2m1Plus : kE2m1Minus) : 0u;
-      v[(size_t)r * kb + w.m0 / 2 + b] = (uint8_t)(lo | (hi << 4));
-    } else if (w.m0 + b < n) {
-      v[(size_t)r * kb + w.m0 + b] = x[w.m0 + b] > 0.0f ? (uint8_t)0x38 : (uint8_t)0xB8;
+      v[(size_t)r * kb + m0 / 2 + b] = (uint8_t)(lo | (hi << 4));
+    } else if (m0 + b < n) {
+      v[(size_t)r * kb + m0 + b] = x[m0 + b] > 0.0f ? (uint8_t)0x38 : (uint8_t)0xB8;
     }
   }
+}
+
+// V of every instance at its step tick - t0, from x: one block per item.
+__global__ void g_signs_items_kernel(const GInst *insts, const RunItem *items, int nr, int op, int tick) {
+  const RunItem w = items[blockIdx.x];
+  const GInst *in = insts + w.inst;
+  signs_of_item(in, in->v[(tick - in->t0) & 1], w.m0, w.r0, nr, op);
+}
+
+// The initial state of every instance (seed + its index), V(0) and zeroed energies, one block per item: what two
+// launches and a memset per instance did (96 instances: 1.6 ms of a batch of 16.5).
+__global__ void g_init_items_kernel(const GInst *insts, const GItem *items, int nr, int op, uint64_t seed) {
+  const GItem w = items[blockIdx.x];
+  const GInst *in = insts + w.inst;
+  const int n = in->n, xp = in->xp, rows = min(nr, in->R - w.r0);
+  const uint64_t s = seed + (uint64_t)(int64_t)in->index;
+  for (int k = threadIdx.x; k < rows * kBM; k += blockDim.x) {
+    const int r = w.r0 + k / kBM, i = w.m0 + k % kBM;
+    if (i >= n) continue;
+    const uint64_t e = 2 * ((uint64_t)r * n + i);
+    in->x[(size_t)r * xp + i] = uniform_value(s, e);
+    in->y[(size_t)r * xp + i] = uniform_value(s, e + 1);
+  }
+  __syncthreads();
+  signs_of_item(in, in->v[0], w.m0, w.r0, nr, op);
+}
+
+__global__ void g_zero_energies_kernel(const GInst *insts) {
+  const GInst *in = insts + blockIdx.x;
+  for (int r = threadIdx.x; r < in->R; r += blockDim.x) in->energy[r] = 0.0;
+}
+
+// An instance's energies, the first replica of the least one and its spins, at out + in->out: R doubles, the index
+// (8 bytes), n bytes. One block per instance.
+__global__ void g_results_kernel(const GInst *insts, uint8_t *out) {
+  __shared__ double chunk[256];
+  __shared__ int best_sh;
+  const GInst *in = insts + blockIdx.x;
+  uint8_t *dst = out + in->out;
+  double least = 0.0;  // thread 0's
+  int best = 0;
+  for (int r0 = 0; r0 < in->R; r0 += 256) {
+    const int r = r0 + (int)threadIdx.x, m = min(256, in->R - r0);
+    if (r < in->R) chunk[threadIdx.x] = reinterpret_cast<double *>(dst)[r] = in->energy[r];
+    __syncthreads();
+    if (threadIdx.x == 0)
+      for (int k = 0; k < m; ++k)
+        if (r0 + k == 0 || chunk[k] < least) {
+          least = chunk[k];
+          best = r0 + k;
+        }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    best_sh = best;
+    *reinterpret_cast<int64_t *>(dst + 8 * (size_t)in->R) = best;
+  }
+  __syncthreads();
+  const float *x = in->x + (size_t)best_sh * in->xp;
+  int8_t *s = reinterpret_cast<int8_t *>(dst) + 8 * ((size_t)in->R + 1);
+  for (int i = threadIdx.x; i < in->n; i += blockDim.x) s[i] = x[i] > 0.0f ? 1 : -1;
 }
 
 bool grouped_kernel_for(int nr, int emode, int op, const void **k, size_t *smem) {
@@ -392,6 +451,9 @@ void Grouped::clear() {
   cudaFree(d_run);
   cudaFree(d_rest);
   cudaFree(d_ll);
+  cudaFree(d_out);
+  d_out = nullptr;
+  cap_out = 0;
   d_run = nullptr;
   d_rest = nullptr;
   d_ll = nullptr;
@@ -605,10 +667,15 @@ sb_status Grouped::sync_tables(std::string &err) {
     }
   }
   std::vector<GInst> descs(insts.size());
+  out_bytes = 0;
   std::vector<GItem> items;
   for (size_t i = 0; i < insts.size(); ++i) {
-    descs[i] = insts[i].desc;
-    const GHost &g = insts[i];
+    GHost &g = insts[i];
+    g.out = out_bytes;
+    out_bytes += 8 * ((size_t)g.R + 1) + ((size_t)g.n + 7) / 8 * 8;
+    descs[i] = g.desc;
+    descs[i].index = g.tag;
+    descs[i].out = g.out;
     for (int m0 = 0; m0 < g.Np; m0 += kBM)
       for (int r0 = 0; r0 < g.Rp; r0 += nr) items.push_back(GItem{(int)i, m0, r0, grouped_kchunks(g.Kp, g.op)});
   }
@@ -831,12 +898,29 @@ cudaError_t Grouped::run_steps(int tick0, int count, bool use_graph) {
   return cudaGraphLaunch(graph, st);
 }
 
+cudaError_t Grouped::init_states(uint64_t seed) {
+  if (n_items == 0) return cudaSuccess;
+  ++launches;
+  g_init_items_kernel<<<n_items, 256, 0, st>>>(d_insts, d_items, nr, op, seed);
+  return cudaGetLastError();
+}
+
 cudaError_t Grouped::energy_pass(int tick) {
-  for (auto &g : insts) {
-    cudaError_t e = cudaMemsetAsync(g.energy, 0, (size_t)g.R * sizeof(double), st);
-    if (e != cudaSuccess) return e;
-  }
+  if (insts.empty()) return cudaSuccess;
+  ++launches;
+  g_zero_energies_kernel<<<(unsigned)insts.size(), 128, 0, st>>>(d_insts);
+  if (cudaError_t e = cudaGetLastError(); e != cudaSuccess) return e;
   return launch(tick, kEmodeEnergy);
+}
+
+cudaError_t Grouped::results(std::vector<uint8_t> &host) {
+  host.resize(out_bytes);
+  if (insts.empty()) return cudaSuccess;
+  if (!reserve(d_out, cap_out, out_bytes)) return cudaErrorMemoryAllocation;
+  ++launches;
+  g_results_kernel<<<(unsigned)insts.size(), 256, 0, st>>>(d_insts, d_out);
+  if (cudaError_t e = cudaGetLastError(); e != cudaSuccess) return e;
+  return cudaMemcpyAsync(host.data(), d_out, out_bytes, cudaMemcpyDeviceToHost, st);
 }
 
 cudaError_t Grouped::energy_pass_for(const std::vector<int> &idx, int tick) {

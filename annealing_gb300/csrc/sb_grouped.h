@@ -30,6 +30,8 @@ struct alignas(64) GInst {
   int t0;                // the instance's step t = tick - t0
   float c0, dt, dta0;
   int kbytes;            // bytes of one operand row in global memory: Kp (FP8), Kp / 2 (E2M1), 3 Kp / 4 (E2M3)
+  int index;             // the caller's index: its seed is the run's plus this
+  size_t out;            // offset of its results in the packed copy
 };
 
 // One work item: a 128-spin x NR-replica tile of one instance.
@@ -59,6 +61,7 @@ struct GHost {
   uint8_t *a = nullptr, *v[2] = {nullptr, nullptr};
   float *x = nullptr, *y = nullptr, *h = nullptr, *pumps = nullptr;
   double *energy = nullptr;
+  size_t out = 0;  // offset of its results in results()
   GInst desc;
 };
 
@@ -99,9 +102,14 @@ class Grouped {
   cudaError_t run_steps(int tick0, int count, bool use_graph);
   // whether some instance does not fit a wave (valid after sync_tables)
   bool has_rest() const { return n_rest > 0; }
+  // The initial state of every resident instance, seeded with seed + its tag (after sync_tables).
+  cudaError_t init_states(uint64_t seed);
   // Energies of every resident instance's current spins (instances must be at step t = tick - t0).
   cudaError_t energy_pass(int tick);
-  // The same for a subset of resident instances (indices into insts).
+  // Per instance at its `out`: R energies, the index of the least (8 bytes), that replica's n spins; complete once
+  // the stream is.
+  cudaError_t results(std::vector<uint8_t> &host);
+  // The energies for a subset of resident instances (indices into insts).
   cudaError_t energy_pass_for(const std::vector<int> &idx, int tick);
   // Index of the resident instance with this tag, or -1.
   int find(int tag) const {
@@ -146,6 +154,8 @@ class Grouped {
   unsigned long long *d_ll = nullptr;  // exchange words of one wave
   int n_run = 0, n_rest = 0;
   size_t cap_run = 0, cap_rest = 0, cap_ll = 0;
+  uint8_t *d_out = nullptr;            // results of the resident instances, packed
+  size_t cap_out = 0, out_bytes = 0;
   bool v_stale = false;              // the V buffers lag x (a wave has run since)
   GItem *d_sub_items = nullptr;
   int cap_sub = 0;
