@@ -110,12 +110,35 @@ sb_status check_params(const sb_problem *p, const sb_params *prm, std::string &e
   return SB_OK;
 }
 
+// The automatic mode's dSB solves of 32 replicas or more that the bit planes (sb_signs.cuh) run faster than the
+// tensor cores. A step of them costs n / 32 words of logic per row, plane and replica, so up to some n^2 R P it stays
+// at its latency of 0.3 to 1 us; a tensor-core step's chain takes 1.6 to 2.3 (E2M1 operands, |J| <= 4), 3 to 9 (FP8).
+// us per step, planes / tensor cores, +-1 unless noted:
+//   one CTA holds the solve, limit 134e6: n = 128 R = 1000 0.37 / 1.72, n = 256 R = 1000 0.90 / 1.72, n = 512 R = 300
+//   0.74 / 2.05, R = 512 (134e6) 1.36 / 1.84, R = 1000 2.23 / 1.85; |J| <= 3 n = 256 R = 1000 1.41 / 1.71;
+//   a cluster, 64e6: n = 700 R = 100 0.99 / 2.33, n = 1000 R = 64 0.88 / 2.21, n = 513 R = 300 (79e6) 2.10 / 2.22,
+//   R = 512 3.05 / 2.22; |J| <= 3 n = 513 R = 100 1.57 / 2.25, R = 200 (105e6) 2.56 / 2.30;
+//   |J| of 5 to 7, 300e6: n = 256 R = 1000 1.73 / 7.14, n = 700 R = 200 4.22 / 8.68, n = 513 R = 512 (404e6) 8.11 / 8.44.
+bool signs_beat_tc(const sb_problem *p, const sb_params *prm) {
+  if (prm->variant != SB_DSB || prm->trace || prm->trace_all || prm->steps <= 0 || !p->integer_valued ||
+      prm->operand_dtype != SB_OPERAND_AUTO)
+    return false;
+  const char *env = getenv("SB_PLAIN_PERSIST");
+  if (env && env[0] == '0') return false;
+  const int n = p->n, R = prm->replicas, P = p->max_abs_j <= 1 ? 1 : p->max_abs_j <= 3 ? 2 : 3;
+  // (what the tensor-core kernel has no room for, a unit of 128 x 128 to an SM, is not taken here either)
+  if ((int64_t)((n + 127) / 128) * ((R + 127) / 128) > 128) return false;
+  const bool one_cta = n <= (P == 1 ? sbk::kSignsOneCta : sbk::kSignsOneCta / 2);
+  const double limit = p->max_abs_j > 4 ? 300e6 : one_cta ? 134.5e6 : 64e6;
+  return (double)n * n * R * P <= limit && sbk::sign_planes(n, R, p->max_abs_j) > 0;
+}
+
 // Field mode and operand dtype for (problem, params).
 sb_status resolve_mode(const sb_problem *p, const sb_params *prm, int &mode, int &dtype,
                        std::string &err) {
   mode = prm->field_mode;
   if (mode == SB_FIELD_AUTO)
-    mode = (prm->variant != SB_ASB && prm->replicas >= 32) ? SB_FIELD_TC : SB_FIELD_FP32;
+    mode = (prm->variant != SB_ASB && prm->replicas >= 32 && !signs_beat_tc(p, prm)) ? SB_FIELD_TC : SB_FIELD_FP32;
   dtype = 0;
   if (mode == SB_FIELD_FP32) return SB_OK;
   if (prm->variant == SB_ASB) {

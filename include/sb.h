@@ -77,13 +77,17 @@ typedef enum sb_variant { SB_ASB = 0, SB_BSB = 1, SB_DSB = 2 } sb_variant;
 
 /* How the field J*v is computed.
  *  SB_FIELD_AUTO: tensor cores when replicas >= 32 and the problem allows an exact/declared
- *                 precision, otherwise the plain FP32 kernel.
- *  SB_FIELD_FP32: the plain fused FP32 kernel (the drop-in form): the whole solve in one cooperative
- *                 launch when the rows fit one co-resident grid (n <= 2048, ceil(n / 16) x replicas
- *                 CTAs on the SMs, no energy trace), else one launch per step; the same bits either
- *                 way (environment SB_PLAIN_PERSIST=0 keeps one launch per step).
+ *                 precision, otherwise the plain FP32 path; dSB with integer |J| <= 7 whose bit
+ *                 planes are faster (n^2 x replicas small: up to 64 to 300 million) takes the
+ *                 plain path too (the same bits).
+ *  SB_FIELD_FP32: the plain fused FP32 path (the drop-in form). dSB with integer |J| <= 7 and
+ *                 n <= 1024 (|J| <= 1: n <= 2048) runs the whole solve in one launch on bit planes of
+ *                 J (exact integer fields). Otherwise the whole solve is one cooperative launch when
+ *                 the rows fit one co-resident grid (n <= 2048, ceil(n / 16) x replicas CTAs on the
+ *                 SMs), else, and with an energy trace, one launch per step; the same bits each way
+ *                 (environment SB_PLAIN_PERSIST=0 keeps one launch per step).
  *  SB_FIELD_TC:   tcgen05 tensor cores. dSB with integer |J| <= 4 and n <= ~2300: packed E2M1
- *                 operands with J resident in shared memory, FP32 accumulation (bit-exact).
+ *                 operands, FP32 accumulation (bit-exact); without a trace every step in one launch.
  *                 dSB with integer |J| <= 16: FP8 E4M3 operands (grouped batches and serving:
  *                 packed E2M3, J / 4 in six bits), FP32 accumulation (bit-exact).
  *                 dSB with integer |J| <= 256: BF16 operands (bit-exact).

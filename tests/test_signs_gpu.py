@@ -87,3 +87,31 @@ def test_a_cached_plan_takes_other_couplings(monkeypatch):
             ctx.close()
         np.testing.assert_array_equal(a.final_x, b.final_x)
         np.testing.assert_array_equal(a.final_y, b.final_y)
+
+
+@pytest.mark.parametrize("n,jmax,R,planes", [
+    (100, 1, 64, True),
+    (256, 4, 300, True),     # three planes, one CTA
+    (512, 1, 512, True),     # 134e6: the one-CTA limit
+    (512, 1, 514, False),
+    (513, 3, 100, True),     # 53e6, a cluster of five
+    (513, 3, 130, False),    # 68e6
+    (640, 7, 243, True),     # FP8 on the tensor cores: 300e6
+    (640, 7, 245, False),
+    (200, 9, 40, False),     # more planes than the kernel has
+])
+def test_automatic_mode_takes_the_faster_form(n, jmax, R, planes):
+    J = instances.erdos_renyi(n, 0.7, seed=n + R, jmax=jmax, allow_zero=True)
+    J[0, 1] = J[1, 0] = jmax
+    prob = sb.Problem.from_dense(J)
+    ctx = sb.Context(0)
+    try:
+        auto = ctx.solve(prob, sb.Params.default(sb.DSB, steps=25, replicas=R, seed=3), want_state=True)
+        tc = ctx.solve(prob, sb.Params.default(sb.DSB, steps=25, replicas=R, seed=3, field_mode=sb.FIELD_TC), want_state=True)
+    finally:
+        ctx.close()
+    assert auto.field_mode == (sb.FIELD_FP32 if planes else sb.FIELD_TC) and tc.field_mode == sb.FIELD_TC
+    np.testing.assert_array_equal(auto.final_x, tc.final_x)
+    np.testing.assert_array_equal(auto.final_y, tc.final_y)
+    np.testing.assert_array_equal(auto.replica_energies, tc.replica_energies)
+    assert auto.energy_check_ok
