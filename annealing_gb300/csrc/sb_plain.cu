@@ -940,6 +940,9 @@ __global__ void __launch_bounds__(kPersistThreads, 1) plain_persist_kernel(Plain
   for (int t = 0; t < a.steps && ok; ++t) {
     const float pump = pump_next;
     if (t + 1 < a.steps) pump_next = a.pumps[t + 1];  // off the step's critical path
+    float z0 = z1;  // NMFA sweep t (stage t / 2): the stage's second sample, or
+    if constexpr (VARIANT == 3)
+      if ((t & 1) == 0) sbm::nmfa_gauss(wd, a.noise, z0, z1);  // a pair, drawn while the states are on their way
     ok = __syncthreads_and(gather(t) ? 1 : 0) != 0;
     if (!ok) break;
     // field of this warp's row over groups g = lane + 32 k (spins 4 g .. 4 g + 3)
@@ -963,13 +966,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1) plain_persist_kernel(Plain
         // aSB: the coupling kick; the next step's local sub-steps follow below
         y = __fmaf_rn(a.coeff, acc, y);
       } else if constexpr (VARIANT == 3) {
-        // NMFA sweep t (stage t / 2): the stage's first sweep draws its Gaussian pair
-        float z;
-        if ((t & 1) == 0)
-          sbm::nmfa_gauss(wd, a.noise, z, z1);
-        else
-          z = z1;
-        x = sbm::nmfa_update(acc, nv, z, pump, a.keep, a.mix, x);
+        x = sbm::nmfa_update(acc, nv, z0, pump, a.keep, a.mix, x);
       } else {
         sb_update(acc, hv, pump, a.c0, a.dt, a.dta0, x, y);
       }
