@@ -55,6 +55,7 @@ struct sb_plan {
   unsigned long long *dwords = nullptr;
   size_t words_bytes = 0;
   uint32_t *dplanes = nullptr;  // dSB with small integer couplings: their bit planes, and how many magnitudes
+  bool cluster = false;         // the plain FP32 steps run in clusters (sb_cluster.cuh)
   int planes = 0;               // they have (0: the couplings uploaded are not such)
   float *dxk = nullptr;    // [kTopK][xp] rows of the best candidates (real-valued J)
   double *dek = nullptr;   // [kTopK] their FP64 energies
@@ -246,7 +247,7 @@ void plan_free_device(sb_plan *pl) {
 }
 
 // The plain FP32 steps of a solve run in one launch.
-bool one_launch(const sb_plan *pl) { return pl->planes || pl->dwords; }
+bool one_launch(const sb_plan *pl) { return pl->planes || pl->cluster || pl->dwords; }
 
 bool needs_trace(const sb_params &p) { return p.trace || p.trace_all; }
 
@@ -338,7 +339,8 @@ sb_status plan_create(sb_ctx *ctx, const sb_problem *p, const sb_params *prm, sb
     // dSB with couplings up to 3 or 7: no exchange through L2 at all (sb_signs.cuh)
     if (want && prm->variant == SB_DSB && p->integer_valued && sbk::sign_planes(pl->n, pl->R, p->max_abs_j))
       PLAN_ALLOC(pl->dplanes, sbk::sign_plane_bytes(pl->n));
-    const int ctas = want ? sbk::plain_persist_ctas(pl->n, pl->R, pl->jp) : 0;
+    pl->cluster = want && sbk::plain_cluster_fits(prm->variant, pl->n, pl->R, pl->jp);
+    const int ctas = want && !pl->cluster ? sbk::plain_persist_ctas(pl->n, pl->R, pl->jp) : 0;
     if (ctas > 0) {
       pl->words_bytes = (size_t)2 * ctas * 128;  // at most one 128-byte line per CTA
       PLAN_ALLOC(pl->dwords, pl->words_bytes);
@@ -444,10 +446,10 @@ cudaError_t enqueue_loop(sb_plan *pl, cudaStream_t st, std::vector<cudaEvent_t> 
     if (launches) *launches = nl;
     return cudaSuccess;
   }
-  if (pl->dwords) {
-    // plain FP32 SB in one cooperative launch (same fields and updates as the per-step kernel)
+  if (pl->cluster || pl->dwords) {
+    // plain FP32 SB in one launch (same fields and updates as the per-step kernel)
     if (p.steps > 0) {
-      cudaError_t e = cudaMemsetAsync(pl->dwords, 0, pl->words_bytes, st);
+      cudaError_t e = pl->cluster ? cudaSuccess : cudaMemsetAsync(pl->dwords, 0, pl->words_bytes, st);
       if (e != cudaSuccess) return e;
       sbk::PlainPersist a;
       memset(&a, 0, sizeof(a));
@@ -474,7 +476,7 @@ cudaError_t enqueue_loop(sb_plan *pl, cudaStream_t st, std::vector<cudaEvent_t> 
       a.words = pl->dwords;
       a.status = pl->dstatus;
       if (evs) cudaEventRecord((*evs)[0], st);
-      if ((e = sbk::launch_plain_persist(a, st)) != cudaSuccess) return e;
+      if ((e = pl->cluster ? sbk::launch_plain_cluster(a, st) : sbk::launch_plain_persist(a, st)) != cudaSuccess) return e;
       if (evs) cudaEventRecord((*evs)[1], st);
       nl = 1;
     }

@@ -81,6 +81,12 @@ constexpr int kPersistMaxJp = 2048;
 int plain_persist_ctas(int n, int R, int jp);
 cudaError_t launch_plain_persist(const PlainPersist &a, cudaStream_t st);
 
+// The same in one launch of independent clusters, x exchanged through distributed shared memory (sb_cluster.cuh):
+// n <= kClusterMaxN, any number of replicas, `words` unused.
+constexpr int kClusterMaxN = 512;
+bool plain_cluster_fits(int variant, int n, int R, int jp);
+cudaError_t launch_plain_cluster(const PlainPersist &a, cudaStream_t st);
+
 // Plain FP32 dSB with small integer couplings, the whole solve in one launch of independent clusters (sb_signs.cuh).
 struct SignSolve {
   int n, R, xp, words;        // words = ceil(n / 32)

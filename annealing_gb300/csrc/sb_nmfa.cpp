@@ -102,6 +102,7 @@ sb_status nmfa_run(sb_ctx *ctx, const sb_problem *prob, const sb_nmfa_params *pr
     return fail(ctx, SB_ERR_UNSUPPORTED, std::string(who) + ": the tensor-core field needs integer couplings "
                                                             "with |J| <= 256");
   bool use_tc = prm->field_mode == SB_FIELD_TC || (prm->field_mode == SB_FIELD_AUTO && tc_ok && R >= 32);
+  bool in_clusters = false;  // FP32 field: the one-launch solve in clusters
   int persist_ctas = 0;  // FP32 field: CTAs of the one-launch solve, 0 when it does not fit
   std::vector<float> sweep_betas((size_t)2 * stages);
   for (int t = 0; t < 2 * stages; ++t) sweep_betas[t] = betas[t / 2];
@@ -193,7 +194,9 @@ sb_status nmfa_run(sb_ctx *ctx, const sb_problem *prob, const sb_nmfa_params *pr
   if (!use_tc) {
     // SB_PLAIN_PERSIST=0 keeps one launch per sweep
     const char *env = getenv("SB_PLAIN_PERSIST");
-    persist_ctas = (env && env[0] == '0') ? 0 : sbk::plain_persist_ctas(n, R, jp);
+    const bool want = !(env && env[0] == '0');
+    in_clusters = want && sbk::plain_cluster_fits(3, n, R, jp);
+    persist_ctas = want && !in_clusters ? sbk::plain_persist_ctas(n, R, jp) : 0;
     const size_t need = (size_t)2 * persist_ctas * 128;  // one 128-byte line per CTA and parity
     if (persist_ctas > 0 && c->words_bytes < need) {
       cudaFree(c->dwords);
@@ -213,11 +216,11 @@ sb_status nmfa_run(sb_ctx *ctx, const sb_problem *prob, const sb_nmfa_params *pr
     NM_CUDA(sbk::launch_nmfa_signs(c->ds, n, R, xp, c->dsamp, st));
     NM_CUDA(sbk::tc_energy_signs(c->te, c->ds, nullptr, c->den, c->dstatus, st));
     launches += 5;
-  } else if (persist_ctas > 0) {
+  } else if (in_clusters || persist_ctas > 0) {
     // every sweep in one cooperative launch: J rows in registers, states exchanged as tagged words
     // (the plain solve's one-launch kernel with the NMFA update; the same bits as one launch per
     // sweep)
-    NM_CUDA(cudaMemsetAsync(c->dwords, 0, c->words_bytes, st));
+    if (!in_clusters) NM_CUDA(cudaMemsetAsync(c->dwords, 0, c->words_bytes, st));
     sbk::PlainPersist a;
     memset(&a, 0, sizeof(a));
     a.variant = 3;
@@ -238,7 +241,7 @@ sb_status nmfa_run(sb_ctx *ctx, const sb_problem *prob, const sb_nmfa_params *pr
     a.noise = prm->noise;
     a.keep = (float)(1.0 - (double)prm->recombination);  // nmfa.cu:95, 1.0 - recombination
     a.mix = prm->recombination;
-    NM_CUDA(sbk::launch_plain_persist(a, st));
+    NM_CUDA(in_clusters ? sbk::launch_plain_cluster(a, st) : sbk::launch_plain_persist(a, st));
     ++launches;
     sbk::PlainEnergy pe;
     memset(&pe, 0, sizeof(pe));

@@ -1011,6 +1011,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1) plain_persist_kernel(Plain
 }
 
 #include "sb_signs.cuh"
+#include "sb_cluster.cuh"
 
 }  // namespace
 
@@ -1171,22 +1172,47 @@ cudaError_t launch_plain_persist(const PlainPersist &a, cudaStream_t st) {
 }
 
 namespace {
+const void *cluster_kernel_for(int variant) {
+  switch (variant) {
+    case 0: return reinterpret_cast<const void *>(&cluster::cluster_kernel<0>);
+    case 1: return reinterpret_cast<const void *>(&cluster::cluster_kernel<1>);
+    case 2: return reinterpret_cast<const void *>(&cluster::cluster_kernel<2>);
+    case 3: return reinterpret_cast<const void *>(&cluster::cluster_kernel<3>);
+  }
+  return nullptr;
+}
+// Launch shape of a cluster of C CTAs for each of R replicas.
+void cluster_config(int C, int R, int threads, cudaLaunchConfig_t &cfg, cudaLaunchAttribute &attr) {
+  memset(&cfg, 0, sizeof(cfg));
+  memset(&attr, 0, sizeof(attr));
+  cfg.gridDim = dim3((unsigned)C, (unsigned)R);
+  cfg.blockDim = dim3((unsigned)threads);
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = (unsigned)C;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+}
+// Whether such a cluster can run: more than eight CTAs need the attribute, and SMs of one GPC free for them.
+bool cluster_runs(const void *k, const cudaLaunchConfig_t &cfg) {
+  int clusters = 0;
+  if (cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&clusters, k, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return clusters > 0;
+}
+
 const void *signs_kernel_for(int n, int P) {
   return P == 1 ? signs::kernel_for<1>(n) : P == 2 ? signs::kernel_for<2>(n) : signs::kernel_for<3>(n);
 }
 // Launch shape for R solves of n spins.
 void signs_config(int n, int R, int P, cudaLaunchConfig_t &cfg, cudaLaunchAttribute &attr) {
-  memset(&cfg, 0, sizeof(cfg));
-  memset(&attr, 0, sizeof(attr));
   const bool one = signs::one_cta(n, P);
-  const int C = one ? 1 : (n + signs::kClusterRows - 1) / signs::kClusterRows;
-  cfg.gridDim = dim3((unsigned)C, (unsigned)R);
-  cfg.blockDim = dim3((unsigned)(one ? (n + 31) / 32 * 32 : signs::kClusterRows));
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = (unsigned)C;
-  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = one ? 0 : 1;
+  cluster_config(one ? 1 : (n + signs::kClusterRows - 1) / signs::kClusterRows, R,
+                 one ? (n + 31) / 32 * 32 : signs::kClusterRows, cfg, attr);
+  if (one) cfg.numAttrs = 0;
 }
 }  // namespace
 
@@ -1199,13 +1225,36 @@ int sign_planes(int n, int R, int max_abs_j) {
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr;
   signs_config(n, R, P, cfg, attr);
-  int clusters = 0;  // more than eight CTAs to a cluster need the attribute, and SMs of one GPC free for them
-  if (cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-      cudaOccupancyMaxActiveClusters(&clusters, k, &cfg) != cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
-  return clusters > 0 ? P : 0;
+  return cluster_runs(k, cfg) ? P : 0;
+}
+
+// Up to four CTAs to an SM the clusters beat every other form; beyond, a launch per step on register tiles runs more
+// replicas at once. us per step, clusters / tiles: n = 128 R = 200 (800 CTAs) 2.8 / 3.6, R = 300 3.6 / 3.8 (NMFA
+// 4.7 / 3.9); n = 256 R = 64 (512) 2.6 / 4.3, R = 150 (1200) 4.9 / 4.3; n = 512 R = 32 (512) 4.5 / 5.4, R = 64 6.8 / 5.5.
+bool plain_cluster_fits(int variant, int n, int R, int jp) {
+  if (n < 1 || n > kClusterMaxN || R < 1 || jp < 4 || jp % 4 || jp > kClusterMaxN) return false;
+  const int C = (n + cluster::kRows - 1) / cluster::kRows;
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || (long long)C * R > 4ll * sms)
+    return false;
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute attr;
+  cluster_config(C, R, cluster::kThreads, cfg, attr);
+  return cluster_runs(cluster_kernel_for(variant), cfg);
+}
+
+cudaError_t launch_plain_cluster(const PlainPersist &a, cudaStream_t st) {
+  const void *k = cluster_kernel_for(a.variant);
+  if (!k || a.n < 1 || a.n > kClusterMaxN || a.jp % 4 || a.jp < a.n || a.jp > kClusterMaxN || a.xp < a.n || a.steps < 0)
+    return cudaErrorInvalidValue;
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute attr;
+  cluster_config((a.n + cluster::kRows - 1) / cluster::kRows, a.R, cluster::kThreads, cfg, attr);
+  cfg.stream = st;
+  PlainPersist v = a;
+  void *args[] = {&v};
+  return cudaLaunchKernelExC(&cfg, k, args);
 }
 
 size_t sign_plane_bytes(int n) {
