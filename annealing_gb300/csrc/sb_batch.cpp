@@ -1,9 +1,9 @@
 // sb_batch_*: many instances of uneven size solved together by the grouped tensor-core kernel.
 //
 // The reference solves one instance per program run and its trials one after another
-// (SB/CUDA_GPU/m2_opt.cu:152); a batch here advances every instance and every replica of it in
-// one grouped launch per SB step and operand bucket (packed E2M1 where the couplings allow it,
-// packed E2M3 for the rest), the step loop replayed from a CUDA graph. Per instance the outputs are those
+// (SB/CUDA_GPU/m2_opt.cu:152); a batch here advances every instance and every replica of it, per
+// operand bucket (packed E2M1 where the couplings allow it, packed E2M3 for the rest) in waves of
+// instances whose steps run in one launch (sb_run.cuh). Per instance the outputs are those
 // of sb_solve (best spins, per-replica energies, host int64 re-check).
 #include <math.h>
 #include <string.h>

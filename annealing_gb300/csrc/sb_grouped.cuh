@@ -4,12 +4,13 @@
 // Uneven batches (hundreds of instances with N from 64 to 16384, each with its own replicas) and
 // the serving stream do not fit the one-unit-per-SM residency of
 // the single-instance kernel (sb_tc_kernel.cuh): their state is far larger than TMEM. Here one
-// launch advances every instance by one SB step:
+// launch advances every instance by one SB step (single and profiled steps, energies, and instances with more
+// items than a wave of sb_run.cuh holds):
 //   * work item = (instance, 128-spin tile, NR-replica tile); the CTAs of a persistent grid (one
 //     per SM) walk a cost-sorted item list round-robin;
-//   * warp 0 (lane 0) streams each item's J tile and V tile with 2-D TMA through the shared-memory
+//   * warp 0 (one elected lane issues) streams each item's J tile and V tile with 2-D TMA through the shared-memory
 //     ring, using the instance's tensor maps, which live in device memory next to its descriptor;
-//   * warp 1 (lane 0) issues tcgen05.mma (kind::f8f6f4, or kind::mxf4 for E2M1) into one of two
+//   * warp 1 (likewise) issues tcgen05.mma (kind::f8f6f4, or kind::mxf4 for E2M1) into one of two
 //     TMEM accumulators, so the
 //     epilogue of item k overlaps the contraction of item k + 1;
 //   * 8 epilogue warps read the accumulator, load x and y from global memory (coalesced), apply

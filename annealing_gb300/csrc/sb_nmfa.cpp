@@ -4,10 +4,11 @@
 // gpu_nmfa_kernel with one CTA per sample, copy the samples back, return the kernel's event time).
 // Here the samples are replicas. J is padded to [n][jp] once and every (sample, spin) gets its
 // XORWOW words from one seeding launch; then either
-//   * FP32 (the plain fused kernel's layout, sb_plain.cu): when the rows fit one co-resident grid
-//     (few samples: the reference program's single sample), every sweep runs in one cooperative
+//   * FP32 (the plain fused kernel's layout, sb_plain.cu): up to 512 spins and some 600 / (n / 32) samples
+//     every sweep runs in one launch of clusters (sb_cluster.cuh); larger instances whose rows fit one
+//     co-resident grid (few samples: the reference program's single sample) take one cooperative
 //     launch of the plain solve's persistent kernel (J rows in registers, the states exchanged as
-//     tagged words through L2, the same summation order and bits); otherwise each of a stage's two
+//     tagged words through L2); both in the same summation order, the same bits; otherwise each of a stage's two
 //     sweeps is one fused launch (field + noise + tanh update), issued back to back so that
 //     consecutive launches overlap (programmatic dependent launch); the last sweep writes the +-1
 //     samples and one energy pass gives every sample's energy; or

@@ -5,8 +5,8 @@
 // (one per replica tile). Requests queue in arrival order; the worker admits them while the
 // in-flight limit and the HBM budget allow (the budget counts each resident request's device
 // bytes), so requests that arrive while others run join the running set at the next tick and
-// their steps overlap on the device with everyone else's: one grouped launch per tick advances
-// every resident request by one SB step, each on its own schedule. A request retires at its own
+// their steps overlap on the device with everyone else's: the resident set advances by up to 64 SB
+// steps in a launch per wave, each request on its own schedule. A request retires at its own
 // step budget (energy pass, best spins back to the host, exact int64 re-check) and its memory is
 // freed for the next. Requests the grouped engine does not cover (bSB, aSB, real couplings,
 // |J| > 16) are solved one at a time on the worker's stream between ticks.

@@ -10,8 +10,8 @@
 //   * the work is tiled into units of 128 spins (TMEM lanes, MMA M) x NR replicas (MMA N); each
 //     CTA owns one unit for every step, so its x and y live in TMEM for the whole solve
 //     (columns [NR, 2NR) and [2NR, 3NR); the FP32 accumulator is columns [0, NR));
-//   * warp 0 (one lane) streams J tiles and V tiles with 2-D TMA into 128-byte-swizzled shared
-//     memory through a STAGES-deep mbarrier ring; warp 1 (one lane) issues tcgen05.mma
+//   * warp 0 (one elected lane issues) streams J tiles and V tiles with 2-D TMA into 128-byte-swizzled shared
+//     memory through a STAGES-deep mbarrier ring; warp 1 (likewise) issues tcgen05.mma
 //     (kind::f8f6f4 for FP8 E4M3 operands, kind::f16 for BF16), committing each stage back to the
 //     producer and the finished accumulator to the epilogue;
 //   * warps 2..9 (two per TMEM lane quadrant, each half of the replica columns) read the

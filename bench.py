@@ -58,7 +58,7 @@ WORKLOADS = {
                     "BF16 hi+lo tensor-core field"),
     "uneven-batch": ("dsb", 0, 64, 1500, "grouped",
                      "uneven batch: 512 instances, N ~ U[64,4096], Erdos-Renyi density ~ U[0.05,1], "
-                     "J = +-1, R=64, 1500 steps, one grouped tensor-core launch per step"),
+                     "J = +-1, R=64, 1500 steps, grouped tensor-core launches"),
     "sqa": ("sqa", 4096, 304, 100, "sqa",
             "SQA: complete N=4096, J iid +-1, M=64 Trotter slices, 100 annealing steps (the sizes of "
             "SQA_fully/fully_test/pre_calculate.cu), 304 replicas (two per SM)"),
@@ -75,14 +75,13 @@ WORKLOADS = {
 # DRAM traffic per launch (dram__bytes_read.sum + dram__bytes_write.sum) from one ncu capture of
 # each dominant kernel; the summaries, with the commands, are the files named here.
 NCU_TRAFFIC = {
-    # batched dSB, N=2000, R=1024, E2M1 kernel: bytes per launch, the same for 30 and 240 steps
-    # (everything after the first step is L2-resident)
-    "batched-dsb": (19.58e6, "profiles/tc_fp4_kernel_batched_dsb_n2000_r1024.md"),
+    # batched dSB, N=2000, R=1024, E2M1 kernel: bytes per launch (20-step capture; everything after the
+    # first step is on chip)
+    "batched-dsb": (19.11e6, "profiles/one_launch_kernels.md"),
     # plain dSB, N=2000, R=1: bytes per launch (ncu runs the launch with cold caches)
     "plain-dsb": (16.03e6, "profiles/plain_step_kernel_plain_dsb_n2000.md"),
-    # the same in one cooperative launch per solve: DRAM read + write per launch from a one-pass
-    # capture (J read once; 16.06 MB read, 15.9 KB written)
-    "plain-dsb-persist": (16.07e6, "profiles/plain_persist_kernel_plain_dsb_n2000.md"),
+    # the same in one launch per solve: the couplings' bit planes, read once
+    "plain-dsb-signs": (1.06e6, "profiles/one_launch_kernels.md"),
     # batched bSB, N=8192, R=256, BF16 hi+lo with the field accumulated in K segments: bytes per SB
     # step (8-step capture of the step launch: 2.587 GB; 4 steps: 1.146 GB), times the launch's steps
     "batched-bsb": (2.587e9 / 8, "profiles/tc_sb_kernel_batched_bsb_n8192_r256.md"),
@@ -437,7 +436,7 @@ def run_ours(args, rank, world, local_rank):
             traffic = (None, None)
         roof = {"bound": "tensor", "achieved": achieved, "peak": tc_peak, "unit": "TFLOP/s",
                 "frac": achieved / tc_peak, "traffic": traffic[0], "traffic_source": traffic[1],
-                "kernel": ("tc_fp4_kernel" if fdt == "fp4e2m1" else "tc_sb_kernel") + " (persistent, one launch per solve)",
+                "kernel": ("run_kernel" if fdt == "fp4e2m1" else "tc_sb_kernel") + " (persistent, one launch per solve)",
                 "launch_ms": rp.kernel_ms_avg, "sb_steps_per_launch": rp.steps_per_launch,
                 "flops_per_launch": flops_per_launch, "peak_source": label.format(src),
                 "frac_of_bf16_burst": achieved / bf16}
@@ -450,20 +449,17 @@ def run_ours(args, rank, world, local_rank):
         achieved = bytes_per_launch / (rp.kernel_ms_avg * 1e-3) / 1e9
         limiter = None
         if spl > 1:
-            traffic = NCU_TRAFFIC.get("plain-dsb-persist", (None, None)) if n == 2000 and R == 1 else (None, None)
-            kernel = "plain_persist_kernel (one cooperative launch per solve)"
-            note = ("achieved counts the algorithmic 4 N^2 bytes of J per SB step, but J lives in registers for "
-                    "the whole launch and is read from HBM once (traffic); the kernel is not HBM-bound, see "
-                    "limiter")
-            us = 1e3 * rp.kernel_ms_avg / spl
-            limiter = {"kind": "latency of the per-step sign exchange through L2",
-                       "us_per_sb_step": us,
-                       "serial_l2_trips_per_step": 2,
-                       "us_per_l2_trip": us / 2,
-                       "exchange": "each CTA stores one tagged sign word on its own 128-byte line; thread q of "
-                                   "every CTA polls CTA q's line until the tag of the step appears",
-                       "hbm_bytes_per_launch": 4.0 * n * n + 16.0 * n * R,
-                       "hbm_frac_of_launch": (4.0 * n * n + 16.0 * n * R) / (rp.kernel_ms_avg * 1e-3) / 1e9 / hbm}
+            traffic = NCU_TRAFFIC["plain-dsb-signs"] if n == 2000 and R == 1 else (None, None)
+            kernel = "signs_kernel (one launch per solve)"
+            note = ("achieved counts the algorithmic 4 N^2 bytes of J per SB step, but the +-1 couplings live in "
+                    "registers as bit planes for the whole launch and are read once (traffic); the kernel is not "
+                    "HBM-bound, see limiter")
+            limiter = {"kind": "a step's chain: sign words through distributed shared memory, then the rows' logic",
+                       "us_per_sb_step": 1e3 * rp.kernel_ms_avg / spl,
+                       "exchange": "each warp sends its 32 rows' sign word to every CTA of the cluster (st.async, "
+                                   "bytes counted on the receiver's mbarrier)",
+                       "hbm_bytes_per_launch": n * n / 4.0 + 16.0 * n * R,
+                       "hbm_frac_of_launch": (n * n / 4.0 + 16.0 * n * R) / (rp.kernel_ms_avg * 1e-3) / 1e9 / hbm}
         else:
             traffic = NCU_TRAFFIC["plain-dsb"] if n == 2000 and R == 1 else (None, None)
             kernel = "plain_step_kernel"
@@ -638,11 +634,10 @@ def run_batch(args, rank, world, local_rank):
             "kernel": "grouped_kernel (one launch per SB step)",
             "launch_ms": rp[0].kernel_ms_avg, "bytes_per_launch": bytes_per_launch,
             "peak_source": f"{src} HBM copy",
-            # the timed solves replay the step launches from a CUDA graph: per SB step, their time
-            # (init and final energies included) against the event-timed launch above bounds what a
-            # multi-step persistent launch could save (launch gaps and step-boundary tails)
-            "graph_ms_per_sb_step": total_ms / args.steps / sb_steps,
-            "gap_frac_bound": 1.0 - rp[0].kernel_ms_avg / (total_ms / args.steps / sb_steps)}
+            # the timed solves run sets of instances whose couplings stay in L2 for all steps in one launch
+            # (run_kernel), so their time per SB step, init and energies included, is below that of the
+            # event-timed launch above, the form that takes one step of every instance from HBM
+            "timed_ms_per_sb_step": total_ms / args.steps / sb_steps}
     # e2e: from host couplings every step through the public calls: sb_problem_wrap of each
     # instance (its coupling scan), then the batch (upload, convert, run, results back)
     import ctypes

@@ -299,11 +299,13 @@ int64_t sb_plan_footprint(const sb_problem *p, const sb_params *params);
 /* ---- batches: many instances of uneven size, solved together ----
  * The reference runs one instance per program run and its trials one after another
  * (SB/CUDA_GPU/m2_opt.cu:152). A batch advances every instance, with all of its replicas, by
- * grouped tensor-core launches, the step loop replayed from a CUDA graph (dSB, integer |J| <= 16).
- * Instances whose couplings are integers |J| <= 4 run on packed E2M1 operands (half the bytes), the
- * others on FP8 (params->operand_dtype SB_OPERAND_FP8 / SB_OPERAND_FP4 forces one type); each operand
- * bucket has one grouped launch per SB step, with its replica tile and work order chosen by timing
- * the candidates on the bucket itself (cached per shape). params is shared; instance k uses seed
+ * grouped tensor-core launches (dSB, integer |J| <= 16). Instances whose couplings are integers
+ * |J| <= 4 run on packed E2M1 operands (half the bytes), the others on packed E2M3
+ * (params->operand_dtype SB_OPERAND_FP8 / SB_OPERAND_FP6 / SB_OPERAND_FP4 forces one type). Each operand
+ * bucket runs in waves of instances whose couplings share L2, all steps of a wave in one launch; an
+ * instance with more work items than a wave holds takes one grouped launch per step, the replica tile
+ * and work order then chosen by timing the candidates on the bucket itself (cached per shape).
+ * params is shared; instance k uses seed
  * seed + k; results[k] is filled as sb_solve would fill it (arrays sized for instance k). The
  * problems must stay alive until sb_batch_destroy. */
 typedef struct sb_batch sb_batch;
@@ -318,9 +320,9 @@ sb_status sb_solve_batch(sb_ctx *ctx, const sb_problem *problems, int32_t count,
  * sb_submit queues a request and returns a ticket at once; the problem (and its J / h) must stay
  * alive until sb_poll has returned the request's final status. A worker thread admits queued
  * requests in arrival order while the context's HBM budget and in-flight limit allow, and
- * advances every admitted request together (one grouped tensor-core launch per step over all
+ * advances every admitted request together (grouped tensor-core launches of up to 64 steps over all
  * resident requests, each on its own schedule), so requests that arrive while others run join
- * them at the next step. Each request retires at its own step budget (energies, best spins, exact
+ * them at the next launch. Each request retires at its own step budget (energies, best spins, exact
  * host re-check) and its device memory goes to the next. dSB requests with integer |J| <= 16 use
  * the grouped engine; others are solved one at a time between steps. Results equal those of
  * sb_solve with the same parameters (field_mode SB_FIELD_TC for the grouped ones). */
