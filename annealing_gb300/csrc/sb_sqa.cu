@@ -555,7 +555,7 @@ extern "C" sb_status sb_sqa_solve(sb_ctx *ctx, const sb_problem *prob, const sb_
       const size_t bytes = (size_t)(M + d) * RS * 4 + sp_words * 4 + thr_words * 4 + (size_t)(M + d) * 8;
       if (bytes <= budget) S = M + d;
     }
-  if (S == 0 && !use_tc) return fail(ctx, SB_ERR_UNSUPPORTED, "sb_sqa_solve: trotter x n too large for one CTA's shared memory");
+  if (S == 0) return fail(ctx, SB_ERR_UNSUPPORTED, "sb_sqa_solve: trotter x n too large for one CTA's shared memory");
   const size_t smem = (size_t)S * RS * 4 + sp_words * 4 + thr_words * 4 + (size_t)S * 8;
   const int threads = 32 * ((M + kSqaSlicesPerWarp - 1) / kSqaSlicesPerWarp);
   cudaStream_t st = ctx->stream;
