@@ -54,6 +54,8 @@ struct sb_plan {
   // plain FP32 SB that fits one cooperative launch: the exchange lines of PlainPersist
   unsigned long long *dwords = nullptr;
   size_t words_bytes = 0;
+  uint8_t *dout = nullptr;      // results, packed
+  uint64_t seed = 0;            // of the run in progress
   uint32_t *dplanes = nullptr;  // dSB with small integer couplings: their bit planes, and how many magnitudes
   bool cluster = false;         // the plain FP32 steps run in clusters (sb_cluster.cuh)
   int planes = 0;               // they have (0: the couplings uploaded are not such)
@@ -224,8 +226,9 @@ void plan_free_device(sb_plan *pl) {
   cudaFree(pl->dx[0]);
   cudaFree(pl->dx[1]);
   cudaFree(pl->dy);
-  cudaFree(pl->denergy);
-  cudaFree(pl->dstatus);
+  cudaFree(pl->denergy);  // and the status word behind it
+  cudaFree(pl->dout);
+  pl->dout = nullptr;
   cudaFree(pl->dpump);
   cudaFree(pl->dxk);
   cudaFree(pl->dek);
@@ -244,6 +247,11 @@ void plan_free_device(sb_plan *pl) {
   pl->denergy = nullptr;
   pl->dstatus = nullptr;
   pl->ev0 = pl->ev1 = nullptr;
+}
+
+// The step launch makes the initial state itself.
+bool makes_init(const sb_plan *pl) {
+  return pl->prm.init_mode != SB_INIT_REFERENCE && (pl->planes || (pl->cluster && pl->prm.variant != SB_ASB));
 }
 
 // The plain FP32 steps of a solve run in one launch.
@@ -326,8 +334,10 @@ sb_status plan_create(sb_ctx *ctx, const sb_problem *p, const sb_params *prm, sb
     PLAN_ALLOC(pl->dx[1], xs);
   }
   PLAN_ALLOC(pl->dy, xs);
-  PLAN_ALLOC(pl->denergy, energy_slots(*prm) * (size_t)pl->R * sizeof(double));
-  PLAN_ALLOC(pl->dstatus, sizeof(uint32_t));
+  // the energies and, behind them, the status word: one reset a run
+  PLAN_ALLOC(pl->denergy, (energy_slots(*prm) * (size_t)pl->R + 1) * sizeof(double));
+  pl->dstatus = reinterpret_cast<uint32_t *>(pl->denergy + energy_slots(*prm) * (size_t)pl->R);
+  PLAN_ALLOC(pl->dout, sbk::packed_results_bytes(pl->n, pl->R));
   PLAN_ALLOC(pl->dpump, (size_t)(prm->steps > 0 ? prm->steps : 1) * sizeof(float));
   // plain FP32 solves whose rows fit one co-resident grid run every step in one launch (N=2000,
   // 1000 steps: dSB 5.7 -> 1.4 ms, its signs one tagged word per CTA; bSB 6.3 -> 1.5 ms and aSB
@@ -438,6 +448,8 @@ cudaError_t enqueue_loop(sb_plan *pl, cudaStream_t st, std::vector<cudaEvent_t> 
       a.dta0 = pl->dta0;
       a.steps = p.steps;
       a.status = pl->dstatus;
+      a.init = makes_init(pl) ? 1 : 0;
+      a.seed = pl->seed;
       if (evs) cudaEventRecord((*evs)[0], st);
       const cudaError_t e = sbk::launch_signs(a, pl->planes, st);
       if (e != cudaSuccess) return e;
@@ -476,6 +488,8 @@ cudaError_t enqueue_loop(sb_plan *pl, cudaStream_t st, std::vector<cudaEvent_t> 
       a.steps = p.steps;
       a.words = pl->dwords;
       a.status = pl->dstatus;
+      a.init = makes_init(pl) ? 1 : 0;
+      a.seed = pl->seed;
       if (evs) cudaEventRecord((*evs)[0], st);
       if ((e = pl->cluster ? sbk::launch_plain_cluster(a, st) : sbk::launch_plain_persist(a, st)) != cudaSuccess) return e;
       if (evs) cudaEventRecord((*evs)[1], st);
@@ -547,14 +561,16 @@ sb_status plan_run(sb_plan *pl, uint64_t seed, sb_result *res, std::string &err)
   const bool tr = needs_trace(p);
   const auto t_start = std::chrono::steady_clock::now();
   int64_t launches = 0;
-  SB_CUDA(cudaMemsetAsync(pl->dstatus, 0, sizeof(uint32_t), st));
-  SB_CUDA(cudaMemsetAsync(pl->denergy, 0, energy_slots(p) * (size_t)R * sizeof(double), st));
+  SB_CUDA(cudaMemsetAsync(pl->denergy, 0, (energy_slots(p) * (size_t)R + 1) * sizeof(double), st));
   SB_CUDA(cudaEventRecord(pl->ev0, st));
-  if (p.init_mode == SB_INIT_REFERENCE)
-    SB_CUDA(sbk::launch_init_reference(pl->dx[0], pl->dy, n, R, pl->xp, st));
-  else
-    SB_CUDA(sbk::launch_init_uniform(pl->dx[0], pl->dy, n, R, pl->xp, seed, st));
-  ++launches;
+  pl->seed = seed;
+  if (!makes_init(pl)) {
+    if (p.init_mode == SB_INIT_REFERENCE)
+      SB_CUDA(sbk::launch_init_reference(pl->dx[0], pl->dy, n, R, pl->xp, st));
+    else
+      SB_CUDA(sbk::launch_init_uniform(pl->dx[0], pl->dy, n, R, pl->xp, seed, st));
+    ++launches;
+  }
   if (p.variant == SB_ASB) {
     if (tr) {
       SB_CUDA(enqueue_energy(pl, pl->dx[0], pl->denergy, st, -1));
@@ -628,10 +644,34 @@ sb_status plan_run(sb_plan *pl, uint64_t seed, sb_result *res, std::string &err)
   ++launches;
   std::vector<double> e_final((size_t)R);
   uint32_t status = 0;
+  // The energies stand as they are and nothing before them needs the host: the best replica is found and packed with
+  // its spins on the device, and everything comes back behind one synchronisation (two, with a copy between them,
+  // took 25 us of a small solve). The other forms keep their launches.
+  const bool packed = !tr && (!refine || R <= kTopK) && (makes_init(pl) || pl->mode == SB_FIELD_TC);
+  std::vector<uint8_t> pack(packed ? sbk::packed_results_bytes(n, R) : 0);
+  auto copy_states = [&]() -> cudaError_t {
+    cudaError_t e = cudaSuccess;
+    if (res->final_x)
+      e = cudaMemcpy2DAsync(res->final_x, (size_t)n * sizeof(float), final_x(pl), (size_t)pl->xp * sizeof(float),
+                            (size_t)n * sizeof(float), (size_t)R, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess && res->final_y)
+      e = cudaMemcpy2DAsync(res->final_y, (size_t)n * sizeof(float), pl->dy, (size_t)pl->xp * sizeof(float),
+                            (size_t)n * sizeof(float), (size_t)R, cudaMemcpyDeviceToHost, st);
+    return e;
+  };
+  if (packed) {
+    SB_CUDA(sbk::launch_results(final_slot, final_x(pl), n, R, pl->xp, pl->dout, st));
+    ++launches;
+    SB_CUDA(cudaEventRecord(pl->ev1, st));
+  }
   sbh::touch_pages(res->final_x, (size_t)R * n * sizeof(float));
   sbh::touch_pages(res->final_y, (size_t)R * n * sizeof(float));
-  SB_CUDA(cudaMemcpyAsync(e_final.data(), final_slot, (size_t)R * sizeof(double),
-                          cudaMemcpyDeviceToHost, st));
+  if (packed) {
+    SB_CUDA(cudaMemcpyAsync(pack.data(), pl->dout, pack.size(), cudaMemcpyDeviceToHost, st));
+    SB_CUDA(copy_states());
+  } else {
+    SB_CUDA(cudaMemcpyAsync(e_final.data(), final_slot, (size_t)R * sizeof(double), cudaMemcpyDeviceToHost, st));
+  }
   SB_CUDA(cudaMemcpyAsync(&status, pl->dstatus, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
   SB_CUDA(cudaStreamSynchronize(st));
   bool refined = false;
@@ -660,7 +700,7 @@ sb_status plan_run(sb_plan *pl, uint64_t seed, sb_result *res, std::string &err)
     for (int q = 1; q < kTopK; ++q)
       if (e_final[order[q]] < e_final[order_best]) order_best = order[q];
   }
-  SB_CUDA(cudaEventRecord(pl->ev1, st));
+  if (!packed) SB_CUDA(cudaEventRecord(pl->ev1, st));
   if (status != 0) {
     err = sbh::device_status_text(status);
     return (status & sbk::kErrWaitTimeout) ? SB_ERR_TIMEOUT : SB_ERR_CUDA;
@@ -669,32 +709,35 @@ sb_status plan_run(sb_plan *pl, uint64_t seed, sb_result *res, std::string &err)
   // the same state as one of them but outside the top kTopK keeps its FP32 energy, which may sit a
   // rounding below the exact one
   int best = refined ? order_best : 0;
-  if (!refined)
-    for (int r = 1; r < R; ++r)
-      if (e_final[r] < e_final[best]) best = r;
-  SB_CUDA(cudaEventSynchronize(pl->ev1));
-  std::vector<float> xb((size_t)n);
-  SB_CUDA(cudaMemcpyAsync(xb.data(), final_x(pl) + (size_t)best * pl->xp, (size_t)n * sizeof(float),
-                          cudaMemcpyDeviceToHost, st));
-  if (res->final_x)
-    SB_CUDA(cudaMemcpy2DAsync(res->final_x, (size_t)n * sizeof(float), final_x(pl),
-                              (size_t)pl->xp * sizeof(float), (size_t)n * sizeof(float), (size_t)R,
-                              cudaMemcpyDeviceToHost, st));
-  if (res->final_y)
-    SB_CUDA(cudaMemcpy2DAsync(res->final_y, (size_t)n * sizeof(float), pl->dy,
-                              (size_t)pl->xp * sizeof(float), (size_t)n * sizeof(float), (size_t)R,
-                              cudaMemcpyDeviceToHost, st));
+  std::vector<int8_t> spins((size_t)n);
+  std::vector<float> xb;
+  if (packed) {
+    memcpy(e_final.data(), pack.data(), (size_t)R * sizeof(double));
+    int64_t b;
+    memcpy(&b, pack.data() + 8 * (size_t)R, sizeof(b));
+    best = (int)b;
+    memcpy(spins.data(), pack.data() + 8 * ((size_t)R + 1), (size_t)n);
+  } else {
+    if (!refined)
+      for (int r = 1; r < R; ++r)
+        if (e_final[r] < e_final[best]) best = r;
+    SB_CUDA(cudaEventSynchronize(pl->ev1));
+    xb.resize((size_t)n);
+    SB_CUDA(cudaMemcpyAsync(xb.data(), final_x(pl) + (size_t)best * pl->xp, (size_t)n * sizeof(float),
+                            cudaMemcpyDeviceToHost, st));
+    SB_CUDA(copy_states());
+  }
   std::vector<double> tr_all;
   if (tr && (res->energy_trace || res->energy_trace_all)) {
     tr_all.resize(energy_slots(p) * (size_t)R);
     SB_CUDA(cudaMemcpyAsync(tr_all.data(), pl->denergy, tr_all.size() * sizeof(double),
                             cudaMemcpyDeviceToHost, st));
   }
-  SB_CUDA(cudaStreamSynchronize(st));
+  if (!packed) SB_CUDA(cudaStreamSynchronize(st));
   float dev_ms = 0.0f;
   SB_CUDA(cudaEventElapsedTime(&dev_ms, pl->ev0, pl->ev1));
-  std::vector<int8_t> spins((size_t)n);
-  for (int i = 0; i < n; ++i) spins[i] = xb[i] > 0.0f ? 1 : -1;
+  if (!packed)
+    for (int i = 0; i < n; ++i) spins[i] = xb[i] > 0.0f ? 1 : -1;
   if (res->best_spins) memcpy(res->best_spins, spins.data(), (size_t)n);
   if (res->replica_energies) memcpy(res->replica_energies, e_final.data(), (size_t)R * sizeof(double));
   if (!tr_all.empty()) {

@@ -19,6 +19,7 @@
 #include "sb_grouped.h"
 #include "sb_host.h"
 #include "sb_init.cuh"
+#include "sb_results.cuh"
 #include "sb_run.cuh"
 #include "sb_run.h"
 
@@ -216,35 +217,10 @@ __global__ void g_zero_energies_kernel(const GInst *insts) {
   for (int r = threadIdx.x; r < in->R; r += blockDim.x) in->energy[r] = 0.0;
 }
 
-// An instance's energies, the first replica of the least one and its spins, at out + in->out: R doubles, the index
-// (8 bytes), n bytes. One block per instance.
+// Every instance's results at out + in->out, one block per instance.
 __global__ void g_results_kernel(const GInst *insts, uint8_t *out) {
-  __shared__ double chunk[256];
-  __shared__ int best_sh;
   const GInst *in = insts + blockIdx.x;
-  uint8_t *dst = out + in->out;
-  double least = 0.0;  // thread 0's
-  int best = 0;
-  for (int r0 = 0; r0 < in->R; r0 += 256) {
-    const int r = r0 + (int)threadIdx.x, m = min(256, in->R - r0);
-    if (r < in->R) chunk[threadIdx.x] = reinterpret_cast<double *>(dst)[r] = in->energy[r];
-    __syncthreads();
-    if (threadIdx.x == 0)
-      for (int k = 0; k < m; ++k)
-        if (r0 + k == 0 || chunk[k] < least) {
-          least = chunk[k];
-          best = r0 + k;
-        }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    best_sh = best;
-    *reinterpret_cast<int64_t *>(dst + 8 * (size_t)in->R) = best;
-  }
-  __syncthreads();
-  const float *x = in->x + (size_t)best_sh * in->xp;
-  int8_t *s = reinterpret_cast<int8_t *>(dst) + 8 * ((size_t)in->R + 1);
-  for (int i = threadIdx.x; i < in->n; i += blockDim.x) s[i] = x[i] > 0.0f ? 1 : -1;
+  pack_results(in->energy, in->x, in->n, in->R, in->xp, out + in->out);
 }
 
 bool grouped_kernel_for(int nr, int emode, int op, const void **k, size_t *smem) {
@@ -672,7 +648,7 @@ sb_status Grouped::sync_tables(std::string &err) {
   for (size_t i = 0; i < insts.size(); ++i) {
     GHost &g = insts[i];
     g.out = out_bytes;
-    out_bytes += 8 * ((size_t)g.R + 1) + ((size_t)g.n + 7) / 8 * 8;
+    out_bytes += packed_results_bytes(g.n, g.R);
     descs[i] = g.desc;
     descs[i].index = g.tag;
     descs[i].out = g.out;

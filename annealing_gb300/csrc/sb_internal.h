@@ -74,6 +74,9 @@ struct PlainPersist {
   uint32_t *rng;
   int32_t *samples;
   float noise, keep, mix;
+  // clusters, bSB and dSB: as SignSolve
+  int init;
+  uint64_t seed;
 };
 constexpr int kPersistRows = 16;
 constexpr int kPersistMaxJp = 2048;
@@ -98,6 +101,8 @@ struct SignSolve {
   float c0, dt, dta0;
   int steps;
   uint32_t *status;
+  int init;                   // 1: x(0), y(0) are the hash-mode initial state of `seed`, x_in and y are not read
+  uint64_t seed;
 };
 constexpr int kSignsMaxN = 2048;
 constexpr int kSignsOneCta = 512;  // spins of the one-CTA form with one magnitude plane
@@ -106,6 +111,10 @@ int sign_planes(int n, int R, int max_abs_j);
 size_t sign_plane_bytes(int n);  // for any couplings that n allows
 cudaError_t launch_sign_planes(const float *J, int n, int jp, int P, uint32_t *planes, cudaStream_t st);
 cudaError_t launch_signs(const SignSolve &a, int P, cudaStream_t st);
+
+// R energies, the first least one's index and its replica's spins (sb_results.cuh) at out, packed_results_bytes of it.
+inline size_t packed_results_bytes(int n, int R) { return 8 * ((size_t)R + 1) + ((size_t)n + 7) / 8 * 8; }
+cudaError_t launch_results(const double *e, const float *x, int n, int R, int xp, uint8_t *out, cudaStream_t st);
 
 struct PlainEnergy {
   int n, R, jp, xp, rb;

@@ -28,6 +28,7 @@
 #include "sb_internal.h"
 #include "sb_math.cuh"
 #include "sb_ptx.cuh"
+#include "sb_results.cuh"
 
 namespace sbk {
 namespace {
@@ -1169,6 +1170,18 @@ cudaError_t launch_plain_persist(const PlainPersist &a, cudaStream_t st) {
     case 3: return cudaLaunchKernelEx(&cfg, plain_persist_kernel<3>, a);
   }
   return cudaErrorInvalidValue;
+}
+
+namespace {
+__global__ void __launch_bounds__(1024) results_kernel(const double *e, const float *x, int n, int R, int xp, uint8_t *out) {
+  pack_results(e, x, n, R, xp, out);
+}
+}  // namespace
+
+cudaError_t launch_results(const double *e, const float *x, int n, int R, int xp, uint8_t *out, cudaStream_t st) {
+  const int most = n > R ? n : R;
+  results_kernel<<<1, most >= 1024 ? 1024 : (most + 31) / 32 * 32, 0, st>>>(e, x, n, R, xp, out);
+  return cudaGetLastError();
 }
 
 namespace {

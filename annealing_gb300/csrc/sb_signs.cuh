@@ -53,8 +53,9 @@ __global__ void __launch_bounds__(CLUSTER ? kClusterRows : kSignsOneCta) signs_k
   const size_t k_xy = (size_t)r * a.xp + row;
   float x = 0.0f, y = 0.0f;
   if (have && SB_BOUNDS(k_xy < (size_t)a.R * a.xp, a.status)) {
-    x = a.x_in[k_xy];
-    y = a.y[k_xy];
+    const uint64_t e = 2 * ((uint64_t)r * a.n + row);
+    x = a.init ? uniform_value(a.seed, e) : a.x_in[k_xy];
+    y = a.init ? uniform_value(a.seed, e + 1) : a.y[k_xy];
   }
   const float hv = have && a.h ? a.h[row] : 0.0f;
   for (int k = tid; k < 2 * kMaxWords; k += (int)blockDim.x) (&sg[0][0])[k] = 0u;
