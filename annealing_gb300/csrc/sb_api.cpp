@@ -251,7 +251,8 @@ void plan_free_device(sb_plan *pl) {
 
 // The step launch makes the initial state itself.
 bool makes_init(const sb_plan *pl) {
-  return pl->prm.init_mode != SB_INIT_REFERENCE && (pl->planes || (pl->cluster && pl->prm.variant != SB_ASB));
+  return pl->prm.init_mode != SB_INIT_REFERENCE && pl->prm.variant != SB_ASB &&
+         (pl->planes || pl->cluster || pl->dwords);
 }
 
 // The plain FP32 steps of a solve run in one launch.
@@ -265,9 +266,14 @@ size_t energy_slots(const sb_params &p) { return needs_trace(p) ? (size_t)p.step
 sb_status upload_problem(sb_plan *pl, const sb_problem *p, std::string &err) {
   cudaStream_t st = pl->ctx->stream;
   const int n = pl->n;
-  SB_CUDA(cudaMemsetAsync(pl->dJ, 0, (size_t)n * pl->jp * sizeof(float), st));
-  SB_CUDA(cudaMemcpy2DAsync(pl->dJ, (size_t)pl->jp * sizeof(float), p->J, (size_t)n * sizeof(float),
-                            (size_t)n * sizeof(float), (size_t)n, cudaMemcpyHostToDevice, st));
+  // (a row copy from pageable memory takes twice the time of a plain one: N = 2000 158 us with its reset against 98)
+  if (pl->jp == n) {
+    SB_CUDA(cudaMemcpyAsync(pl->dJ, p->J, (size_t)n * n * sizeof(float), cudaMemcpyHostToDevice, st));
+  } else {
+    SB_CUDA(cudaMemsetAsync(pl->dJ, 0, (size_t)n * pl->jp * sizeof(float), st));
+    SB_CUDA(cudaMemcpy2DAsync(pl->dJ, (size_t)pl->jp * sizeof(float), p->J, (size_t)n * sizeof(float),
+                              (size_t)n * sizeof(float), (size_t)n, cudaMemcpyHostToDevice, st));
+  }
   if (p->h) SB_CUDA(cudaMemcpyAsync(pl->dh, p->h, (size_t)n * sizeof(float), cudaMemcpyHostToDevice, st));
   if (pl->mode == SB_FIELD_TC) {
     if (pl->tc) {
@@ -647,7 +653,8 @@ sb_status plan_run(sb_plan *pl, uint64_t seed, sb_result *res, std::string &err)
   // The energies stand as they are and nothing before them needs the host: the best replica is found and packed with
   // its spins on the device, and everything comes back behind one synchronisation (two, with a copy between them,
   // took 25 us of a small solve). The other forms keep their launches.
-  const bool packed = !tr && (!refine || R <= kTopK) && (makes_init(pl) || pl->mode == SB_FIELD_TC);
+  const bool packed = !tr && (!refine || R <= kTopK) &&
+                      (makes_init(pl) || pl->mode == SB_FIELD_TC || p.variant == SB_ASB);
   std::vector<uint8_t> pack(packed ? sbk::packed_results_bytes(n, R) : 0);
   auto copy_states = [&]() -> cudaError_t {
     cudaError_t e = cudaSuccess;

@@ -74,7 +74,7 @@ struct PlainPersist {
   uint32_t *rng;
   int32_t *samples;
   float noise, keep, mix;
-  // clusters, bSB and dSB: as SignSolve
+  // bSB and dSB: as SignSolve
   int init;
   uint64_t seed;
 };

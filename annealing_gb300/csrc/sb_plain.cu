@@ -835,8 +835,9 @@ __global__ void __launch_bounds__(kPersistThreads, 1) plain_persist_kernel(Plain
   const size_t k_xy = (size_t)r * a.xp + row;
   float x = 0.0f, y = 0.0f;
   if (have && SB_BOUNDS(k_xy < (size_t)a.R * a.xp, a.status)) {
-    x = a.x_in[k_xy];
-    if constexpr (VARIANT != 3) y = a.y[k_xy];
+    const uint64_t e = 2 * ((uint64_t)r * a.n + row);
+    x = a.init ? uniform_value(a.seed, e) : a.x_in[k_xy];
+    if constexpr (VARIANT != 3) y = a.init ? uniform_value(a.seed, e + 1) : a.y[k_xy];
   }
   const float hv = (have && a.h) ? a.h[row] : 0.0f;
   // NMFA: the row norm, the spin's XORWOW words and the stage's second Gaussian sample (drawn with
