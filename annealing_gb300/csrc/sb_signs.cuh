@@ -13,8 +13,8 @@
 // Popcounts run at a quarter of the logic rate, so carry-save adders fold four masked words into two popcounts.
 // us per step of 1000, against the kernels before it (signs through L2, or one launch per step where its grid is
 // not co-resident): J = +-1, one replica n = 128 0.98 -> 0.18, n = 512 1.27 -> 0.40, n = 513 1.28 -> 0.58,
-// n = 1000 1.38 -> 0.58, n = 2000 1.57 -> 0.75; twelve replicas n = 1000 8.2 -> 0.62, n = 2000 16.8 -> 0.88; |J| <= 7
-// n = 128 0.98 -> 0.26, n = 512 1.25 -> 0.49, n = 1000 1.38 -> 0.90. 100 replicas of n = 2000 95 -> 6.0 (50 steps).
+// n = 1000 1.38 -> 0.52, n = 2000 1.57 -> 0.71; twelve replicas n = 1000 8.2 -> 0.6, n = 2000 16.8 -> 0.81; |J| <= 7
+// n = 128 0.98 -> 0.26, n = 512 1.25 -> 0.49, n = 1000 1.38 -> 0.84. 100 replicas of n = 2000 95 -> 6.0 (50 steps).
 // A cluster's step is some 0.45 us of exchange, the rest its 128 rows' logic, one warp to a scheduler.
 // Replicas are independent clusters: nothing waits across them, so any number runs.
 #pragma once
@@ -33,7 +33,7 @@ __device__ __forceinline__ void st_async_u32(uint32_t caddr, uint32_t v, uint32_
 // W: words of a row's planes in registers (a multiple of four, at least a.words), P magnitude planes.
 template <int W, int P, bool CLUSTER>
 __global__ void __launch_bounds__(CLUSTER ? kClusterRows : kSignsOneCta) signs_kernel(const __grid_constant__ SignSolve a) {
-  constexpr int kBlock = W < 16 ? W : 16;  // words a branch covers
+  constexpr int kBlock = W <= 48 ? W : 32;  // words a branch covers (sixteen: n = 1000 0.56 us a step against 0.52)
   __shared__ __align__(16) uint32_t sg[2][kMaxWords];  // sign words (bit set: -1) of a step, by parity
   __shared__ __align__(8) uint64_t full[2];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, r = blockIdx.y;
@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(CLUSTER ? kClusterRows : kSignsOneCta) signs_k
     }
 #pragma unroll
     for (int b = 0; b < W; b += kBlock)
-      if (b < a.words) {  // a branch for every four words kept their chains apart: 76 clocks a piece
+      if (b < a.words) {  // a branch for every four words kept their chains apart: 1.14 us at n = 2000
 #pragma unroll
         for (int q = b / 4; q < (b + kBlock) / 4; ++q) {
           const uint4 s = s4[q];
