@@ -56,7 +56,7 @@ struct sb_plan {
   size_t words_bytes = 0;
   uint8_t *dout = nullptr;      // results, packed
   uint64_t seed = 0;            // of the run in progress
-  uint32_t *dplanes = nullptr;  // dSB with small integer couplings: their bit planes, and how many magnitudes
+  uint32_t *dplanes = nullptr;  // dSB with integer couplings up to 127: their bit planes, and how many magnitudes
   bool cluster = false;         // the plain FP32 steps run in clusters (sb_cluster.cuh)
   int planes = 0;               // they have (0: the couplings uploaded are not such)
   float *dxk = nullptr;    // [kTopK][xp] rows of the best candidates (real-valued J)
@@ -121,14 +121,15 @@ sb_status check_params(const sb_problem *p, const sb_params *prm, std::string &e
 //   0.74 / 2.05, R = 512 (134e6) 1.36 / 1.84, R = 1000 2.23 / 1.85; |J| <= 3 n = 256 R = 1000 1.41 / 1.71;
 //   a cluster, 64e6: n = 700 R = 100 0.99 / 2.33, n = 1000 R = 64 0.88 / 2.21, n = 513 R = 300 (79e6) 2.10 / 2.22,
 //   R = 512 3.05 / 2.22; |J| <= 3 n = 513 R = 100 1.57 / 2.25, R = 200 (105e6) 2.56 / 2.30;
-//   |J| of 5 to 7, 300e6: n = 256 R = 1000 1.73 / 7.14, n = 700 R = 200 4.22 / 8.68, n = 513 R = 512 (404e6) 8.11 / 8.44.
+//   |J| of 5 to 127, 300e6: n = 88 R = 599 |J| <= 16 0.45 / 7.2, n = 256 R = 600 |J| <= 127 (275e6) 2.03 / 8.01,
+//   n = 512 R = 100 1.71 / 8.51; |J| <= 7 n = 256 R = 1000 1.73 / 7.14, n = 700 R = 200 4.22 / 8.68, n = 513 R = 512 (404e6) 8.11 / 8.44.
 bool signs_beat_tc(const sb_problem *p, const sb_params *prm) {
   if (prm->variant != SB_DSB || prm->trace || prm->trace_all || prm->steps <= 0 || !p->integer_valued ||
       prm->operand_dtype != SB_OPERAND_AUTO)
     return false;
   const char *env = getenv("SB_PLAIN_PERSIST");
   if (env && env[0] == '0') return false;
-  const int n = p->n, R = prm->replicas, P = p->max_abs_j <= 1 ? 1 : p->max_abs_j <= 3 ? 2 : 3;
+  const int n = p->n, R = prm->replicas, P = sbk::planes_of(p->max_abs_j);
   // (what the tensor-core kernel has no room for, a unit of 128 x 128 to an SM, is not taken here either)
   if ((int64_t)((n + 127) / 128) * ((R + 127) / 128) > 128) return false;
   const bool one_cta = n <= (P == 1 ? sbk::kSignsOneCta : sbk::kSignsOneCta / 2);
@@ -353,7 +354,7 @@ sb_status plan_create(sb_ctx *ctx, const sb_problem *p, const sb_params *prm, sb
   if (mode == SB_FIELD_FP32 && !needs_trace(*prm) && prm->steps > 0) {
     const char *env = getenv("SB_PLAIN_PERSIST");
     const bool want = !(env && env[0] == '0');
-    // dSB with couplings up to 3 or 7: no exchange through L2 at all (sb_signs.cuh)
+    // dSB with integer couplings: no exchange through L2 at all (sb_signs.cuh)
     if (want && prm->variant == SB_DSB && p->integer_valued && sbk::sign_planes(pl->n, pl->R, p->max_abs_j))
       PLAN_ALLOC(pl->dplanes, sbk::sign_plane_bytes(pl->n));
     pl->cluster = want && sbk::plain_cluster_fits(prm->variant, pl->n, pl->R, pl->jp);

@@ -90,7 +90,7 @@ constexpr int kClusterMaxN = 512;
 bool plain_cluster_fits(int variant, int n, int R, int jp);
 cudaError_t launch_plain_cluster(const PlainPersist &a, cudaStream_t st);
 
-// Plain FP32 dSB with small integer couplings, the whole solve in one launch of independent clusters (sb_signs.cuh).
+// Plain FP32 dSB with integer couplings up to 127, the whole solve in one launch of independent clusters (sb_signs.cuh).
 struct SignSolve {
   int n, R, xp, words;        // words = ceil(n / 32)
   const uint32_t *planes;     // [P + 1][words][n] from launch_sign_planes
@@ -106,6 +106,12 @@ struct SignSolve {
 };
 constexpr int kSignsMaxN = 2048;
 constexpr int kSignsOneCta = 512;  // spins of the one-CTA form with one magnitude plane
+// Magnitude planes of couplings up to max_abs_j.
+inline int planes_of(int max_abs_j) {
+  int P = 1;
+  while (max_abs_j >> P) ++P;
+  return P;
+}
 // Magnitude planes of the one-launch sign kernel for couplings up to max_abs_j, or 0 when it does not take the shape.
 int sign_planes(int n, int R, int max_abs_j);
 size_t sign_plane_bytes(int n);  // for any couplings that n allows

@@ -1219,7 +1219,16 @@ bool cluster_runs(const void *k, const cudaLaunchConfig_t &cfg) {
 }
 
 const void *signs_kernel_for(int n, int P) {
-  return P == 1 ? signs::kernel_for<1>(n) : P == 2 ? signs::kernel_for<2>(n) : signs::kernel_for<3>(n);
+  switch (P) {
+    case 1: return signs::kernel_for<1>(n);
+    case 2: return signs::kernel_for<2>(n);
+    case 3: return signs::kernel_for<3>(n);
+    case 4: return signs::kernel_for<4>(n);
+    case 5: return signs::kernel_for<5>(n);
+    case 6: return signs::kernel_for<6>(n);
+    case 7: return signs::kernel_for<7>(n);
+  }
+  return nullptr;
 }
 // Launch shape for R solves of n spins.
 void signs_config(int n, int R, int P, cudaLaunchConfig_t &cfg, cudaLaunchAttribute &attr) {
@@ -1231,8 +1240,8 @@ void signs_config(int n, int R, int P, cudaLaunchConfig_t &cfg, cudaLaunchAttrib
 }  // namespace
 
 int sign_planes(int n, int R, int max_abs_j) {
-  if (n < 1 || n > kSignsMaxN || R < 1 || R > 65535 || max_abs_j > 7) return 0;
-  const int P = max_abs_j <= 1 ? 1 : max_abs_j <= 3 ? 2 : 3;
+  if (n < 1 || n > kSignsMaxN || R < 1 || R > 65535 || max_abs_j > 127) return 0;
+  const int P = planes_of(max_abs_j);
   const void *k = signs_kernel_for(n, P);
   if (!k) return 0;  // more planes than registers hold
   if (signs::one_cta(n, P)) return P;
@@ -1273,7 +1282,7 @@ cudaError_t launch_plain_cluster(const PlainPersist &a, cudaStream_t st) {
 
 size_t sign_plane_bytes(int n) {
   const size_t words = (size_t)(n + 31) / 32;
-  return (words <= 32 ? 4 : 2) * words * n * sizeof(uint32_t);
+  return (words <= 16 ? 8 : words <= 32 ? 5 : 2) * words * n * sizeof(uint32_t);
 }
 
 cudaError_t launch_sign_planes(const float *J, int n, int jp, int P, uint32_t *planes, cudaStream_t st) {

@@ -1,10 +1,10 @@
-// Plain dSB with small integer couplings, the whole solve in one launch without a trip through L2 between steps
+// Plain dSB with integer couplings up to 127, the whole solve in one launch without a trip through L2 between steps
 // (SignSolve). A dSB step needs only the signs of the other spins, so with J as bit planes (per 32 columns a sign
 // word and P magnitude words) a field is
 //   f_i = sum_j |J_ij| - 2 sum_k 2^(k-1) popc(mag_k & (sign ^ s)),
 // an exact integer, as the FP32 sums of the other kernels are (n max |J| < 2^24): the same bits. A thread owns a
 // row: its planes in registers, x and y too, no reduction; a warp's ballot is the sign word of its 32 rows.
-//   * n <= 512 (one magnitude plane; 256 with two or three): one CTA holds every row; a step is a few broadcast reads, popcounts, the update, a ballot
+//   * n <= 512 (one magnitude plane; 256 with more): one CTA holds every row; a step is a few broadcast reads, popcounts, the update, a ballot
 //     and a barrier.
 //   * above, a cluster of ceil(n / 128) CTAs of 128 rows: each warp sends its word to every CTA of the cluster with
 //     st.async, counted in bytes on the receiver's mbarrier (one per parity of the step). A warp sends step t + 2's
@@ -15,7 +15,7 @@
 // not co-resident): J = +-1, one replica n = 128 0.98 -> 0.18, n = 512 1.27 -> 0.40, n = 513 1.28 -> 0.58,
 // n = 1000 1.38 -> 0.52, n = 2000 1.57 -> 0.71; twelve replicas n = 1000 8.2 -> 0.6, n = 2000 16.8 -> 0.81; |J| <= 7
 // n = 128 0.98 -> 0.26, n = 512 1.25 -> 0.49, n = 1000 1.38 -> 0.84. 100 replicas of n = 2000 95 -> 6.0 (50 steps).
-// A cluster's step is some 0.45 us of exchange, the rest its 128 rows' logic, one warp to a scheduler.
+// |J| <= 127 (seven planes) n = 128 0.37, n = 256 0.64, n = 512 0.78. A cluster's step is some 0.45 us of exchange, the rest its 128 rows' logic, one warp to a scheduler.
 // Replicas are independent clusters: nothing waits across them, so any number runs.
 #pragma once
 
@@ -175,7 +175,8 @@ const void *kernel_for(int n) {
   if (words <= 4) return reinterpret_cast<const void *>(&signs_kernel<4, P, false>);
   if (words <= 8) return reinterpret_cast<const void *>(&signs_kernel<8, P, false>);
   if (words <= 16) return reinterpret_cast<const void *>(&signs_kernel<16, P, P != 1>);
-  if (words <= 32) return reinterpret_cast<const void *>(&signs_kernel<32, P, true>);
+  if constexpr (P <= 4)
+    if (words <= 32) return reinterpret_cast<const void *>(&signs_kernel<32, P, true>);
   if constexpr (P == 1) {
     if (words <= 48) return reinterpret_cast<const void *>(&signs_kernel<48, P, true>);
     return reinterpret_cast<const void *>(&signs_kernel<64, P, true>);

@@ -77,12 +77,12 @@ typedef enum sb_variant { SB_ASB = 0, SB_BSB = 1, SB_DSB = 2 } sb_variant;
 
 /* How the field J*v is computed.
  *  SB_FIELD_AUTO: tensor cores when replicas >= 32 and the problem allows an exact/declared
- *                 precision, otherwise the plain FP32 path; dSB with integer |J| <= 7 whose bit
+ *                 precision, otherwise the plain FP32 path; dSB with integer couplings whose bit
  *                 planes are faster (n^2 x replicas small: up to 64 to 300 million) takes the
  *                 plain path too (the same bits).
- *  SB_FIELD_FP32: the plain fused FP32 path (the drop-in form). dSB with integer |J| <= 7 and
- *                 n <= 1024 (|J| <= 1: n <= 2048) runs the whole solve in one launch on bit planes of
- *                 J (exact integer fields). Otherwise the whole solve is one cooperative launch when
+ *  SB_FIELD_FP32: the plain fused FP32 path (the drop-in form). dSB with integer |J| <= 127 and
+ *                 n <= 512 (|J| <= 15: n <= 1024, |J| <= 1: n <= 2048) runs the whole solve in one launch
+ *                 on bit planes of J (exact integer fields). Otherwise the whole solve is one cooperative launch when
  *                 the rows fit one co-resident grid (n <= 2048, ceil(n / 16) x replicas CTAs on the
  *                 SMs), else, and with an energy trace, one launch per step; the same bits each way
  *                 (environment SB_PLAIN_PERSIST=0 keeps one launch per step).

@@ -1,4 +1,4 @@
-"""Plain FP32 dSB with small integer couplings in one launch (bit planes and popcounts; one CTA up to 512 spins, a
+"""Plain FP32 dSB with integer couplings up to 127 in one launch (bit planes and popcounts; one CTA up to 512 spins, a
 cluster above) against the general one-launch-per-step kernel, bit for bit: the fields are exact integers in both.
 
 Sizes sit on the edges of words, register forms, the one-CTA limit and the clusters (up to sixteen CTAs), and on both
@@ -45,7 +45,13 @@ def _solve(prob, n, R, steps, seed, persist, monkeypatch):
     (1900, 1, 3, 40, True),    # fifteen
     (2048, 1, 2, 100, False),  # sixteen
     (1025, 3, 1, 30, False),   # more planes than registers hold: signs through L2
-    (300, 8, 2, 30, True),     # |J| above seven
+    (300, 8, 2, 30, True),     # four planes
+    (64, 127, 3, 40, True),    # seven, one CTA
+    (256, 31, 5, 40, False),
+    (511, 64, 2, 40, True),    # seven, a cluster of four
+    (1024, 15, 2, 40, False),  # four, eight CTAs
+    (1000, 16, 1, 20, True),   # five planes of this size: signs through L2
+    (300, 128, 2, 30, False),  # |J| above 127
     (2049, 1, 1, 20, False),
 ])
 def test_sign_solve_equals_per_step(n, jmax, R, steps, fields, monkeypatch):
@@ -55,7 +61,7 @@ def test_sign_solve_equals_per_step(n, jmax, R, steps, fields, monkeypatch):
     a = _solve(prob, n, R, steps, 11, True, monkeypatch)
     b = _solve(prob, n, R, steps, 11, False, monkeypatch)
     assert b.steps_per_launch == 1
-    if n <= 1024 and jmax <= 7 or n <= 2048 and jmax == 1:
+    if n <= 512 and jmax <= 127 or n <= 1024 and jmax <= 15 or n <= 2048 and jmax == 1:
         assert a.steps_per_launch == steps and a.kernel_launches == 3
     np.testing.assert_array_equal(a.final_x, b.final_x)
     np.testing.assert_array_equal(a.final_y, b.final_y)
@@ -98,7 +104,9 @@ def test_a_cached_plan_takes_other_couplings(monkeypatch):
     (513, 3, 130, False),    # 68e6
     (640, 7, 243, True),     # FP8 on the tensor cores: 300e6
     (640, 7, 245, False),
-    (200, 9, 40, False),     # more planes than the kernel has
+    (88, 16, 599, True),
+    (200, 100, 40, True),    # BF16 on the tensor cores
+    (200, 200, 40, False),   # more planes than the kernel has
 ])
 def test_automatic_mode_takes_the_faster_form(n, jmax, R, planes):
     J = instances.erdos_renyi(n, 0.7, seed=n + R, jmax=jmax, allow_zero=True)
