@@ -221,7 +221,7 @@ struct TcEngine {
   CUtensorMap tmE;    // V operand buffer 0, part 0, whole replica tiles (the energy contraction)
   float jscale = 1.0f, jinv = 1.0f;  // FP16 hi + lo: the coupling scale (a power of two) and its inverse
   int flag_stride = 1;  // words between consecutive units' step flags
-  // E2M1 solves without a trace run in the multi-step kernel with tagged sign words (sb_run.cuh)
+  // E2M1 and FP8 solves without a trace run in the multi-step kernel with tagged sign words (sb_run.cuh)
   int run_nr = 0, run_grid = 0;  // its replica tile (0: not used) and CTAs
   GInst *d_inst = nullptr;       // the one instance
   GInst h_inst;                  // what d_inst holds
@@ -379,14 +379,20 @@ const char *bind(TcEngine *e, cudaError_t *ce) {
 }  // namespace
 
 namespace {
+// 128-byte chunks of an operand row of n spins in the multi-step kernel.
+int run_chunks(int dt, int n) { return kp_for(dt, n) / (dt == kTcFp4 ? 256 : 128); }
+
 // Replica tile of the multi-step kernel for n spins x R replicas, and how its items share CTAs (per_cta
 // items of one spin tile each, its J rows resident): the smallest tile whose items have an SM each, since a
 // step is bound by its dependent chain and a smaller tile shortens every part of it; else two 64-replica
 // items per CTA. Measured, us per step: (N, R) = (300, 1000) 1.85 with 32-replica items, 2.45 with 64;
 // (1111, 300) 2.34 / 3.16; (2000, 256) 2.64 / 3.55; (2000, 512) 3.42 with 64; (2000, 1024) 4.16 with two of
-// 64. The kernel that exchanges operands (sb_tc_fp4.cuh) took 4.43, 6.49, 6.28, 6.27 and 6.20.
-bool run_shape(int n, int R, int sms, int *nr, int *per_cta) {
-  if (kp_for(kTcFp4, n) / 256 > kResChunks) return false;
+// 64. The kernel that exchanges operands (sb_tc_fp4.cuh) took 4.43, 6.49, 6.28, 6.27 and 6.20. FP8 operands, J resident
+// up to nine chunks (1152 spins) and streamed beyond, against the kernel that exchanges them (sb_tc_kernel.cuh):
+// (300, 1000) 2.30 / 8.15, (1152, 300) 3.05 / 9.62, (1153, 300) 3.48 / 10.2, (2000, 1024) 7.8 / 12.1, (4096, 290) 13.5 /
+// 16.8. (E2M1 shapes beyond nine chunks take FP8.)
+bool run_shape(int dt, int n, int R, int sms, int *nr, int *per_cta) {
+  if (dt == kTcFp4 && run_chunks(dt, n) > kResChunks) return false;
   const int mt = (n + kBM - 1) / kBM, t32 = (R + 31) / 32, t64 = (R + 63) / 64;
   *per_cta = 1;
   if (mt * t32 <= sms) {
@@ -405,7 +411,7 @@ bool run_shape(int n, int R, int sms, int *nr, int *per_cta) {
 // Items, exchange words and instance slot of the multi-step kernel; buffers of the engine's own.
 sb_status run_create(TcEngine *e, cudaStream_t st, cudaError_t *ce) {
   int nr = 0, per = 0;
-  if (e->pair || e->s.variant != 2 || !run_shape(e->s.n, e->s.R, sm_count(), &nr, &per)) return SB_OK;
+  if (e->pair || e->s.variant != 2 || !run_shape(e->s.dtype, e->s.n, e->s.R, sm_count(), &nr, &per)) return SB_OK;
   const int mt = (e->s.n + kBM - 1) / kBM, rt = (e->s.R + nr - 1) / nr, cta_r = (rt + per - 1) / per;
   const size_t words = (size_t)2 * 4 * mt * nr;
   std::vector<RunItem> items;
@@ -415,7 +421,7 @@ sb_status run_create(TcEngine *e, cudaStream_t st, cudaError_t *ce) {
   for (int j = 0; j < per; ++j)
     for (int b = 0; b < grid; ++b) {
       const int r = per * (b / mt) + j;
-      if (r < rt) items.push_back(RunItem{0, (b % mt) * kBM, r * nr, e->Kp / 256, mt, (uint32_t)(r * words)});
+      if (r < rt) items.push_back(RunItem{0, (b % mt) * kBM, r * nr, run_chunks(e->s.dtype, e->s.n), mt, (uint32_t)(r * words)});
     }
   e->ll_words = words * rt;
   e->n_items = (int)items.size();
@@ -498,7 +504,8 @@ int64_t tc_footprint(const TcSetup &s) {
   const int64_t Rp = (s.R + 127) / 128 * 128;
   const int ap = tc_split(s.dtype) ? 2 : 1;
   const int bp = ((tc_split(s.dtype) && s.variant == 1) || s.variant == 3) ? 2 : 1;
-  return Np * Kp * elem * ap + 2 * Rp * Kp * elem * bp + 4096;
+  return Np * Kp * elem * ap + 2 * Rp * Kp * elem * bp + 4096 +
+         (s.dtype == kTcFp8 ? Np * Rp / 2 + 65536 : 0);  // the multi-step kernel's exchange words and items
 }
 
 sb_status tc_create(TcEngine **out, const TcSetup &s, const float *dJ, int jp, std::string &err,
@@ -548,7 +555,7 @@ sb_status tc_create(TcEngine **out, const TcSetup &s, const float *dJ, int jp, s
   if ((ce = tc_reload(e, dJ, jp, st)) != cudaSuccess) return fail("convert_j_kernel", ce);
   const char *what = bind(e, &ce);
   if (what) return fail(what, ce);
-  if (s.dtype == kTcFp4 && run_create(e, st, &ce) != SB_OK) return fail("multi-step kernel tables", ce);
+  if ((s.dtype == kTcFp4 || s.dtype == kTcFp8) && run_create(e, st, &ce) != SB_OK) return fail("multi-step kernel tables", ce);
   *out = e;
   return SB_OK;
 }
@@ -637,7 +644,7 @@ static cudaError_t launch(TcEngine *e, int emode, const TcArgs &a, cudaStream_t 
   return cudaLaunchKernelExC(&cfg, e->kernel[emode], params);
 }
 
-// All steps of an E2M1 solve in the multi-step kernel, then V(steps) for the energy pass.
+// All steps of an E2M1 or FP8 solve in the multi-step kernel, then V(steps) for the energy pass.
 static cudaError_t run_multi(TcEngine *e, const TcArgs &a, cudaStream_t st) {
   GInst in;
   memset(&in, 0, sizeof(in));
@@ -654,7 +661,7 @@ static cudaError_t run_multi(TcEngine *e, const TcArgs &a, cudaStream_t st) {
   in.c0 = a.c0;
   in.dt = a.dt;
   in.dta0 = a.dta0;
-  in.kbytes = e->Kp / 2;
+  in.kbytes = e->s.dtype == kTcFp4 ? e->Kp / 2 : e->Kp;
   cudaError_t ce;
   if (memcmp(&in, &e->h_inst, sizeof(in)) != 0) {
     if ((ce = cudaMemcpyAsync(e->d_inst, &in, sizeof(in), cudaMemcpyHostToDevice, st)) != cudaSuccess ||
@@ -675,7 +682,13 @@ static cudaError_t run_multi(TcEngine *e, const TcArgs &a, cudaStream_t st) {
   r.skip_item = a.skip_unit;
   r.skip_step = a.skip_step;
   r.wait_cycles = a.wait_cycles;
-  if ((ce = launch_run(e->run_nr, kGopE2m1, true, r, e->run_grid, st)) != cudaSuccess) return ce;
+  const bool fp4 = e->s.dtype == kTcFp4, res = run_chunks(e->s.dtype, e->s.n) <= kResChunks;
+  if ((ce = launch_run(e->run_nr, fp4 ? kGopE2m1 : kGopFp8, res, r, e->run_grid, st)) != cudaSuccess) return ce;
+  if (!fp4) {
+    prepare_v_kernel<<<grid_1d((size_t)e->s.n * e->s.R), 256, 0, st>>>(a.x, e->s.n, e->s.R, e->s.xp, e->v[a.steps & 1][0],
+                                                                        nullptr, e->Kp, e->s.dtype, e->s.variant, 1.0f);
+    return cudaGetLastError();
+  }
   const int Kb = e->Kp / 2;
   prepare_v_fp4_kernel<<<grid_1d((size_t)e->s.R * Kb), 256, 0, st>>>(a.x, e->s.n, e->s.R, e->s.xp,
                                                                      e->v[a.steps & 1][0], Kb);

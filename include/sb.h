@@ -89,7 +89,8 @@ typedef enum sb_variant { SB_ASB = 0, SB_BSB = 1, SB_DSB = 2 } sb_variant;
  *  SB_FIELD_TC:   tcgen05 tensor cores. dSB with integer |J| <= 4 and n <= ~2300: packed E2M1
  *                 operands, FP32 accumulation (bit-exact); without a trace every step in one launch.
  *                 dSB with integer |J| <= 16: FP8 E4M3 operands (grouped batches and serving:
- *                 packed E2M3, J / 4 in six bits), FP32 accumulation (bit-exact).
+ *                 packed E2M3, J / 4 in six bits), FP32 accumulation (bit-exact), without a trace
+ *                 every step in one launch likewise.
  *                 dSB with integer |J| <= 256: BF16 operands (bit-exact).
  *                 dSB with real J: BF16 hi+lo split of J. bSB: BF16 hi+lo split of J and of x
  *                 (three products), FP32 accumulation. aSB is not offered on tensor cores. */
