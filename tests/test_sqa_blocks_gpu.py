@@ -71,3 +71,9 @@ def _check(ctx, J, M, R, steps, mode):
     np.testing.assert_array_equal(res.energy_trace, tr.astype(np.float64))
     np.testing.assert_array_equal(res.replica_energies, tr[:, -1].astype(np.float64))
     assert res.energy_check_ok
+
+
+@pytest.mark.parametrize("R", [31, 32, 33, 65, 100])
+def test_reference_states_of_many_replicas(ctx, R):
+    """Reference mode starts replicas in up to 32 rows, each jumping ahead in the xorshift sequence."""
+    _check(ctx, _couplings(150, "pm1"), 5, R, 2, sb.SQA_RNG_REFERENCE)
