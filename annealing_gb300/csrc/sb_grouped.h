@@ -14,7 +14,8 @@ namespace sbk {
 
 // Operand types of the grouped kernel: FP8 E4M3 (integer |J| <= 16), packed E2M1 (|J| <= 4), or
 // packed E2M3, six bits per value (|J| <= 16 held as J / 4 against signs of +-4, exact products).
-enum GOperand : int { kGopFp8 = 0, kGopE2m1 = 1, kGopE2m3 = 2 };
+// kGopFp8x2 (the multi-step kernel alone): J = 16 hi + lo as two E4M3 chunks per 128 spins, one after the other
+enum GOperand : int { kGopFp8 = 0, kGopE2m1 = 1, kGopE2m3 = 2, kGopFp8x2 = 3 };
 
 // Per-instance descriptor read by the grouped kernel (device memory, 64-byte aligned for the
 // tensor maps).

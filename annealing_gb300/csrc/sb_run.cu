@@ -13,8 +13,9 @@ template <int NR, bool RES>
 cudaError_t launch_as(int op, const RunArgs &a, int grid, cudaStream_t st) {
   const void *k = op == kGopE2m1   ? reinterpret_cast<const void *>(&run_kernel<NR, kGopE2m1, RES>)
                   : op == kGopE2m3 ? reinterpret_cast<const void *>(&run_kernel<NR, kGopE2m3, RES>)
+                  : op == kGopFp8x2 ? reinterpret_cast<const void *>(&run_kernel<NR, kGopFp8x2, RES>)
                                    : reinterpret_cast<const void *>(&run_kernel<NR, kGopFp8, RES>);
-  const size_t smem = RunCfg<NR, RES>::kSmem;
+  const size_t smem = op == kGopFp8x2 ? RunCfg<NR, RES, 1>::kSmem : RunCfg<NR, RES>::kSmem;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   void *args[] = {const_cast<RunArgs *>(&a)};

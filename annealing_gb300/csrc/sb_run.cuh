@@ -18,6 +18,8 @@
 //   RES: J rows resident in shared memory, loaded once (all items of a CTA share them): the items of one
 //        instance whose J rows fit, e.g. two 64-replica halves of a spin tile.
 //   else J tiles stream through the ring from L2 each step.
+// Couplings beyond E4M3's 16 (integers up to 256) come as 16 hi + lo, both exact in E4M3: a chunk of each multiplies the
+// same 128 signs, so the signs are expanded once and the sums are the integers all the same.
 // Word order: bit position 4 i + k of a word holds spin 8 k + i for E2M1 operands (nibble i of the k-th
 // 32-bit word of the granule is then (w << (3 - k)) & 0x88888888 | 0x22222222), bit 8 j + k holds spin 4 k + j
 // for the byte operands; the writer's lanes take their spins' bits in that order before they transpose.
@@ -58,19 +60,20 @@ constexpr int kLoadWarps = 4;
 constexpr int kRunThreads = kTcThreads + 32 * kLoadWarps;
 constexpr int kResChunks = 9;   // J chunks (16 KB each) of a resident item: leaves four 16 KB V stages at 64 replicas
 
-template <int NR, bool RES>
+// VS: V chunks of a ring stage (one for J in two parts: both multiply the same signs)
+template <int NR, bool RES, int VS = 2>
 struct RunCfg {
   static_assert(NR == 32 || NR == 64, "replica tile");
   static constexpr int kAcc = 2, kSlots = NR == 32 ? 6 : 2;
   // TMEM columns: accumulators, 32 block-scale columns, then x and y of each slot
   static constexpr uint32_t kSf = kAcc * NR, kState = kSf + 32;
   static_assert(kState + 2 * NR * kSlots <= 512, "TMEM columns");
-  // A ring stage holds kSub chunks: J tiles (streaming), then V tiles. Waiting for a stage costs the MMA
+  // A ring stage holds kSub J chunks (streaming), then VS V chunks. Waiting for a stage costs the MMA
   // warp ~110 clocks: 89 clocks per MMA with one chunk (4 MMAs) per stage, 63 with two, 48 without waits.
   static constexpr int kSub = 2;
   static constexpr int kATile = kBM * kChunkBytes, kBTile = NR * kChunkBytes;
   static constexpr int kVOff = RES ? 0 : kSub * kATile;  // V tiles within a stage
-  static constexpr int kStage = kVOff + kSub * kBTile;
+  static constexpr int kStage = kVOff + VS * kBTile;
   static constexpr int kRing = 212 * 1024 - (RES ? kResChunks * kATile : 0);
   static constexpr int kStages = kRing / kStage > 8 ? 8 : kRing / kStage;
   static constexpr size_t kSmem = (size_t)kStages * kStage + (RES ? kResChunks * kATile : 0) + 1024;
@@ -130,7 +133,9 @@ __device__ __forceinline__ uint32_t transpose32(uint32_t w, int lane) {
 
 template <int NR, int OP, bool RES>
 __global__ void __launch_bounds__(kRunThreads, 1) run_kernel(const __grid_constant__ RunArgs p) {
-  using C = RunCfg<NR, RES>;
+  constexpr bool X2 = OP == kGopFp8x2;
+  constexpr int kVSub = X2 ? 1 : 2;  // V chunks of a stage
+  using C = RunCfg<NR, RES, kVSub>;
   constexpr int STAGES = C::kStages, kAcc = C::kAcc, kSlots = C::kSlots;
   constexpr int kATile = C::kATile, kBTile = C::kBTile, kStage = C::kStage, kSub = C::kSub;
   constexpr bool FP4 = OP == kGopE2m1, FP6 = OP == kGopE2m3;
@@ -167,7 +172,7 @@ __global__ void __launch_bounds__(kRunThreads, 1) run_kernel(const __grid_consta
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
       ptx::mbar_init(&fullj_bar[s], 1);
-      ptx::mbar_init(&fullv_bar[s], kSub);
+      ptx::mbar_init(&fullv_bar[s], kVSub);
       ptx::mbar_init(&empty_bar[s], 1);
     }
     for (int b = 0; b < kAcc; ++b) {
@@ -289,7 +294,7 @@ __global__ void __launch_bounds__(kRunThreads, 1) run_kernel(const __grid_consta
               if (c > 0 && kc + c >= kchunks) continue;
 #pragma unroll
               for (int k = 0; k < kChunkBytes / 32; ++k) {
-                const uint64_t ad = ad0 + ao + c * (kATile / 16) + 2 * k, bd = bd0 + bo + c * (kBTile / 16) + 2 * k;
+                const uint64_t ad = ad0 + ao + c * (kATile / 16) + 2 * k, bd = bd0 + bo + (X2 ? 0 : c * (kBTile / 16)) + 2 * k;
                 const uint32_t add = (kc > 0 || c > 0 || k > 0) ? 1u : 0u;
                 if constexpr (FP4)
                   ptx::mma_mxf4(t_acc, ad, bd, kIdesc, tmem + kSf, tmem + kSf + 16, add);
@@ -312,11 +317,13 @@ __global__ void __launch_bounds__(kRunThreads, 1) run_kernel(const __grid_consta
     }
   } else if (warp >= 2 + kEpiWarps) {
     // ---------------- loaders: tagged words -> operand bytes in shared memory ----------------
-    // Warp lw takes chunk lw % 2 of every second stage whole, so that the four warps' polls, waits and fences
+    // Warp lw takes chunk lw % kVSub of every kTurn-th stage whole, so that the four warps' polls, waits and fences
     // overlap (all four on one chunk took 0.5 us per chunk). Load i of lane l: word i and replicas 2 l, 2 l + 1
     // of the chunk (NR = 64), or word 2 i + l / 16 and replicas 2 (l % 16) + {0, 1} (NR = 32).
     const uint32_t lw = (uint32_t)(warp - (2 + kEpiWarps));
-    const uint32_t ring = ptx::smem_u32(smem) + C::kVOff + (lw & 1) * kBTile;
+    constexpr int kTurn = kLoadWarps / kVSub;
+    const int sub = (int)(lw % kVSub);
+    const uint32_t ring = ptx::smem_u32(smem) + C::kVOff + sub * kBTile;
     const int wl = NR == 64 ? 0 : lane >> 4, pr = NR == 64 ? lane : lane & 15;
     // of eight lanes the first four write their even row first, the others their odd row: the eight swizzled
     // granules then fall in eight different bank groups
@@ -333,23 +340,23 @@ __global__ void __launch_bounds__(kRunThreads, 1) run_kernel(const __grid_consta
         auto load = [&](int st, int i, ulonglong2 &d) {
           // a chunk past the last (an odd count's second half) has its words past `words`: nothing is read or
           // waited for, and the MMAs leave it out
-          const int wd = (st * kSub + (int)(lw & 1)) * kWords + i * kWordsPerLoad;
+          const int wd = (st * kVSub + sub) * kWords + i * kWordsPerLoad;
           if (wd + wl < words)
             d = ld_relaxed64x2(src + (size_t)wd * NR);
           else
             d.x = d.y = (unsigned long long)want << 32;
         };
         auto fresh = [&](const ulonglong2 &d) { return (uint32_t)(d.x >> 32) == want && (uint32_t)(d.y >> 32) == want; };
-        int st = (int)(((lw >> 1) - g0) & 1u);
+        int st = (int)((lw / kVSub - g0) & (uint32_t)(kTurn - 1));
         if (st < nst)
 #pragma unroll
           for (int i = 0; i < kLoads; ++i) load(st, i, nx[i]);
-        for (; st < nst; st += 2) {
+        for (; st < nst; st += kTurn) {
 #pragma unroll
           for (int i = 0; i < kLoads; ++i) v[i] = nx[i];
-          if (st + 2 < nst)
+          if (st + kTurn < nst)
 #pragma unroll
-            for (int i = 0; i < kLoads; ++i) load(st + 2, i, nx[i]);
+            for (int i = 0; i < kLoads; ++i) load(st + kTurn, i, nx[i]);
           bool all = true;
 #pragma unroll
           for (int i = 0; i < kLoads; ++i) all = all && fresh(v[i]);

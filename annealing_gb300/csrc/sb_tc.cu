@@ -86,6 +86,21 @@ __global__ void convert_j_kernel(const float *J, int n, int jp, uint8_t *a0, uin
   }
 }
 
+// Integers |J| <= 256 as 16 hi + lo, |hi| <= 15 and |lo| <= 16, both exact in E4M3: per 128 spins a chunk of 16 hi, then
+// one of lo.
+__global__ void convert_j_fp8x2_kernel(const float *J, int n, int jp, uint8_t *a, int Np, int Kp) {
+  const size_t total = (size_t)Np * Kp;
+  for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < total;
+       k += (size_t)gridDim.x * blockDim.x) {
+    const size_t i = k / Kp, j = k % Kp;
+    const float v = (i < (size_t)n && j < (size_t)n) ? J[i * jp + j] : 0.0f;
+    const float hi = 16.0f * fminf(15.0f, fmaxf(-15.0f, rintf(v * 0.0625f)));
+    uint8_t *d = a + i * 2 * Kp + (j / 128) * 256 + j % 128;
+    d[0] = (uint8_t)__nv_cvt_float_to_fp8(hi, __NV_SATFINITE, __NV_E4M3);
+    d[128] = (uint8_t)__nv_cvt_float_to_fp8(v - hi, __NV_SATFINITE, __NV_E4M3);
+  }
+}
+
 __global__ void prepare_v_kernel(const float *x, int n, int R, int xp, uint8_t *v0, uint8_t *v1,
                                  int Kp, int dt, int variant, float xscale) {
   const size_t total = (size_t)n * R;
@@ -221,7 +236,9 @@ struct TcEngine {
   CUtensorMap tmE;    // V operand buffer 0, part 0, whole replica tiles (the energy contraction)
   float jscale = 1.0f, jinv = 1.0f;  // FP16 hi + lo: the coupling scale (a power of two) and its inverse
   int flag_stride = 1;  // words between consecutive units' step flags
-  // E2M1 and FP8 solves without a trace run in the multi-step kernel with tagged sign words (sb_run.cuh)
+  // E2M1, FP8 and BF16 dSB solves without a trace run in the multi-step kernel with tagged sign words (sb_run.cuh);
+  // BF16 couplings as 16 hi + lo in E4M3, in a[1] with the map tm_run
+  CUtensorMap tm_run;
   int run_nr = 0, run_grid = 0;  // its replica tile (0: not used) and CTAs
   GInst *d_inst = nullptr;       // the one instance
   GInst h_inst;                  // what d_inst holds
@@ -380,7 +397,7 @@ const char *bind(TcEngine *e, cudaError_t *ce) {
 
 namespace {
 // 128-byte chunks of an operand row of n spins in the multi-step kernel.
-int run_chunks(int dt, int n) { return kp_for(dt, n) / (dt == kTcFp4 ? 256 : 128); }
+int run_chunks(int dt, int n) { return kp_for(dt, n) / (dt == kTcFp4 ? 256 : 128) * (dt == kTcBf16 ? 2 : 1); }
 
 // Replica tile of the multi-step kernel for n spins x R replicas, and how its items share CTAs (per_cta
 // items of one spin tile each, its J rows resident): the smallest tile whose items have an SM each, since a
@@ -390,7 +407,9 @@ int run_chunks(int dt, int n) { return kp_for(dt, n) / (dt == kTcFp4 ? 256 : 128
 // 64. The kernel that exchanges operands (sb_tc_fp4.cuh) took 4.43, 6.49, 6.28, 6.27 and 6.20. FP8 operands, J resident
 // up to nine chunks (1152 spins) and streamed beyond, against the kernel that exchanges them (sb_tc_kernel.cuh):
 // (300, 1000) 2.30 / 8.15, (1152, 300) 3.05 / 9.62, (1153, 300) 3.48 / 10.2, (2000, 1024) 7.8 / 12.1, (4096, 290) 13.5 /
-// 16.8. (E2M1 shapes beyond nine chunks take FP8.)
+// 16.8. (E2M1 shapes beyond nine chunks take FP8.) BF16 couplings as 16 hi + lo in E4M3, resident up to 512 spins,
+// against the kernel on BF16 operands: (88, 599) 1.71 / 7.90, (300, 1000) 2.53 / 9.39, (1000, 300) 4.07 / 11.7,
+// (2000, 1024) 12.6 / 17.1, (4096, 290) 23.7 / 26.4, (8192, 64) 29.3 / 41.5, (16384, 32) 79.5 / 91.6.
 bool run_shape(int dt, int n, int R, int sms, int *nr, int *per_cta) {
   if (dt == kTcFp4 && run_chunks(dt, n) > kResChunks) return false;
   const int mt = (n + kBM - 1) / kBM, t32 = (R + 31) / 32, t64 = (R + 63) / 64;
@@ -424,6 +443,10 @@ sb_status run_create(TcEngine *e, cudaStream_t st, cudaError_t *ce) {
       if (r < rt) items.push_back(RunItem{0, (b % mt) * kBM, r * nr, run_chunks(e->s.dtype, e->s.n), mt, (uint32_t)(r * words)});
     }
   e->ll_words = words * rt;
+  if (e->s.dtype == kTcBf16) {
+    *ce = cudaMalloc(&e->a[1], (size_t)e->Np * 2 * e->Kp);
+    if (*ce != cudaSuccess || !encode_2d(&e->tm_run, e->a[1], 1, 2 * (uint64_t)e->Kp, (uint64_t)e->Np, kBM)) return SB_ERR_CUDA;
+  }
   e->n_items = (int)items.size();
   if ((*ce = cudaMalloc(&e->d_inst, sizeof(GInst))) != cudaSuccess ||
       (*ce = cudaMalloc(&e->d_items, items.size() * sizeof(RunItem))) != cudaSuccess ||
@@ -505,7 +528,8 @@ int64_t tc_footprint(const TcSetup &s) {
   const int ap = tc_split(s.dtype) ? 2 : 1;
   const int bp = ((tc_split(s.dtype) && s.variant == 1) || s.variant == 3) ? 2 : 1;
   return Np * Kp * elem * ap + 2 * Rp * Kp * elem * bp + 4096 +
-         (s.dtype == kTcFp8 ? Np * Rp / 2 + 65536 : 0);  // the multi-step kernel's exchange words and items
+         // the multi-step kernel's exchange words and items, and its form of BF16 couplings
+         (s.variant == 2 && !tc_split(s.dtype) ? Np * Rp / 2 + 65536 + (s.dtype == kTcBf16 ? 2 * Np * Kp : 0) : 0);
 }
 
 sb_status tc_create(TcEngine **out, const TcSetup &s, const float *dJ, int jp, std::string &err,
@@ -552,10 +576,11 @@ sb_status tc_create(TcEngine **out, const TcSetup &s, const float *dJ, int jp, s
       if ((ce = cudaMemsetAsync(e->v[b][pp], 0, vbytes, st)) != cudaSuccess) return fail("memset", ce);
     }
   if ((ce = cudaMalloc(&e->flags, flag_bytes(e))) != cudaSuccess) return fail("cudaMalloc(flags)", ce);
+  ce = cudaSuccess;
+  if (!tc_split(s.dtype) && run_create(e, st, &ce) != SB_OK) return fail("multi-step kernel tables", ce);
   if ((ce = tc_reload(e, dJ, jp, st)) != cudaSuccess) return fail("convert_j_kernel", ce);
   const char *what = bind(e, &ce);
   if (what) return fail(what, ce);
-  if ((s.dtype == kTcFp4 || s.dtype == kTcFp8) && run_create(e, st, &ce) != SB_OK) return fail("multi-step kernel tables", ce);
   *out = e;
   return SB_OK;
 }
@@ -597,6 +622,8 @@ cudaError_t tc_reload(TcEngine *e, const float *dJ, int jp, cudaStream_t st) {
     convert_j_fp4_kernel<<<grid_1d((size_t)e->Np * Kb), 256, 0, st>>>(dJ, e->s.n, jp, e->a[0], e->Np, Kb);
     return cudaGetLastError();
   }
+  if (e->s.dtype == kTcBf16 && e->run_nr > 0)
+    convert_j_fp8x2_kernel<<<grid_1d((size_t)e->Np * e->Kp), 256, 0, st>>>(dJ, e->s.n, jp, e->a[1], e->Np, e->Kp);
   convert_j_kernel<<<grid_1d((size_t)e->Np * e->Kp), 256, 0, st>>>(dJ, e->s.n, jp, e->a[0], e->a[1], e->Np, e->Kp,
                                                                    e->s.dtype, e->jscale);
   return cudaGetLastError();
@@ -644,11 +671,12 @@ static cudaError_t launch(TcEngine *e, int emode, const TcArgs &a, cudaStream_t 
   return cudaLaunchKernelExC(&cfg, e->kernel[emode], params);
 }
 
-// All steps of an E2M1 or FP8 solve in the multi-step kernel, then V(steps) for the energy pass.
+// All steps of an E2M1, FP8 or BF16 solve in the multi-step kernel, then V(steps) for the energy pass.
 static cudaError_t run_multi(TcEngine *e, const TcArgs &a, cudaStream_t st) {
   GInst in;
   memset(&in, 0, sizeof(in));
-  in.tmA = e->args.tmA[0];
+  const bool bf16 = e->s.dtype == kTcBf16;
+  in.tmA = bf16 ? e->tm_run : e->args.tmA[0];
   in.x = a.x;
   in.y = a.y;
   in.h = a.h;
@@ -661,7 +689,7 @@ static cudaError_t run_multi(TcEngine *e, const TcArgs &a, cudaStream_t st) {
   in.c0 = a.c0;
   in.dt = a.dt;
   in.dta0 = a.dta0;
-  in.kbytes = e->s.dtype == kTcFp4 ? e->Kp / 2 : e->Kp;
+  in.kbytes = e->s.dtype == kTcFp4 ? e->Kp / 2 : bf16 ? 2 * e->Kp : e->Kp;
   cudaError_t ce;
   if (memcmp(&in, &e->h_inst, sizeof(in)) != 0) {
     if ((ce = cudaMemcpyAsync(e->d_inst, &in, sizeof(in), cudaMemcpyHostToDevice, st)) != cudaSuccess ||
@@ -683,7 +711,7 @@ static cudaError_t run_multi(TcEngine *e, const TcArgs &a, cudaStream_t st) {
   r.skip_step = a.skip_step;
   r.wait_cycles = a.wait_cycles;
   const bool fp4 = e->s.dtype == kTcFp4, res = run_chunks(e->s.dtype, e->s.n) <= kResChunks;
-  if ((ce = launch_run(e->run_nr, fp4 ? kGopE2m1 : kGopFp8, res, r, e->run_grid, st)) != cudaSuccess) return ce;
+  if ((ce = launch_run(e->run_nr, fp4 ? kGopE2m1 : bf16 ? kGopFp8x2 : kGopFp8, res, r, e->run_grid, st)) != cudaSuccess) return ce;
   if (!fp4) {
     prepare_v_kernel<<<grid_1d((size_t)e->s.n * e->s.R), 256, 0, st>>>(a.x, e->s.n, e->s.R, e->s.xp, e->v[a.steps & 1][0],
                                                                         nullptr, e->Kp, e->s.dtype, e->s.variant, 1.0f);

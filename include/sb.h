@@ -91,7 +91,8 @@ typedef enum sb_variant { SB_ASB = 0, SB_BSB = 1, SB_DSB = 2 } sb_variant;
  *                 dSB with integer |J| <= 16: FP8 E4M3 operands (grouped batches and serving:
  *                 packed E2M3, J / 4 in six bits), FP32 accumulation (bit-exact), without a trace
  *                 every step in one launch likewise.
- *                 dSB with integer |J| <= 256: BF16 operands (bit-exact).
+ *                 dSB with integer |J| <= 256: BF16 operands (bit-exact); without a trace as 16 hi + lo
+ *                 in FP8 E4M3, every step in one launch (bit-exact too).
  *                 dSB with real J: BF16 hi+lo split of J. bSB: BF16 hi+lo split of J and of x
  *                 (three products), FP32 accumulation. aSB is not offered on tensor cores. */
 typedef enum sb_field_mode { SB_FIELD_AUTO = 0, SB_FIELD_FP32 = 1, SB_FIELD_TC = 2 } sb_field_mode;
