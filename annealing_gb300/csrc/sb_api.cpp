@@ -115,14 +115,17 @@ sb_status check_params(const sb_problem *p, const sb_params *prm, std::string &e
 
 // The automatic mode's dSB solves of 32 replicas or more that the bit planes (sb_signs.cuh) run faster than the
 // tensor cores. A step of them costs n / 32 words of logic per row, plane and replica, so up to some n^2 R P it stays
-// at its latency of 0.3 to 1 us; a tensor-core step's chain takes 1.6 to 2.3 (E2M1 operands, |J| <= 4), 3 to 9 (FP8).
+// at its latency of 0.3 to 1 us; a tensor-core step's chain takes 1.5 to 2.6 (E2M1, E4M3), to 3.4 (16 hi + lo), n <= 1024.
 // us per step, planes / tensor cores, +-1 unless noted:
 //   one CTA holds the solve, limit 134e6: n = 128 R = 1000 0.37 / 1.72, n = 256 R = 1000 0.90 / 1.72, n = 512 R = 300
 //   0.74 / 2.05, R = 512 (134e6) 1.36 / 1.84, R = 1000 2.23 / 1.85; |J| <= 3 n = 256 R = 1000 1.41 / 1.71;
 //   a cluster, 64e6: n = 700 R = 100 0.99 / 2.33, n = 1000 R = 64 0.88 / 2.21, n = 513 R = 300 (79e6) 2.10 / 2.22,
 //   R = 512 3.05 / 2.22; |J| <= 3 n = 513 R = 100 1.57 / 2.25, R = 200 (105e6) 2.56 / 2.30;
-//   |J| of 5 to 127, 300e6: n = 88 R = 599 |J| <= 16 0.45 / 7.2, n = 256 R = 600 |J| <= 127 (275e6) 2.03 / 8.01,
-//   n = 512 R = 100 1.71 / 8.51; |J| <= 7 n = 256 R = 1000 1.73 / 7.14, n = 700 R = 200 4.22 / 8.68, n = 513 R = 512 (404e6) 8.11 / 8.44.
+//   |J| of 5 to 127, 205e6 with n rounded up to a power of two, as the planes' time goes (n = 300 takes that of 512):
+//   |J| <= 7 n = 256 R = 1000 (197e6) 1.72 / 1.71, n = 400 R = 250 (197e6) 1.73 / 1.93, n = 512 R = 300 (236e6) 2.17 /
+//   2.05, n = 1000 R = 64 (201e6) 2.07 / 2.62; |J| <= 16 n = 512 R = 100 (131e6) 1.21 / 2.10, n = 160 R = 1000 (328e6)
+//   1.90 / 1.70, n = 300 R = 300 (393e6) 2.54 / 2.04; |J| <= 100 n = 88 R = 599 (69e6) 0.56 / 1.59, n = 512 R = 100
+//   (184e6) 1.64 / 2.48, n = 300 R = 300 (551e6) 3.52 / 2.23.
 bool signs_beat_tc(const sb_problem *p, const sb_params *prm) {
   if (prm->variant != SB_DSB || prm->trace || prm->trace_all || prm->steps <= 0 || !p->integer_valued ||
       prm->operand_dtype != SB_OPERAND_AUTO)
@@ -133,8 +136,12 @@ bool signs_beat_tc(const sb_problem *p, const sb_params *prm) {
   // (what the tensor-core kernel has no room for, a unit of 128 x 128 to an SM, is not taken here either)
   if ((int64_t)((n + 127) / 128) * ((R + 127) / 128) > 128) return false;
   const bool one_cta = n <= (P == 1 ? sbk::kSignsOneCta : sbk::kSignsOneCta / 2);
-  const double limit = p->max_abs_j > 4 ? 300e6 : one_cta ? 134.5e6 : 64e6;
-  return (double)n * n * R * P <= limit && sbk::sign_planes(n, R, p->max_abs_j) > 0;
+  const double limit = p->max_abs_j > 4 ? 205e6 : one_cta ? 134.5e6 : 64e6;
+  int nt = n;  // the extent that the planes' time goes by
+  if (p->max_abs_j > 4)
+    for (nt = 1; nt < n; nt *= 2) {
+    }
+  return (double)nt * nt * R * P <= limit && sbk::sign_planes(n, R, p->max_abs_j) > 0;
 }
 
 // Field mode and operand dtype for (problem, params).

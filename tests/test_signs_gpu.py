@@ -102,8 +102,8 @@ def test_a_cached_plan_takes_other_couplings(monkeypatch):
     (512, 1, 514, False),
     (513, 3, 100, True),     # 53e6, a cluster of five
     (513, 3, 130, False),    # 68e6
-    (640, 7, 243, True),     # FP8 on the tensor cores: 300e6
-    (640, 7, 245, False),
+    (640, 7, 65, True),      # FP8 on the tensor cores: 205e6, 640 counting as 1024
+    (640, 7, 66, False),
     (88, 16, 599, True),
     (200, 100, 40, True),    # BF16 on the tensor cores
     (200, 200, 40, False),   # more planes than the kernel has
