@@ -334,8 +334,7 @@ namespace {
 // (replica, slice, spin). One thread per spin, one ballot per 32 spins.
 // A block row makes ceil(R / rows) consecutive replicas. The xorshift step is linear over GF(2), so in reference mode
 // row c starts from its spins' state after the rows before it by c products with `jump`, the step to the power of a
-// row's calls (one row of all calls: a solve 0.6 ms longer at N = 150 and at
-// N = 4096 alike, M = 64, R = 304).
+// row's calls (one row of all calls: a solve 0.6 ms longer at N = 150 and at N = 4096 alike, M = 64, R = 304).
 struct XorshiftJump {
   uint32_t col[32];  // the images of the state's bits
 };
