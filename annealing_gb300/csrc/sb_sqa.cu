@@ -573,8 +573,8 @@ extern "C" sb_status sb_sqa_solve(sb_ctx *ctx, const sb_problem *prob, const sb_
   const size_t sp_words = (size_t)M * SPS;
   // |J| <= 4, M <= 64: the tensor-core kernel, whose fields fit 16 bits and whose rows of a block are distinct
   // (n >= 128). Faster wherever it runs, ms of 6 annealing steps against sqa_kernel: n = 150, M = R = 4 0.14 / 0.65;
-  // n = 500, M = 16, R = 64 0.41 / 2.06; n = 1000, M = 64, R = 304 1.5 / 8.7; n = 4096, M = 64, R = 4 6.3 / 26.5,
-  // R = 304 7.7 / 37.8; n = 2000, M = 64, R = 304, |J| <= 3 3.4 / 21.9; n = 6000, M = 64, R = 304 13.2 / 102.
+  // n = 500, M = 16, R = 64 0.41 / 2.06; n = 1000, M = 64, R = 304 1.4 / 8.7; n = 4096, M = 64, R = 4 5.6 / 26.5,
+  // R = 304 7.4 / 37.8; n = 2000, M = 64, R = 304, |J| <= 3 3.3 / 21.9; n = 6000, M = 64, R = 304 13.2 / 102.
   const int tc_sps = W + 1, tc_kp = (n + 255) / 256 * 256;  // W is a multiple of four: odd
   int sms = 1;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
