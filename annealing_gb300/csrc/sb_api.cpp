@@ -274,6 +274,9 @@ size_t energy_slots(const sb_params &p) { return needs_trace(p) ? (size_t)p.step
 sb_status upload_problem(sb_plan *pl, const sb_problem *p, std::string &err) {
   cudaStream_t st = pl->ctx->stream;
   const int n = pl->n;
+  // a cached plan takes any couplings of its shape: how energies are formed and checked follows this problem's
+  pl->integral = p->integer_valued != 0;
+  pl->split_exact = pl->integral && p->max_abs_j < 65536;
   // (a row copy from pageable memory takes twice the time of a plain one: N = 2000 158 us with its reset against 98)
   if (pl->jp == n) {
     SB_CUDA(cudaMemcpyAsync(pl->dJ, p->J, (size_t)n * n * sizeof(float), cudaMemcpyHostToDevice, st));
@@ -319,8 +322,6 @@ sb_status plan_create(sb_ctx *ctx, const sb_problem *p, const sb_params *prm, sb
   pl->xp = pl->jp;
   pl->mode = mode;
   pl->dtype = dtype;
-  pl->integral = p->integer_valued != 0;
-  pl->split_exact = pl->integral && p->max_abs_j < 65536;
   pl->c0 = prm->c0 > 0.0f ? prm->c0 : sb_default_c0(p);
   const float xi = prm->xi > 0.0f ? prm->xi : (float)(0.7 * (double)prm->detune / sqrt((double)p->n));
   pl->coeff = (float)((double)prm->coupling_dt * (double)xi);
