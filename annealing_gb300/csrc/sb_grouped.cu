@@ -635,6 +635,7 @@ sb_status Grouped::sync_tables(std::string &err) {
   cudaError_t e;
   if ((int)insts.size() > cap_insts) {
     cudaFree(d_insts);
+    d_insts = nullptr;
     cap_insts = std::max<int>((int)insts.size(), 2 * cap_insts);
     if ((e = cudaMalloc(&d_insts, (size_t)cap_insts * sizeof(GInst))) != cudaSuccess) {
       cap_insts = 0;
@@ -661,6 +662,7 @@ sb_status Grouped::sync_tables(std::string &err) {
   }
   if ((int)items.size() > cap_items) {
     cudaFree(d_items);
+    d_items = nullptr;
     cap_items = std::max<int>((int)items.size(), 2 * cap_items);
     if ((e = cudaMalloc(&d_items, (size_t)cap_items * sizeof(GItem))) != cudaSuccess) {
       cap_items = 0;
@@ -911,6 +913,7 @@ cudaError_t Grouped::energy_pass_for(const std::vector<int> &idx, int tick) {
   if (items.empty()) return cudaSuccess;
   if ((int)items.size() > cap_sub) {
     cudaFree(d_sub_items);
+    d_sub_items = nullptr;
     cap_sub = std::max<int>((int)items.size(), 2 * cap_sub);
     cudaError_t e = cudaMalloc(&d_sub_items, (size_t)cap_sub * sizeof(GItem));
     if (e != cudaSuccess) {

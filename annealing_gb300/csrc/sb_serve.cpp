@@ -103,6 +103,7 @@ struct Server {
   void run();
 
   void retire(int at_tick);
+  void fail_group(int nr, sb_status s, const std::string &err);
   void finish(Req *r, sb_status s, const std::string &err);
   void solve_alone(Req *r);
 };
@@ -224,39 +225,54 @@ void Server::attach_ready() {
   }
 }
 
-// Retires every resident request whose step budget ends at `at_tick`, and drops cancelled ones.
+// Gives the resident requests of one engine an error: retire takes them out with it, whatever steps they have left.
+void Server::fail_group(int nr, sb_status s, const std::string &err) {
+  for (Req *r : resident)
+    if (r->nr == nr && r->status == SB_OK) {
+      r->status = s;
+      r->err = err;
+    }
+}
+
+// Retires every resident request whose step budget ends at `at_tick` or that has failed, and drops cancelled ones.
 void Server::retire(int at_tick) {
   std::vector<Req *> fin, gone;
   for (Req *r : resident) {
     if (r->cancel) gone.push_back(r);
-    else if (r->ticks >= r->prm.steps) fin.push_back(r);
+    else if (r->status != SB_OK || r->ticks >= r->prm.steps) fin.push_back(r);
   }
   if (fin.empty() && gone.empty()) return;
   // energies of the finishing requests, per engine
   std::map<int, std::vector<int>> by_group;
-  for (Req *r : fin) by_group[r->nr].push_back(groups[r->nr]->find((int)r->ticket));
+  for (Req *r : fin)
+    if (r->status == SB_OK) by_group[r->nr].push_back(groups[r->nr]->find((int)r->ticket));
   for (auto &kv : by_group) {
     cudaError_t e = groups[kv.first]->energy_pass_for(kv.second, at_tick);
-    if (e != cudaSuccess)
+    if (e != cudaSuccess) {
+      cudaGetLastError();  // the next engine's launches look at it too
       for (Req *r : fin)
-        if (r->nr == kv.first) {
+        if (r->nr == kv.first && r->status == SB_OK) {
           r->status = SB_ERR_CUDA;
           r->err = std::string("energy pass: ") + cudaGetErrorString(e);
         }
+    }
   }
   uint32_t status = 0;
   for (auto &kv : groups)
     if (kv.second->d_status) cudaMemcpyAsync(&status, kv.second->d_status, 4, cudaMemcpyDeviceToHost, st);
-  for (Req *r : fin) {
+  std::vector<Req *> good;
+  for (Req *r : fin)
+    if (r->status == SB_OK) good.push_back(r);
+  for (Req *r : good) {
     sbk::Grouped *g = groups[r->nr];
     const sbk::GHost &gi = g->insts[g->find((int)r->ticket)];
     r->energies.resize(gi.R);
     cudaMemcpyAsync(r->energies.data(), gi.energy, (size_t)gi.R * sizeof(double), cudaMemcpyDeviceToHost, st);
   }
   cudaStreamSynchronize(st);
-  std::vector<std::vector<float>> xbs(fin.size());
-  for (size_t q = 0; q < fin.size(); ++q) {
-    Req *r = fin[q];
+  std::vector<std::vector<float>> xbs(good.size());
+  for (size_t q = 0; q < good.size(); ++q) {
+    Req *r = good[q];
     sbk::Grouped *g = groups[r->nr];
     const sbk::GHost &gi = g->insts[g->find((int)r->ticket)];
     int b = 0;
@@ -268,8 +284,8 @@ void Server::retire(int at_tick) {
     cudaMemcpyAsync(xbs[q].data(), gi.x + (size_t)b * gi.xp, (size_t)gi.n * sizeof(float), cudaMemcpyDeviceToHost, st);
   }
   cudaStreamSynchronize(st);
-  for (size_t q = 0; q < fin.size(); ++q) {
-    Req *r = fin[q];
+  for (size_t q = 0; q < good.size(); ++q) {
+    Req *r = good[q];
     r->spins.resize(xbs[q].size());
     for (size_t i = 0; i < xbs[q].size(); ++i) r->spins[i] = xbs[q][i] > 0.0f ? 1 : -1;
   }
@@ -311,24 +327,32 @@ void Server::run() {
     attach_ready();
     if (resident.empty()) continue;
     const auto t0 = Clock::now();
-    std::string err;
-    for (auto &kv : groups)
-      if (kv.second->sync_tables(err) != SB_OK) {
-        // fail everything resident in this engine
-        std::vector<Req *> bad;
-        for (Req *r : resident)
-          if (r->nr == kv.first) bad.push_back(r);
-        for (Req *r : bad) r->cancel = true;
+    // an engine whose tables or launches fail ends its requests with that error; it is not stepped with tables that
+    // may name instances it no longer has
+    std::map<int, bool> usable;
+    for (auto &kv : groups) {
+      std::string err;
+      const sb_status s = kv.second->sync_tables(err);
+      usable[kv.first] = s == SB_OK;
+      if (s != SB_OK) {
+        cudaGetLastError();
+        fail_group(kv.first, s, "instance tables: " + err);
       }
+    }
     // run ticks up to the next retirement (at most 64, to take in new arrivals: fewer than 0.5 ms of a
     // resident set that fits one wave, at ~5 us a tick)
     int nt = 64;
-    for (Req *r : resident) nt = std::min(nt, r->prm.steps - r->ticks);
+    for (Req *r : resident)
+      if (r->status == SB_OK) nt = std::min(nt, r->prm.steps - r->ticks);
     if (nt < 0) nt = 0;
     for (auto &kv : groups)
-      if (kv.second->n_items > 0) {
-        kv.second->run_steps(tick, nt, false);
+      if (kv.second->n_items > 0 && usable[kv.first]) {
+        const cudaError_t e = kv.second->run_steps(tick, nt, false);
         stats.grouped_launches += nt;
+        if (e != cudaSuccess) {
+          cudaGetLastError();
+          fail_group(kv.first, SB_ERR_CUDA, std::string("steps: ") + cudaGetErrorString(e));
+        }
       }
     tick += nt;
     for (Req *r : resident) r->ticks += nt;
