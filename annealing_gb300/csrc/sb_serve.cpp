@@ -237,10 +237,15 @@ void Server::fail_group(int nr, sb_status s, const std::string &err) {
 // Retires every resident request whose step budget ends at `at_tick` or that has failed, and drops cancelled ones.
 void Server::retire(int at_tick) {
   std::vector<Req *> fin, gone;
-  for (Req *r : resident) {
-    if (r->cancel) gone.push_back(r);
-    else if (r->status != SB_OK || r->ticks >= r->prm.steps) fin.push_back(r);
-  }
+  auto collect = [&] {
+    fin.clear();
+    gone.clear();
+    for (Req *r : resident) {
+      if (r->cancel) gone.push_back(r);
+      else if (r->status != SB_OK || r->ticks >= r->prm.steps) fin.push_back(r);
+    }
+  };
+  collect();
   if (fin.empty() && gone.empty()) return;
   // energies of the finishing requests, per engine
   std::map<int, std::vector<int>> by_group;
@@ -257,9 +262,19 @@ void Server::retire(int at_tick) {
         }
     }
   }
-  uint32_t status = 0;
+  // an engine whose waits gave up left some of its requests short of steps: all of them end here, and it starts anew
+  std::map<int, uint32_t> device_status;
   for (auto &kv : groups)
-    if (kv.second->d_status) cudaMemcpyAsync(&status, kv.second->d_status, 4, cudaMemcpyDeviceToHost, st);
+    if (kv.second->d_status)
+      cudaMemcpyAsync(&device_status[kv.first], kv.second->d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
+  cudaStreamSynchronize(st);
+  for (auto &kv : device_status)
+    if (kv.second != 0) {
+      fail_group(kv.first, (kv.second & sbk::kErrWaitTimeout) ? SB_ERR_TIMEOUT : SB_ERR_CUDA,
+                 sbh::device_status_text(kv.second));
+      cudaMemsetAsync(groups[kv.first]->d_status, 0, sizeof(uint32_t), st);
+    }
+  collect();
   std::vector<Req *> good;
   for (Req *r : fin)
     if (r->status == SB_OK) good.push_back(r);
@@ -307,7 +322,7 @@ void Server::retire(int at_tick) {
   {
     std::lock_guard<std::mutex> lk(mu);
     for (Req *r : fin)
-      check_q.push_back({r, (status & sbk::kErrWaitTimeout) ? SB_ERR_TIMEOUT : r->status});
+      check_q.push_back({r, r->status});
   }
   check_cv.notify_all();
   for (Req *r : gone) finish(r, SB_ERR_CANCELLED, "cancelled");

@@ -18,7 +18,7 @@ PROGRAM = r"""
 #include "sb_serve.cpp"
 
 // what fails, by replica tile (0: nothing)
-static std::atomic<int> fail_tables{0}, fail_steps{0}, steps_without_tables{0};
+static std::atomic<int> fail_tables{0}, fail_steps{0}, expire{0}, steps_without_tables{0};
 static std::atomic<int> recorded{0};  // the runtime's last error
 
 // ---- CUDA: device memory is host memory ----
@@ -88,6 +88,10 @@ cudaError_t Grouped::run_steps(int, int, bool) {
     return cudaErrorLaunchOutOfResources;
   }
   if (recorded != 0) return (cudaError_t)recorded.load();  // a launch looks at the last error
+  if (expire == nr) {
+    *d_status |= kErrWaitTimeout;
+    expire = 0;
+  }
   return cudaSuccess;
 }
 cudaError_t Grouped::energy_pass_for(const std::vector<int> &idx, int) {
@@ -135,6 +139,15 @@ int main() {
       poll("r32", d);
       poll("r64", e);
     }
+  for (int tile : {32, 64}) {
+    expire = tile;
+    const uint64_t a = submit(32, 300), b = submit(64, 300);
+    poll("r32", a);
+    poll("r64", b);
+    const uint64_t d = submit(32, 100), e = submit(64, 100);
+    poll("r32", d);
+    poll("r64", e);
+  }
   printf("stepped without tables %d\n", steps_without_tables.load());
   sbs::server_destroy(server);
 }
@@ -168,5 +181,8 @@ def test_each_engine_ends_its_own_requests(lines):
         bad, good = f"{failing} 0 {text}", "0 1 "
         want += [f"r32 {bad}", f"r64 {good}", f"r48 {good}", f"r32 {good}", f"r64 {good}"]   # tile 32 fails
         want += [f"r32 {good}", f"r64 {bad}", f"r48 {bad}", f"r32 {good}", f"r64 {good}"]    # tile 64
+    bad, good = f"{_status('SB_ERR_TIMEOUT')} 0 a bounded wait gave up", "0 1 "
+    want += [f"r32 {bad}", f"r64 {good}", f"r32 {good}", f"r64 {good}"]
+    want += [f"r32 {good}", f"r64 {bad}", f"r32 {good}", f"r64 {good}"]
     want += ["stepped without tables 0"]
     assert lines == want
