@@ -79,6 +79,7 @@ __global__ void __launch_bounds__(kThreads) cluster_kernel(const __grid_constant
     if ((lane & 15) < C) signs::st_async_u32(to + p * (uint32_t)sizeof(xs[0]), __float_as_uint(v), to_bar + p * 8u);
   };
   bool ok = true;
+  const float lost = sbasb::underflow_bound(a.mts_dt, a.kerr);  // aSB
   if (a.steps > 0) publish(0);
   float pump_next = a.steps > 0 ? a.pumps[0] : 0.0f;
   for (int t = 0; t < a.steps; ++t) {
@@ -132,7 +133,7 @@ __global__ void __launch_bounds__(kThreads) cluster_kernel(const __grid_constant
       __syncthreads();
       if (warp == 0) {
         float lx = sx[lane], ly = sy[lane];
-        sbasb::local(lx, ly, __fdiv_rn((float)(t + 1), (float)a.steps), a.m, a.mts_dt, a.detune, a.kerr);
+        sbasb::local(lx, ly, __fdiv_rn((float)(t + 1), (float)a.steps), a.m, a.mts_dt, a.detune, a.kerr, lost);
         sx[lane] = lx;
         sy[lane] = ly;
       }

@@ -938,6 +938,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1) plain_persist_kernel(Plain
   };
   publish(0);
   bool ok = true;
+  const float lost = sbasb::underflow_bound(a.mts_dt, a.kerr);  // aSB
   float pump_next = a.steps > 0 ? a.pumps[0] : 0.0f;
   for (int t = 0; t < a.steps && ok; ++t) {
     const float pump = pump_next;
@@ -985,7 +986,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1) plain_persist_kernel(Plain
         __syncthreads();
         if (warp == 0 && lane < kPersistRows) {
           float lx = sx[lane], ly = sy[lane];
-          sbasb::local(lx, ly, __fdiv_rn((float)(t + 1), (float)a.steps), a.m, a.mts_dt, a.detune, a.kerr);
+          sbasb::local(lx, ly, __fdiv_rn((float)(t + 1), (float)a.steps), a.m, a.mts_dt, a.detune, a.kerr, lost);
           sx[lane] = lx;
           sy[lane] = ly;
         }
