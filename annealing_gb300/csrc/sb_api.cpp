@@ -860,7 +860,9 @@ sb_status sb_destroy(sb_ctx *ctx) {
 sb_status sb_set_wait_limit(sb_ctx *ctx, int64_t cycles) {
   if (!ctx || cycles < 0) return SB_ERR_INVALID_ARG;
   std::lock_guard<std::mutex> lk(ctx->mu);
-  ctx->wait_cycles = cycles;
+  // a kernel whose wait gave up waits as long again for the copies and contractions it has in flight before it frees
+  // what they use: half a millisecond is far beyond any of them, a few clocks are not
+  ctx->wait_cycles = cycles == 0 ? 0 : std::max<int64_t>(cycles, SB_WAIT_LIMIT_LEAST);
   return SB_OK;
 }
 

@@ -221,6 +221,7 @@ __global__ void __launch_bounds__(kRunThreads, 1) run_kernel(const __grid_consta
       }
       __syncwarp();
       ok = __all_sync(0xffffffffu, ptx::mbar_wait(&a_bar, 0, limit));
+      if (!ok) ptx::mbar_wait(&a_bar, 0);  // given up, but the copies land before this CTA exits
     } else {
       int s = 0;
       uint32_t ph = 1;      // parity of the stage's last release (a fresh barrier passes parity 1)

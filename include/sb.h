@@ -277,8 +277,11 @@ const char *sb_last_error(sb_ctx *ctx);
  * another unit, an mbarrier of a copy or a contraction) gives up after `cycles` SM clock cycles;
  * the kernel then lets the copies and contractions it started finish, frees its tensor memory,
  * returns, and the call returns SB_ERR_TIMEOUT with the context still usable. 0 restores the
- * default (2e9 cycles, about one second at the maximum SM clock). Replaces the reference's
- * gpuErrchk, which ends the program on any CUDA error (m2_opt.cu:24-36). */
+ * default (2e9 cycles, about one second at the maximum SM clock); limits below SB_WAIT_LIMIT_LEAST
+ * (half a millisecond) count as that, since the kernel gives the copies it has in flight the same
+ * time to land. Replaces the reference's gpuErrchk, which ends the program on any CUDA error
+ * (m2_opt.cu:24-36). */
+#define SB_WAIT_LIMIT_LEAST 1000000
 sb_status sb_set_wait_limit(sb_ctx *ctx, int64_t cycles);
 /* Test hook for the timeout path above, a host-side fault injection: the next tensor-core solve of
  * this context runs with unit 0 (spins 0..127 of the first replica tile) leaving out its
