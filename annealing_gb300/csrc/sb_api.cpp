@@ -863,6 +863,7 @@ sb_status sb_set_wait_limit(sb_ctx *ctx, int64_t cycles) {
   // a kernel whose wait gave up waits as long again for the copies and contractions it has in flight before it frees
   // what they use: half a millisecond is far beyond any of them, a few clocks are not
   ctx->wait_cycles = cycles == 0 ? 0 : std::max<int64_t>(cycles, SB_WAIT_LIMIT_LEAST);
+  if (ctx->server) sbs::server_set_wait_limit(ctx->server, ctx->wait_cycles);
   return SB_OK;
 }
 
@@ -983,6 +984,7 @@ sb_status sb_submit(sb_ctx *ctx, const sb_problem *p, const sb_params *params, u
         ctx->last_error = err;
         return cs;
       }
+      sbs::server_set_wait_limit(ctx->server, ctx->wait_cycles);
     }
   }
   return sbs::server_submit(ctx->server, p, params, ticket);

@@ -252,6 +252,9 @@ sb_status run(sb_batch *b, uint64_t seed, sb_result *res, std::string &err) {
     if (cudaMemsetAsync(bk.g->d_status, 0, sizeof(uint32_t), st) != cudaSuccess) return SB_ERR_CUDA;
     l0 += bk.g->launches;
   }
+  for (auto &bk : b->buckets) bk.g->wait_cycles = b->ctx->wait_cycles;
+  b->buckets[0].g->skip_step = b->ctx->debug_skip_step;
+  b->ctx->debug_skip_step = -1;
   cudaEventRecord(b->ev0, st);
   for (auto &bk : b->buckets) {
     sb_status s = init_all(bk, seed, err);

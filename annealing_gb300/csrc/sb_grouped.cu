@@ -777,7 +777,12 @@ cudaError_t Grouped::run_wave(const Wave &w, int tick0, int count) {
   a.status = d_status;
   a.n_items = w.count;
   a.skip_item = a.skip_step = -1;
-  a.wait_cycles = ptx::kWaitCycles;
+  a.wait_cycles = wait_cycles > 0 ? wait_cycles : ptx::kWaitCycles;
+  if (skip_step >= 0) {
+    a.skip_item = 0;
+    a.skip_step = skip_step;
+    skip_step = -1;
+  }
   v_stale = true;
   for (int s0 = 0; s0 < count; s0 += kWaveSteps) {
     a.tick0 = tick0 + s0;

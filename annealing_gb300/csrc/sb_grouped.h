@@ -134,6 +134,10 @@ class Grouped {
   std::vector<GHost> insts;
   int64_t launches = 0;
   int n_items = 0;
+  // limit of the multi-step launches' waits (SM clock cycles, 0: the default), and the fault injection for the timeout
+  // path: skip_step >= 0 makes the next such launch's first item leave out its signs of that step
+  int64_t wait_cycles = 0;
+  int skip_step = -1;
   uint32_t *d_status = nullptr;
 
  private:

@@ -215,6 +215,8 @@ sb_status nmfa_run(sb_ctx *ctx, const sb_problem *prob, const sb_nmfa_params *pr
   NM_CUDA(sbk::launch_nmfa_seed(c->drng, n, R, xp, prm->seed, st));
   ++launches;
   if (use_tc) {
+    sbk::tc_set_waits(c->te, (long long)ctx->wait_cycles, ctx->debug_skip_step);
+    ctx->debug_skip_step = -1;
     NM_CUDA(sbk::tc_prepare(c->te, c->ds, st));
     NM_CUDA(sbk::tc_run_nmfa(c->te, 2 * stages, c->dbetas, c->ds, c->dz1, c->dnorm, c->drng, prm->noise,
                              (float)(1.0 - (double)prm->recombination), prm->recombination, c->dstatus, st));

@@ -465,6 +465,7 @@ __global__ void __launch_bounds__(kRunThreads, 1) run_kernel(const __grid_consta
         ptx::tmem_ld16(t_x, vx);
         ptx::tmem_ld16(t_y, vy);
         if (!__all_sync(0xffffffffu, ptx::mbar_wait(&accf_bar[ab], use & 1, limit))) {
+          ptx::tmem_ld_wait();  // the loads above, before tensor memory is freed
           ok = false;
           break;
         }

@@ -90,6 +90,7 @@ struct Server {
   void prepare_loop(int w);
   void attach_ready();
   int tick = 0;
+  std::atomic<int64_t> wait_cycles{0};
   sb_serving_stats stats{};
   sb_ctx *solo = nullptr;  // requests outside the grouped engine
   Clock::time_point t_start = Clock::now();
@@ -362,6 +363,7 @@ void Server::run() {
     if (nt < 0) nt = 0;
     for (auto &kv : groups)
       if (kv.second->n_items > 0 && usable[kv.first]) {
+        kv.second->wait_cycles = wait_cycles;
         const cudaError_t e = kv.second->run_steps(tick, nt, false);
         stats.grouped_launches += nt;
         if (e != cudaSuccess) {
@@ -453,6 +455,11 @@ void server_destroy(Server *s) {
   cudaStreamDestroy(s->st);
   for (auto ps : s->pst) cudaStreamDestroy(ps);
   delete s;
+}
+
+void server_set_wait_limit(Server *s, int64_t cycles) {
+  s->wait_cycles = cycles;
+  if (s->solo) sb_set_wait_limit(s->solo, cycles);
 }
 
 sb_status server_submit(Server *s, const sb_problem *p, const sb_params *prm, uint64_t *ticket) {

@@ -673,6 +673,9 @@ extern "C" sb_status sb_sqa_solve(sb_ctx *ctx, const sb_problem *prob, const sb_
       a.SPS = tc_sps;
       a.R = R;
       a.jstages = tc.jstages;
+      a.wait_cycles = ctx->wait_cycles > 0 ? ctx->wait_cycles : sbk::ptx::kWaitCycles;
+      a.skip_step = ctx->debug_skip_step;
+      ctx->debug_skip_step = -1;
       void *args[] = {&a};
       SQ_CUDA(cudaLaunchKernel(tc.kernel, dim3((unsigned)((R + tc.nrep - 1) / tc.nrep)), dim3((unsigned)sqatc::threads(tc.nrep)), args, tc.smem, st));
       SQ_CUDA(cudaGetLastError());

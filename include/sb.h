@@ -273,8 +273,9 @@ sb_status sb_time_to_target(const double *energies, const double *times_ms, int3
 sb_status sb_create(sb_ctx **out, const sb_device_opts *opts);
 sb_status sb_destroy(sb_ctx *ctx);
 const char *sb_last_error(sb_ctx *ctx);
-/* Bounded device waits. Every wait inside the persistent tensor-core kernels (a dataflow flag of
- * another unit, an mbarrier of a copy or a contraction) gives up after `cycles` SM clock cycles;
+/* Bounded device waits. Every wait inside the persistent tensor-core kernels of the context's solves, batches, SQA and
+ * NMFA calls and its serving loop (a dataflow flag or word of another unit, an mbarrier of a copy or a contraction)
+ * gives up after `cycles` SM clock cycles;
  * the kernel then lets the copies and contractions it started finish, frees its tensor memory,
  * returns, and the call returns SB_ERR_TIMEOUT with the context still usable. 0 restores the
  * default (2e9 cycles, about one second at the maximum SM clock); limits below SB_WAIT_LIMIT_LEAST
@@ -286,7 +287,9 @@ sb_status sb_set_wait_limit(sb_ctx *ctx, int64_t cycles);
 /* Test hook for the timeout path above, a host-side fault injection: the next tensor-core solve of
  * this context runs with unit 0 (spins 0..127 of the first replica tile) leaving out its
  * published flag of SB step `step`, so the units of its replica column wait for a flag that
- * nothing sets and give up at the wait limit. Nothing faults; no counterpart in the reference. */
+ * nothing sets and give up at the wait limit. A batch leaves out the signs of the first item of its
+ * first wave, SQA the first replica's operands of annealing step `step`. Nothing faults; no
+ * counterpart in the reference. */
 sb_status sb_debug_skip_publish(sb_ctx *ctx, int32_t step);
 
 /* One blocking solve from host buffers: upload J, run, copy results back. */

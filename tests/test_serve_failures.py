@@ -36,6 +36,7 @@ cudaError_t cudaGetLastError() { return (cudaError_t)recorded.exchange(0); }
 const char *cudaGetErrorString(cudaError_t) { return "launch refused"; }
 sb_status sb_create(sb_ctx **c, const sb_device_opts *) { *c = nullptr; return SB_ERR_NO_DEVICE; }
 sb_status sb_destroy(sb_ctx *) { return SB_OK; }
+sb_status sb_set_wait_limit(sb_ctx *, int64_t) { return SB_OK; }
 sb_status sb_solve(sb_ctx *, const sb_problem *, const sb_params *, sb_result *) { return SB_ERR_NO_DEVICE; }
 const char *sb_last_error(sb_ctx *) { return ""; }
 int64_t sb_plan_footprint(const sb_problem *, const sb_params *) { return 1; }
