@@ -57,6 +57,7 @@ struct sb_plan {
   uint8_t *dout = nullptr;      // results, packed
   uint64_t seed = 0;            // of the run in progress
   uint32_t *dplanes = nullptr;  // dSB with integer couplings up to 127: their bit planes, and how many magnitudes
+  bool may_plane = false;       // an untraced plain FP32 dSB plan: takes planes with couplings that have them
   bool cluster = false;         // the plain FP32 steps run in clusters (sb_cluster.cuh)
   int planes = 0;               // they have (0: the couplings uploaded are not such)
   float *dxk = nullptr;    // [kTopK][xp] rows of the best candidates (real-valued J)
@@ -296,10 +297,15 @@ sb_status upload_problem(sb_plan *pl, const sb_problem *p, std::string &err) {
       if (ts != SB_OK) return ts;
     }
   }
-  if (pl->dplanes) {
-    pl->planes = p->integer_valued ? sbk::sign_planes(n, pl->R, p->max_abs_j) : 0;
-    if (pl->planes) SB_CUDA(sbk::launch_sign_planes(pl->dJ, n, pl->jp, pl->planes, pl->dplanes, st));
+  // dSB with integer couplings: no exchange through L2 at all (sb_signs.cuh). The planes are made when a problem first
+  // takes them, so that what the plan was created with does not decide; without room for them the other forms run.
+  pl->planes = pl->may_plane && p->integer_valued ? sbk::sign_planes(n, pl->R, p->max_abs_j) : 0;
+  if (pl->planes && !pl->dplanes && cudaMalloc((void **)&pl->dplanes, sbk::sign_plane_bytes(n)) != cudaSuccess) {
+    cudaGetLastError();
+    pl->dplanes = nullptr;
+    pl->planes = 0;
   }
+  if (pl->planes) SB_CUDA(sbk::launch_sign_planes(pl->dJ, n, pl->jp, pl->planes, pl->dplanes, st));
   pl->copies.reset();
   pl->prob = p;
   if (p->integer_valued) pl->copies.reset(new sbh::CouplingCopies({p}));
@@ -362,9 +368,7 @@ sb_status plan_create(sb_ctx *ctx, const sb_problem *p, const sb_params *prm, sb
   if (mode == SB_FIELD_FP32 && !needs_trace(*prm) && prm->steps > 0) {
     const char *env = getenv("SB_PLAIN_PERSIST");
     const bool want = !(env && env[0] == '0');
-    // dSB with integer couplings: no exchange through L2 at all (sb_signs.cuh)
-    if (want && prm->variant == SB_DSB && p->integer_valued && sbk::sign_planes(pl->n, pl->R, p->max_abs_j))
-      PLAN_ALLOC(pl->dplanes, sbk::sign_plane_bytes(pl->n));
+    pl->may_plane = want && prm->variant == SB_DSB;
     pl->cluster = want && sbk::plain_cluster_fits(prm->variant, pl->n, pl->R, pl->jp);
     const int ctas = want && !pl->cluster ? sbk::plain_persist_ctas(pl->n, pl->R, pl->jp) : 0;
     if (ctas > 0) {

@@ -49,3 +49,26 @@ def test_energies_follow_the_problem(n, R, mode, dtype, kinds):
         np.testing.assert_array_equal(a.best_spins, b.best_spins)
         assert a.best_replica == b.best_replica
         assert a.energy_check_ok and b.energy_check_ok
+
+
+def test_the_form_follows_the_problem():
+    """Twelve replicas of 1000 spins fit no co-resident grid: integers take the one-launch bit planes whichever
+    couplings the plan began with, real ones a launch per step."""
+    n, R, steps = 1000, 12, 30
+    prm = sb.Params.default(sb.DSB, steps=steps, replicas=R, seed=4, field_mode=sb.FIELD_FP32, c0=0.03)
+    kinds = ("real", "1", "7", "real", "1")
+    problems = {k: _problem(k, n) for k in kinds}
+    ctx = sb.Context(0)
+    try:
+        got = [ctx.solve(problems[k], prm, want_state=True) for k in kinds]
+    finally:
+        ctx.close()
+    for k, a in zip(kinds, got):
+        ctx = sb.Context(0)
+        try:
+            b = ctx.solve(problems[k], prm, want_state=True)
+        finally:
+            ctx.close()
+        assert a.steps_per_launch == b.steps_per_launch == (1 if k == "real" else steps)
+        np.testing.assert_array_equal(a.final_x, b.final_x)
+        np.testing.assert_array_equal(a.final_y, b.final_y)
