@@ -380,7 +380,7 @@ sb_status run(sb_batch *b, uint64_t seed, sb_result *res, std::string &err) {
     r.energy_check_ok = okv[k];
     r.device_ms = dev_ms;
     r.kernel_ms_avg = kernel_ms;
-    r.steps_per_launch = 1;
+    r.steps_per_launch = b->prm.profile ? 1 : sbk::Grouped::steps_per_launch(*inst[k], steps);
     r.kernel_launches = launches;
     r.total_ms = total_ms;
     r.spin_updates_per_s = dev_ms > 0 ? updates / (dev_ms * 1e-3) : 0.0;

@@ -727,10 +727,11 @@ sb_status Grouped::build_waves(std::string &err) {
   int64_t bytes = 0;
   size_t ll = 0;
   for (int i : by_size) {
-    const GHost &g = insts[i];
+    GHost &g = insts[i];
     const int mt = g.Np / kBM, rt = g.Rp / nr, kc = grouped_kchunks(g.Kp, g.op);
     const size_t words = (size_t)2 * 4 * mt * nr;  // of one replica tile
-    if ((int64_t)mt * rt > most) {
+    g.wave = (int64_t)mt * rt <= most;
+    if (!g.wave) {
       for (int m = 0; m < mt; ++m)
         for (int r = 0; r < rt; ++r) rest.push_back(GItem{i, m * kBM, r * nr, kc});
       continue;
@@ -832,6 +833,8 @@ cudaError_t Grouped::launch_items(const GItem *items_ptr, int count, int tick, i
   ++launches;
   return cudaLaunchKernel(k, dim3(grid), dim3(kTcThreads), args, smem, st);
 }
+
+int Grouped::steps_per_launch(const GHost &g, int count) { return g.wave && count > 1 ? std::min(count, kWaveSteps) : 1; }
 
 cudaError_t Grouped::run_steps(int tick0, int count, bool use_graph) {
   if (count <= 0) return cudaSuccess;

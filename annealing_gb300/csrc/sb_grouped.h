@@ -63,6 +63,7 @@ struct GHost {
   float *x = nullptr, *y = nullptr, *h = nullptr, *pumps = nullptr;
   double *energy = nullptr;
   size_t out = 0;  // offset of its results in results()
+  bool wave = false;            // its steps run in a wave (valid after sync_tables)
   GInst desc;
 };
 
@@ -101,6 +102,8 @@ class Grouped {
   // a wave's steps in one launch (sb_run.cuh); a single step, and instances with more items than
   // a wave holds, take one launch per step (a CUDA graph of them when use_graph).
   cudaError_t run_steps(int tick0, int count, bool use_graph);
+  // SB steps of instance g that one launch of run_steps(., count, .) advances
+  static int steps_per_launch(const GHost &g, int count);
   // whether some instance does not fit a wave (valid after sync_tables)
   bool has_rest() const { return n_rest > 0; }
   // The initial state of every resident instance, seeded with seed + its tag (after sync_tables).

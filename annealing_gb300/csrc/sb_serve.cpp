@@ -53,6 +53,8 @@ struct Req {
   int nr = 0;
   int64_t bytes = 0;
   int ticks = 0;
+  int64_t launches = 0;       // of the kernels that stepped it and formed its energies
+  int steps_per_launch = 1;   // the most steps one of them advanced
   sb_status status = SB_OK;
   std::string err;
   std::vector<int8_t> spins;
@@ -138,6 +140,8 @@ void Server::solve_alone(Req *r) {
   r->best_r = res.best_replica;
   r->ok = res.energy_check_ok;
   r->ticks = p.steps;
+  r->launches = res.kernel_launches;
+  r->steps_per_launch = res.steps_per_launch;
   finish(r, s, s == SB_OK ? "" : std::string(sb_last_error(solo)));
 }
 
@@ -252,6 +256,7 @@ void Server::retire(int at_tick) {
   std::map<int, std::vector<int>> by_group;
   for (Req *r : fin)
     if (r->status == SB_OK) by_group[r->nr].push_back(groups[r->nr]->find((int)r->ticket));
+  for (Req *r : fin) ++r->launches;
   for (auto &kv : by_group) {
     cudaError_t e = groups[kv.first]->energy_pass_for(kv.second, at_tick);
     if (e != cudaSuccess) {
@@ -364,8 +369,15 @@ void Server::run() {
     for (auto &kv : groups)
       if (kv.second->n_items > 0 && usable[kv.first]) {
         kv.second->wait_cycles = wait_cycles;
+        const int64_t before = kv.second->launches;
         const cudaError_t e = kv.second->run_steps(tick, nt, false);
-        stats.grouped_launches += nt;
+        stats.grouped_launches += kv.second->launches - before;
+        for (Req *r : resident)
+          if (r->nr == kv.first && nt > 0) {
+            const int per = sbk::Grouped::steps_per_launch(kv.second->insts[kv.second->find((int)r->ticket)], nt);
+            r->launches += (nt + per - 1) / per;
+            r->steps_per_launch = std::max(r->steps_per_launch, per);
+          }
         if (e != cudaSuccess) {
           cudaGetLastError();
           fail_group(kv.first, SB_ERR_CUDA, std::string("steps: ") + cudaGetErrorString(e));
@@ -507,8 +519,8 @@ sb_status server_poll(Server *s, uint64_t ticket, sb_result *res, int32_t wait_m
     res->field_dtype_used = r->nr ? SB_OPERAND_FP6 : r->dtype;
     res->device_ms = std::chrono::duration<double, std::milli>(r->done - r->admitted).count();
     res->total_ms = std::chrono::duration<double, std::milli>(r->done - r->submitted).count();
-    res->kernel_launches = r->ticks;
-    res->steps_per_launch = 1;
+    res->kernel_launches = r->launches;
+    res->steps_per_launch = r->steps_per_launch;
     res->spin_updates_per_s =
         res->device_ms > 0 ? (double)r->prob->n * r->prm.replicas * r->prm.steps / (res->device_ms * 1e-3) : 0.0;
   }

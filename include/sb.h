@@ -194,9 +194,12 @@ typedef struct sb_result {
   double device_ms;            /* CUDA-event time of init + step loop + final energy */
   double kernel_ms_avg;        /* profile == 1: average device time of one launch of the step kernel
                                   (the tensor-core kernel runs every step in one launch), else 0 */
-  int32_t steps_per_launch;    /* SB steps one step-kernel launch advances (1 for the per-step plain
-                                  kernel, steps for the one-launch plain solve and the TC kernel) */
-  int64_t kernel_launches;     /* kernels this call launched on the device */
+  int32_t steps_per_launch;    /* SB steps one step-kernel launch advances: 1 for the launch-per-step
+                                  forms, steps for the one-launch plain solve, the TC kernel and a
+                                  batch's instance that runs in a wave; the most one launch advanced
+                                  for a served request */
+  int64_t kernel_launches;     /* kernels this call launched on the device (a served request: those
+                                  that stepped it and formed its energies) */
   double total_ms;             /* host wall time of the call, copies included */
   double spin_updates_per_s;   /* n * replicas * steps / (device_ms / 1e3) */
 } sb_result;
@@ -344,7 +347,7 @@ sb_status sb_cancel(sb_ctx *ctx, uint64_t ticket);
 /* latency of every finished request in submission order: arrival->result ms, and queue stats */
 typedef struct sb_serving_stats {
   int64_t submitted, finished, cancelled, inflight, queued;
-  int64_t grouped_launches;     /* device steps run by the serving loop */
+  int64_t grouped_launches;     /* kernels the serving loop launched to advance its requests */
   double busy_ms;               /* time the worker had work resident */
   int64_t peak_inflight;
   int64_t ticks;                /* SB steps the resident set advanced */

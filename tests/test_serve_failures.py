@@ -49,6 +49,7 @@ namespace sbk {
 bool grouped_supports(const sb_problem *, const sb_params *) { return true; }
 int64_t grouped_instance_bytes(int, int, int, int, int) { return 1; }
 Grouped::~Grouped() {}
+int Grouped::steps_per_launch(const GHost &, int) { return 1; }
 sb_status Grouped::prepare(GHost &g, const sb_problem *p, const sb_params *prm, uint64_t, int tag, int, cudaStream_t, Staging &,
                            std::string &, int) {
   g.tag = tag;
