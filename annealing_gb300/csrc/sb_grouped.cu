@@ -27,15 +27,6 @@ namespace sbk {
 namespace {
 using namespace tck;
 
-__global__ void g_convert_kernel(const float *J, int n, uint8_t *a, int Np, int Kp) {
-  const size_t total = (size_t)Np * Kp;
-  for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < total; k += (size_t)gridDim.x * blockDim.x) {
-    const size_t i = k / Kp, j = k % Kp;
-    const float v = (i < (size_t)n && j < (size_t)n) ? J[i * n + j] : 0.0f;
-    a[k] = (uint8_t)__nv_cvt_float_to_fp8(v, __NV_SATFINITE, __NV_E4M3);
-  }
-}
-
 __global__ void g_signs_kernel(const float *x, int n, int R, int xp, uint8_t *v, int Kp) {
   const size_t total = (size_t)n * R;
   for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < total; k += (size_t)gridDim.x * blockDim.x) {
@@ -416,7 +407,6 @@ void Grouped::clear() {
   cudaFree(d_insts);
   cudaFree(d_items);
   cudaFree(d_status);
-  cudaFree(d_stage);
   cudaStreamSynchronize(st);
   cudaFreeHost(stg_.pin);
   stg_.pin = nullptr;
@@ -440,9 +430,7 @@ void Grouped::clear() {
   d_insts = nullptr;
   d_items = nullptr;
   d_status = nullptr;
-  d_stage = nullptr;
   graph = nullptr;
-  stage_bytes = 0;
   cap_insts = cap_items = 0;
 }
 
@@ -570,11 +558,6 @@ sb_status Grouped::add(const sb_problem *p, const sb_params *prm, uint64_t seed,
   if (s != SB_OK) return s;
   attach(g, t0);
   return SB_OK;
-}
-
-
-sb_status Grouped::init_state(GHost &g, uint64_t seed, std::string &err) {
-  return init_state_on(g, seed, st, err);
 }
 
 sb_status Grouped::init_state_on(GHost &g, uint64_t seed, cudaStream_t st, std::string &err) {

@@ -121,7 +121,6 @@ class Grouped {
       if (insts[i].tag == tag) return (int)i;
     return -1;
   }
-  sb_status init_state(GHost &g, uint64_t seed, std::string &err);
   std::string tune_key() const;
   static std::vector<std::pair<int, int>> candidates(int R);
   void set_order(int o) {
@@ -171,8 +170,6 @@ class Grouped {
   GInst *d_insts = nullptr;
   GItem *d_items = nullptr;
   int cap_insts = 0, cap_items = 0;
-  float *d_stage = nullptr;
-  size_t stage_bytes = 0;
   Staging stg_;
   bool dirty = true;
   cudaGraphExec_t graph = nullptr;

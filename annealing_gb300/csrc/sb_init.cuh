@@ -1,4 +1,4 @@
-// The hash-mode initial state, shared by the plain and the grouped kernels.
+// The counter hash of every seeded draw, and the hash-mode initial state of the plain and the grouped kernels.
 #pragma once
 #include <stdint.h>
 

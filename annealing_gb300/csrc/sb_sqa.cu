@@ -42,6 +42,7 @@
 #include "sb.h"
 #include "sb_ctx.h"
 #include "sb_host.h"
+#include "sb_init.cuh"
 #include "sb_internal.h"
 #include "sb_math.cuh"
 #include "sb_ptx.cuh"
@@ -65,12 +66,6 @@ struct SqaArgs {
   int n, W, P, RW, M, steps, S, trace;
   int RS, SPS;            // shared-memory strides of a ring slot and of a slice (bank-spread padding)
 };
-
-__device__ __forceinline__ uint64_t sqa_mix64(uint64_t z) {
-  z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ULL;
-  z = (z ^ (z >> 27)) * 0x94D049BB133111EBULL;
-  return z ^ (z >> 31);
-}
 
 // Field of `row` against slice bits `sm`, summed over the warp (every lane gets it). A row stores,
 // per 32-coupling word w, the sign word then the P magnitude words (row[w (P + 1) + k]), and the
@@ -234,7 +229,7 @@ __global__ void __launch_bounds__(kSqaMaxWarps * 32, 1) sqa_kernel(const __grid_
         const int cnt = min(kSqaChunk, iters - a) * M;
         for (int k = tid; k < cnt; k += blockDim.x) {
           const uint64_t e = e_step + (uint64_t)a * M + (uint64_t)k;  // (a + k / M) M + k % M
-          const uint64_t z = sqa_mix64((p.seed ^ 0xD1B54A32D192ED03ULL) + 0x9E3779B97F4A7C15ULL * (e + 1));
+          const uint64_t z = sbk::mix64((p.seed ^ 0xD1B54A32D192ED03ULL) + 0x9E3779B97F4A7C15ULL * (e + 1));
           thr[k] = sqa_threshold(__fmul_rn((float)(uint32_t)(z >> 40), 0x1p-24f), beta);
         }
         __syncthreads();
@@ -383,7 +378,7 @@ __global__ void sqa_init_kernel(uint32_t *spins, uint32_t *rnd, int n, int W, in
         neg = (st & 1u) == 0u;  // ((st & 1) << 1) - 1 == -1
       } else {
         const uint64_t e = ((uint64_t)r * M + m) * n + i;
-        neg = (sqa_mix64(seed + 0x9E3779B97F4A7C15ULL * (e + 1)) >> 63) != 0;
+        neg = (sbk::mix64(seed + 0x9E3779B97F4A7C15ULL * (e + 1)) >> 63) != 0;
       }
       const uint32_t word = __ballot_sync(0xffffffffu, in && neg);
       if ((threadIdx.x & 31) == 0 && i < W * 32) spins[((size_t)r * M + m) * W + (i >> 5)] = word;
