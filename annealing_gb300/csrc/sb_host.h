@@ -18,7 +18,7 @@ namespace sbh {
 // returns when all have finished. Safe to call from several threads at once; a caller waiting for
 // its own tasks runs queued ones meanwhile.
 void parallel_run(int nt, const std::function<void(int)> &fn);
-// Makes the pages of a caller's result array present (each byte read is written back) while the device works:
+// Makes the pages of a caller's pageable result array present (each byte read is written back) while the device works:
 // a copy from the device into pages that were never touched faults them one by one (16 MB of states took
 // 15 ms to arrive, 0.5 ms into present pages).
 void touch_pages(void *p, size_t bytes);

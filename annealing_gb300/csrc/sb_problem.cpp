@@ -567,6 +567,13 @@ void sbh::touch_pages(void *p, size_t bytes) {
   constexpr size_t kLeast = 256 * 1024;  // below it the copy's own faults take less than 100 us
   volatile char *c = static_cast<volatile char *>(p);
   if (!p || bytes < kLeast) return;
+  // pinned pages are present, and the host may have no access to a device array (the copy into one works)
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return;
+  }
+  if (at.type != cudaMemoryTypeUnregistered) return;
   for (size_t k = 0; k < bytes; k += kPage) c[k] = c[k];
   c[bytes - 1] = c[bytes - 1];
 }
