@@ -82,17 +82,20 @@ NCU_TRAFFIC = {
     "plain-dsb": (16.03e6, "profiles/plain_step_kernel_plain_dsb_n2000.md"),
     # the same in one launch per solve: the couplings' bit planes, read once
     "plain-dsb-signs": (1.06e6, "profiles/one_launch_kernels.md"),
-    # batched bSB, N=8192, R=256, BF16 hi+lo with the field accumulated in K segments: bytes per SB
-    # step (8-step capture of the step launch: 2.587 GB; 4 steps: 1.146 GB), times the launch's steps
-    "batched-bsb": (2.587e9 / 8, "profiles/tc_sb_kernel_batched_bsb_n8192_r256.md"),
-    # uneven batch: measured bytes per algorithmic byte on a 48-instance batch (441.2 MB of
-    # 451.8 MB); the launch of the full batch is scaled by its algorithmic bytes
-    "uneven-batch": (441.2 / 451.8, "profiles/grouped_kernel_uneven_batch_48_instances.md"),
-    # the same with E2M1 couplings (255.2 MB of 284.0 MB)
-    "uneven-batch-e2m1": (255.2 / 284.0, "profiles/grouped_kernel_uneven_batch_48_instances.md"),
-    # the same with packed E2M3 couplings (349.6 MB of 366.7 MB)
-    "uneven-batch-e2m3": (349.6 / 366.75, "profiles/grouped_kernel_uneven_batch_48_instances.md"),
 }
+
+
+def run_kernel_takes(dtype, n, R, sms):
+    """Whether an untraced dSB solve runs in the multi-step kernel (run_shape in csrc/sb_tc.cu)."""
+    if dtype not in ("fp4e2m1", "fp8e4m3", "bf16") or (dtype == "fp4e2m1" and n > 9 * 256):
+        return False
+    return -(-n // 128) * (-(-R // 64) + 1 >> 1) <= sms
+
+
+def tensor_rate(dtype):
+    """A tensor operand type's dense rate over BF16's, from the nominal peaks (BF16 2.25, FP8 and E2M3 4.5, E2M1
+    13.5 PFLOP/s)."""
+    return {"fp4e2m1": 6.0, "fp8e4m3": 2.0, "fp6e2m3": 2.0}.get(dtype, 1.0)
 
 
 def peaks():
@@ -423,20 +426,21 @@ def run_ours(args, rank, world, local_rank):
     if field == "tc":
         fdt = results[0].field_dtype
         # FP8 and E2M1 peaks from the measured BF16 burst by the nominal dense ratios
-        # (BF16 2.25, FP8 4.5, E2M1 13.5 PFLOP/s)
-        scale, label = {"fp4e2m1": (6.0, "6 x {} dense BF16 burst (E2M1 rate, nominal 13.5 / 2.25)"),
-                        "fp8e4m3": (2.0, "2 x {} dense BF16 burst (FP8 E4M3 rate)")}.get(fdt, (1.0, "{} dense BF16 burst"))
-        tc_peak = scale * bf16
+        label = {"fp4e2m1": "6 x {} dense BF16 burst (E2M1 rate, nominal 13.5 / 2.25)",
+                 "fp8e4m3": "2 x {} dense BF16 burst (FP8 E4M3 rate)"}.get(fdt, "{} dense BF16 burst")
+        tc_peak = tensor_rate(fdt) * bf16
+        multi = variant == "dsb" and run_kernel_takes(fdt, n, R, torch.cuda.get_device_properties(dev).multi_processor_count)
         achieved = flops_per_launch / (rp.kernel_ms_avg * 1e-3) / 1e12
-        if fdt == "fp4e2m1" and n == 2000 and R == 1024:
+        if multi and fdt == "fp4e2m1" and n == 2000 and R == 1024:
             traffic = NCU_TRAFFIC["batched-dsb"]
-        elif fdt in ("bf16x2", "fp16x2") and n == 8192 and R == 256:
-            traffic = (NCU_TRAFFIC["batched-bsb"][0] * rp.steps_per_launch, NCU_TRAFFIC["batched-bsb"][1])
+        elif fdt == "bf16x2" and variant == "bsb" and n == 8192 and R == 256:
+            traffic = (None, "none: ncu gives no counters for the cooperative launch of CTA pairs")
         else:
             traffic = (None, None)
         roof = {"bound": "tensor", "achieved": achieved, "peak": tc_peak, "unit": "TFLOP/s",
                 "frac": achieved / tc_peak, "traffic": traffic[0], "traffic_source": traffic[1],
-                "kernel": ("run_kernel" if fdt == "fp4e2m1" else "tc_sb_kernel") + " (persistent, one launch per solve)",
+                "kernel": ("run_kernel" if multi else "tc_fp4_kernel" if fdt == "fp4e2m1" else "tc_sb_kernel")
+                + " (persistent, one launch per solve)",
                 "launch_ms": rp.kernel_ms_avg, "sb_steps_per_launch": rp.steps_per_launch,
                 "flops_per_launch": flops_per_launch, "peak_source": label.format(src),
                 "frac_of_bf16_burst": achieved / bf16}
@@ -448,7 +452,11 @@ def run_ours(args, rank, world, local_rank):
         bytes_per_launch = (4.0 * n * n + 16.0 * n * R) * spl
         achieved = bytes_per_launch / (rp.kernel_ms_avg * 1e-3) / 1e9
         limiter = None
-        if spl > 1:
+        if spl > 1 and not (variant == "dsb" and prob.s.integer_valued and n <= 2048):
+            traffic = (None, None)
+            kernel = ("cluster_kernel" if n <= 512 else "plain_persist_kernel") + " (one launch per solve)"
+            note = "J rows live in registers for the whole launch and are read once; a step's exchange of x bounds it"
+        elif spl > 1:
             traffic = NCU_TRAFFIC["plain-dsb-signs"] if n == 2000 and R == 1 else (None, None)
             kernel = "signs_kernel (one launch per solve)"
             note = ("achieved counts the algorithmic 4 N^2 bytes of J per SB step, but the +-1 couplings live in "
@@ -506,7 +514,7 @@ def run_ours(args, rank, world, local_rank):
                   "fp8e4m3": "fp8e4m3 field (f32 accumulate), f32 state",
                   "bf16x2": "bf16 hi+lo field (f32 accumulate), f32 state",
                   "fp16x2": "fp16 hi+lo field, power-of-two scaled (f32 accumulate), f32 state",
-                  "bf16": "bf16 field (f32 accumulate), f32 state",
+                  "bf16": "int field as 16 hi + lo in e4m3 (f32 accumulate, exact for |J| <= 256), f32 state",
                   "f32": "f32"}[results[0].field_dtype],
         "data": "synthetic (seeded; the reference's WK2000_1.rud is not shipped)",
         "config": {"workload": desc, "n": n, "replicas": R, "sb_steps": sb_steps,
@@ -611,33 +619,26 @@ def run_batch(args, rank, world, local_rank):
     total_ms = reduce_max(float(sum(times)), world)
     updates = float(n_sum) * R * sb_steps
     value = weak_scaling_value(updates, world, args.steps, total_ms)
-    # roofline: one profiled run, event pair around every grouped step launch
-    prm_p = sb.Params.default(sb.DSB, steps=24, replicas=R, seed=7, field_mode=sb.FIELD_TC, profile=1,
-                              operand_dtype=odt)
-    bp = ctx.batch(probs, prm_p)
-    bp.run()
-    rp = bp.run(seed=8)
-    bp.close()
+    # roofline of the timed runs themselves: a wave of instances takes all its steps in one launch, its couplings in L2
+    # (the per-step launch that a profiled run times streams them from HBM every step)
     hbm, bf16, src = peaks()
-    dts = [r.field_dtype for r in rp]  # each instance's operand bucket
+    dts = [r.field_dtype for r in res]  # each instance's operand bucket
     fp4 = all(d == "fp4e2m1" for d in dts)
     np_kp = sum(operand_row_bytes(p.n, d) * ((p.n + 127) // 128 * 128) for p, d in zip(probs, dts))
-    # J + per spin-replica: x, y read and written (16 B) and the next sign operand (1 B, 3/4 or 1/2)
-    bytes_per_launch = np_kp + sum(p.n * R * (16.0 + SIGN_BYTES[d]) for p, d in zip(probs, dts))
-    achieved = bytes_per_launch / (rp[0].kernel_ms_avg * 1e-3) / 1e9
-    tkey = {"fp4e2m1": "uneven-batch-e2m1", "fp6e2m3": "uneven-batch-e2m3"}.get(dts[0], "uneven-batch") \
-        if len(set(dts)) == 1 else None
-    roof = {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
-            "traffic": NCU_TRAFFIC[tkey][0] * bytes_per_launch if tkey else None,
-            "traffic_source": (NCU_TRAFFIC[tkey][1] + " (48-instance capture, scaled by algorithmic bytes)")
-            if tkey else None,
-            "kernel": "grouped_kernel (one launch per SB step)",
-            "launch_ms": rp[0].kernel_ms_avg, "bytes_per_launch": bytes_per_launch,
-            "peak_source": f"{src} HBM copy",
-            # the timed solves run sets of instances whose couplings stay in L2 for all steps in one launch
-            # (run_kernel), so their time per SB step, init and energies included, is below that of the
-            # event-timed launch above, the form that takes one step of every instance from HBM
-            "timed_ms_per_sb_step": total_ms / args.steps / sb_steps}
+    step_s = total_ms * 1e-3 / args.steps / sb_steps
+    flops = sum(2.0 * p.n * p.n * R for p in probs)
+    least_s = sum(2.0 * p.n * p.n * R / (tensor_rate(d) * bf16 * 1e12) for p, d in zip(probs, dts))
+    in_waves = all(r.steps_per_launch > 1 for r in res)
+    roof = {"bound": "tensor", "achieved": flops / step_s / 1e12, "peak": flops / least_s / 1e12, "unit": "TFLOP/s",
+            "frac": least_s / step_s, "traffic": None, "traffic_source": None,
+            "kernel": "run_kernel (every step of a wave in one launch)" if in_waves
+            else "run_kernel, grouped_kernel for instances that fit no wave",
+            "ms_per_sb_step": 1e3 * step_s, "sb_steps_per_launch": int(max(r.steps_per_launch for r in res)),
+            "coupling_gbs": np_kp / step_s / 1e9,
+            "note": "time of the timed runs, initial states and energies included; 2 N^2 R operations a step and instance, "
+                    "peak = each instance's at its operand type's rate; coupling_gbs: operand bytes of J a step over the "
+                    "time, read from L2 after a wave's first step",
+            "peak_source": f"{src} BF16 burst x the nominal dense ratios"}
     # e2e: from host couplings every step through the public calls: sb_problem_wrap of each
     # instance (its coupling scan), then the batch (upload, convert, run, results back)
     import ctypes
@@ -688,10 +689,11 @@ def serve_stream(sb, ctx, count, rate, pool_size, R, seed, device, warmup=2):
     `rate`, N log-uniform in [128, 16384], density U[0.01, 1], J ~ U{-8..8}, R replicas, step budget
     U[500, 4000]. A pool of distinct instances drawn from the same size distribution stands in for
     the couplings (each request takes the pool instance nearest its own N), which keeps host memory
-    bounded. Latency = submit to result (the library's per-request total_ms). The stream's HBM
-    fraction counts the algorithmic bytes the resident requests' steps read and write (FP8 couplings
-    Np x Kp per step, x and y read and written and the next sign operand, 17 B per spin and replica)
-    over the worker's busy time."""
+    bounded. Latency = submit to result (the library's per-request total_ms). algorithmic_over_hbm
+    counts the bytes the resident requests' steps would move if every step went to HBM (couplings as
+    stored, x and y read and written and the next sign operand) over the worker's busy time: how
+    much is asked of the memory system, not HBM's share, since a wave's couplings come from L2 after
+    its first step and its states stay on chip for up to 64."""
     import threading as th
 
     from annealing_gb300 import instances
@@ -758,8 +760,9 @@ def serve_stream(sb, ctx, count, rate, pool_size, R, seed, device, warmup=2):
             "p50_ms_second_half": float(np.percentile(lat[half:], 50)),
             "spin_updates_per_s": updates / makespan, "busy_ms": busy_ms,
             "admit_ms": stats["admit_ms"] - stats0["admit_ms"],
-            "hbm_fraction": (algo_bytes / (busy_ms * 1e-3) / 1e9) / hbm if busy_ms > 0 else None,
-            "hbm_bytes": algo_bytes, "peak_source": f"{src} HBM copy",
+            "algorithmic_bytes": algo_bytes,
+            "algorithmic_over_hbm": (algo_bytes / (busy_ms * 1e-3) / 1e9) / hbm if busy_ms > 0 else None,
+            "peak_source": f"{src} HBM copy",
             "pool_instances": len(pool), "replicas": R,
             "energy_check_ok": all(r.energy_check_ok for r in results), "clocks": clk.summary(),
             "_updates": updates, "_results": results, "_reqs": reqs, "_stats": stats}
@@ -905,7 +908,7 @@ def run_sqa(args, rank, world, local_rank):
         "metric": "SQA spin-updates/s", "value": value, "unit": "spin-updates/s", "n_gpus": world,
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": total_dev / args.steps,
         "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-        "dtype": "int (bit-plane couplings, popcount fields), f32 acceptance test",
+        "dtype": "int (E2M1 couplings on the tensor cores, flips inside a block by popcounts, exact), f32 acceptance test",
         "data": "synthetic (seeded +-1 complete graph)",
         "config": {"workload": desc, "n": n, "trotter": M, "replicas": R, "anneal_steps": steps,
                    "rng": "hash", "parallelism": f"replicas-only x{world}",

@@ -77,15 +77,18 @@ typedef enum sb_variant { SB_ASB = 0, SB_BSB = 1, SB_DSB = 2 } sb_variant;
 
 /* How the field J*v is computed.
  *  SB_FIELD_AUTO: tensor cores when replicas >= 32 and the problem allows an exact/declared
- *                 precision, otherwise the plain FP32 path; dSB with integer couplings whose bit
- *                 planes are faster (n^2 x replicas small: up to 64 to 300 million) takes the
- *                 plain path too (the same bits).
+ *                 precision, otherwise the plain FP32 path. Untraced dSB with integer couplings
+ *                 whose bit planes are faster takes the plain path too (the same bits): with P the
+ *                 bits of max |J|, n^2 x replicas x P up to 134 million for n <= 512 (256 with
+ *                 |J| > 1), up to 64 million above; with |J| of 5 to 127 up to 205 million, n rounded
+ *                 up to a power of two.
  *  SB_FIELD_FP32: the plain fused FP32 path (the drop-in form). dSB with integer |J| <= 127 and
  *                 n <= 512 (|J| <= 15: n <= 1024, |J| <= 1: n <= 2048) runs the whole solve in one launch
- *                 on bit planes of J (exact integer fields). Otherwise the whole solve is one cooperative launch when
- *                 the rows fit one co-resident grid (n <= 2048, ceil(n / 16) x replicas CTAs on the
- *                 SMs), else, and with an energy trace, one launch per step; the same bits each way
- *                 (environment SB_PLAIN_PERSIST=0 keeps one launch per step).
+ *                 on bit planes of J (exact integer fields). Otherwise the whole solve is one launch of
+ *                 clusters for n <= 512 (ceil(n / 32) x replicas CTAs, up to four to an SM), or one
+ *                 cooperative launch when the rows fit one co-resident grid (n <= 2048, ceil(n / 16) x
+ *                 replicas CTAs on the SMs), else, and with an energy trace, one launch per step; the
+ *                 same bits each way (environment SB_PLAIN_PERSIST=0 keeps one launch per step).
  *  SB_FIELD_TC:   tcgen05 tensor cores. dSB with integer |J| <= 4 and n <= ~2300: packed E2M1
  *                 operands, FP32 accumulation (bit-exact); without a trace every step in one launch.
  *                 dSB with integer |J| <= 16: FP8 E4M3 operands (grouped batches and serving:
