@@ -422,6 +422,8 @@ cudaError_t enqueue_energy(sb_plan *pl, const float *x, double *slot, cudaStream
   a.x = x;
   a.energy = slot;
   a.status = pl->dstatus;
+  a.variant = pl->prm.variant;
+  a.traced = needs_trace(pl->prm) ? 1 : 0;
   return sbk::launch_plain_energy(a, fp64, st);
 }
 
@@ -558,6 +560,7 @@ cudaError_t enqueue_loop(sb_plan *pl, cudaStream_t st, std::vector<cudaEvent_t> 
     // consecutive steps overlap (J is never written inside the loop); profiled runs time each
     // launch alone between its events
     a.overlap = evs ? 0 : 1;
+    a.traced = tr ? 1 : 0;
     e = sbk::launch_plain_step(a, st);
     if (e != cudaSuccess) return e;
     if (evs) cudaEventRecord((*evs)[2 * t + 1], st);

@@ -45,6 +45,7 @@ struct PlainStep {
   // 1: launched with programmatic stream serialization, so the launch overlaps the previous
   // kernel's tail (J must not be written by that kernel: J copies start before the wait for it)
   int overlap;
+  int traced;              // 1: a solve that records every step's energies (they decide the kernel's form too)
   int stages;              // set by launch_plain_step
 };
 
@@ -128,6 +129,7 @@ struct PlainEnergy {
   const float *x;
   double *energy;          // [R] += energy of s(x)
   uint32_t *status;
+  int variant, traced;     // as PlainStep's of the steps it runs between (traced 0: by itself)
   int stages;              // set by launch_plain_energy
 };
 

@@ -1111,17 +1111,43 @@ cudaError_t launch_row_warps(void (*ring)(Args), void (*wide)(Args), const Args 
 }
 
 // Which shapes take the register tiles. A tile CTA covers 32 rows x 16 replicas whatever R is, so with
-// few replicas or rows it leaves SMs idle and lanes on padding. Measured, us per dSB step, row-per-warp
-// against tiles: n = 300 R = 6 4.9 / 5.2, R = 8 5.4 / 5.2; n = 1000 R = 6 7.8 / 7.9, R = 8 8.8 / 7.9;
-// n = 2048 R = 5 12.8 / 13.7, R = 8 15.5 / 13.6, R = 100 94 / 32; n = 4000 R = 3 25.0 / 26.2, R = 5
-// 29.9 / 26.0, R = 100 365 / 118.
-bool use_tiles(int n, int R) { return R >= 8 || (n >= 3000 && R >= 4); }
+// few replicas or rows it leaves SMs idle and lanes on padding. Measured, us per step, row-per-warp against tiles:
+//   bSB, dSB, NMFA: dSB n = 300 R = 6 4.9 / 5.2, R = 8 5.4 / 5.2; n = 1000 R = 6 7.8 / 7.9, R = 8 8.8 / 7.9;
+//   n = 2048 R = 5 12.8 / 13.7, R = 8 15.5 / 13.6, R = 100 94 / 32; n = 4000 R = 3 25.0 / 26.2, R = 5 29.9 / 26.0,
+//   R = 100 365 / 118. A traced dSB step, which sums energies too: n = 400 R = 12 5.0 / 6.2, R = 20 5.9 / 6.3, R = 40 6.4 / 6.3;
+//   n = 300 R = 12 5.2 / 5.7; n = 513 R = 16 7.1 / 7.0; n = 200 R = 16 5.7 / 5.1; n = 512 R = 12 4.7 / 5.9, R = 20
+//   5.5 / 5.6. Traced bSB: n = 400 R = 16 9.9 / 10.3, R = 32 1.10 times; n = 256 R = 20 8.6 / 7.6.
+//   aSB: a tile's threads take two elements' local sub-steps one after the other, a row-per-warp CTA's two warps
+//   one each: n = 300 R = 64 6.7 / 9.4, R = 128 9.0 / 9.5; n = 400 R = 80 9.3 / 9.9, R = 100 11.6 / 10.3; n = 512 R = 64
+//   9.4 / 9.8; n = 513 R = 12 7.0 / 10.3, R = 40 9.7 / 10.5, R = 64 1.05 times; n = 700 R = 12 9.1 / 10.7, R = 24 0.91 times, R = 32 1.01;
+//   n = 1000 R = 20 0.88 times, R = 32 1.11; n = 1400 R = 8 1.16, R = 12 0.96, R = 16 1.09 times.
+//   A traced solve's energy pass takes the form of its steps: mixed (n = 200 R = 12, bSB) 8.7 against 8.0 in tiles.
+enum TileUse { kTileStep, kTileTraced, kTileAsb, kTileTracedAsb };
+bool use_tiles(TileUse use, int n, int R) {
+  if (n >= 3000) return R >= 4;
+  if (R < 8) return false;
+  const int ctas = ((n + 7) / 8) * ((R + 7) / 8);  // of the row-per-warp form
+  switch (use) {
+    case kTileStep: return true;
+    case kTileTraced: return n <= 256 || n > 512 || R > (n <= 480 ? 24 : 16);
+    case kTileAsb:
+    case kTileTracedAsb:
+      if (n >= 1400) return true;
+      if (n >= 640) return R >= 24 || (R == 8 && n < 900);
+      if (use == kTileAsb) return ctas >= (n <= 512 ? 600 : 520);
+      return n <= 64 || (n <= 512 ? ctas >= 400 : R >= 40);
+  }
+  return false;
+}
+TileUse tile_use(int variant, int traced) {
+  return variant == 0 ? (traced ? kTileTracedAsb : kTileAsb) : traced ? kTileTraced : kTileStep;
+}
 
 cudaError_t launch_plain_step(const PlainStep &a0, cudaStream_t st) {
   plain_attrs();
   if (a0.rb < 1 || a0.rb > kMaxRB || a0.jp % 4 || a0.xp % 4 || a0.jp > a0.xp || a0.jp < 4)
     return cudaErrorInvalidValue;
-  const bool tile = use_tiles(a0.n, a0.R), ov = a0.overlap != 0;
+  const bool tile = use_tiles(tile_use(a0.variant, a0.traced), a0.n, a0.R), ov = a0.overlap != 0;
   switch (a0.variant) {
     case 0:
       return tile ? launch_tiles(plain_tile_kernel<0>, a0, a0.x_in, ov, st)
@@ -1211,15 +1237,15 @@ void cluster_config(int C, int R, int threads, cudaLaunchConfig_t &cfg, cudaLaun
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
 }
-// Whether such a cluster can run: more than eight CTAs need the attribute, and SMs of one GPC free for them.
-bool cluster_runs(const void *k, const cudaLaunchConfig_t &cfg) {
+// How many such clusters run at once (0: none; more than eight CTAs need the attribute, and SMs of one GPC free for them).
+int clusters_at_once(const void *k, const cudaLaunchConfig_t &cfg) {
   int clusters = 0;
   if (cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
       cudaOccupancyMaxActiveClusters(&clusters, k, &cfg) != cudaSuccess) {
     cudaGetLastError();
-    return false;
+    return 0;
   }
-  return clusters > 0;
+  return clusters;
 }
 
 const void *signs_kernel_for(int n, int P) {
@@ -1252,12 +1278,14 @@ int sign_planes(int n, int R, int max_abs_j) {
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr;
   signs_config(n, R, P, cfg, attr);
-  return cluster_runs(k, cfg) ? P : 0;
+  return clusters_at_once(k, cfg) > 0 ? P : 0;
 }
 
 // Up to four CTAs to an SM the clusters beat every other form; beyond, a launch per step on register tiles runs more
 // replicas at once. us per step, clusters / tiles: n = 128 R = 200 (800 CTAs) 2.8 / 3.6, R = 300 3.6 / 3.8 (NMFA
 // 4.7 / 3.9); n = 256 R = 64 (512) 2.6 / 4.3, R = 150 (1200) 4.9 / 4.3; n = 512 R = 32 (512) 4.5 / 5.4, R = 64 6.8 / 5.5.
+// aSB, whose step is mostly the local sub-steps' chain, while its clusters run in two rounds: n = 512 R = 28 5.9 against 7.0
+// a launch per step, R = 31 (a third round) 8.5 / 6.9; n = 400 R = 36 5.7 / 6.9, R = 40 7.9 / 6.9; n = 300 R = 56 5.3 / 6.7.
 bool plain_cluster_fits(int variant, int n, int R, int jp) {
   if (n < 1 || n > kClusterMaxN || R < 1 || jp < 4 || jp % 4 || jp > kClusterMaxN) return false;
   const int C = (n + cluster::kRows - 1) / cluster::kRows;
@@ -1268,7 +1296,8 @@ bool plain_cluster_fits(int variant, int n, int R, int jp) {
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr;
   cluster_config(C, R, cluster::kThreads, cfg, attr);
-  return cluster_runs(cluster_kernel_for(variant), cfg);
+  const int at_once = clusters_at_once(cluster_kernel_for(variant), cfg);
+  return variant == 0 ? R <= 2 * at_once : at_once > 0;
 }
 
 cudaError_t launch_plain_cluster(const PlainPersist &a, cudaStream_t st) {
@@ -1310,7 +1339,8 @@ cudaError_t launch_plain_energy(const PlainEnergy &a0, bool fp64, cudaStream_t s
   plain_attrs();
   if (a0.rb < 1 || a0.rb > kMaxRB || a0.jp % 4 || a0.xp % 4 || a0.jp > a0.xp || a0.jp < 4)
     return cudaErrorInvalidValue;
-  if (!fp64 && use_tiles(a0.n, a0.R)) return launch_tiles(plain_tile_energy_kernel, a0, a0.x, false, st);
+  if (!fp64 && use_tiles(a0.traced ? tile_use(a0.variant, 1) : kTileStep, a0.n, a0.R))
+    return launch_tiles(plain_tile_energy_kernel, a0, a0.x, false, st);
   PlainEnergy a = a0;
   a.stages = plain_stages(a.jp, a.rb);
   dim3 grid((a.n + kRows - 1) / kRows, (a.R + a.rb - 1) / a.rb);
@@ -1333,7 +1363,7 @@ cudaError_t launch_nmfa_sweep(const NmfaSweep &a0, cudaStream_t st) {
   plain_attrs();
   if (a0.rb < 1 || a0.rb > kMaxRB || a0.jp % 4 || a0.xp % 4 || a0.jp > a0.xp || a0.jp < 4)
     return cudaErrorInvalidValue;
-  return use_tiles(a0.n, a0.R) ? launch_tiles(nmfa_tile_kernel, a0, a0.s_in, a0.overlap != 0, st)
+  return use_tiles(kTileStep, a0.n, a0.R) ? launch_tiles(nmfa_tile_kernel, a0, a0.s_in, a0.overlap != 0, st)
                                : launch_row_warps(nmfa_sweep_kernel<false>, nmfa_sweep_kernel<true>, a0, st);
 }
 
