@@ -267,6 +267,12 @@ bool makes_init(const sb_plan *pl) {
 // The plain FP32 steps of a solve run in one launch.
 bool one_launch(const sb_plan *pl) { return pl->planes || pl->cluster || pl->dwords; }
 
+// The exchange words, aligned (dwords is what is freed).
+unsigned long long *words_of(const sb_plan *pl) {
+  return reinterpret_cast<unsigned long long *>(((uintptr_t)pl->dwords + sbk::kPersistAlign - 1) / sbk::kPersistAlign *
+                                                sbk::kPersistAlign);
+}
+
 bool needs_trace(const sb_params &p) { return p.trace || p.trace_all; }
 
 size_t energy_slots(const sb_params &p) { return needs_trace(p) ? (size_t)p.steps + 1 : 1; }
@@ -373,7 +379,7 @@ sb_status plan_create(sb_ctx *ctx, const sb_problem *p, const sb_params *prm, sb
     const int ctas = want && !pl->cluster ? sbk::plain_persist_ctas(pl->n, pl->R, pl->jp) : 0;
     if (ctas > 0) {
       pl->words_bytes = (size_t)2 * ctas * 128;  // at most one 128-byte line per CTA
-      PLAN_ALLOC(pl->dwords, pl->words_bytes);
+      PLAN_ALLOC(pl->dwords, pl->words_bytes + sbk::kPersistAlign);
     }
   }
 #undef PLAN_ALLOC
@@ -483,7 +489,7 @@ cudaError_t enqueue_loop(sb_plan *pl, cudaStream_t st, std::vector<cudaEvent_t> 
   if (pl->cluster || pl->dwords) {
     // plain FP32 SB in one launch (same fields and updates as the per-step kernel)
     if (p.steps > 0) {
-      cudaError_t e = pl->cluster ? cudaSuccess : cudaMemsetAsync(pl->dwords, 0, pl->words_bytes, st);
+      cudaError_t e = pl->cluster ? cudaSuccess : cudaMemsetAsync(words_of(pl), 0, pl->words_bytes, st);
       if (e != cudaSuccess) return e;
       sbk::PlainPersist a;
       memset(&a, 0, sizeof(a));
@@ -507,7 +513,7 @@ cudaError_t enqueue_loop(sb_plan *pl, cudaStream_t st, std::vector<cudaEvent_t> 
       a.kerr = p.kerr;
       a.m = p.mts_m;
       a.steps = p.steps;
-      a.words = pl->dwords;
+      a.words = words_of(pl);
       a.status = pl->dstatus;
       a.init = makes_init(pl) ? 1 : 0;
       a.seed = pl->seed;

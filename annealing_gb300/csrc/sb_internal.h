@@ -53,7 +53,8 @@ struct PlainStep {
 // [16 c, 16 c + 16) of J in registers (one row per warp; a lane holds the float4 groups g = lane +
 // 32 k, which is the per-step kernel's summation order) and replica r's x, y of those rows. A step
 // exchanges through words[parity][r][c]: dSB 32 bits per CTA (step tag << 16 | 16 sign bits), bSB / aSB / NMFA a
-// 128-byte line per CTA, sixteen words (step tag << 32 | bits of x or of the state s). Eligible
+// 128-byte line per CTA, sixteen words (step tag << 32 | bits of x or of the state s). dSB: words is aligned to
+// kPersistAlign bytes. Eligible
 // when jp <= kPersistMaxJp and G R CTAs (G = ceil(n / 16)) are co-resident.
 struct PlainPersist {
   int variant;                // 0 aSB, 1 bSB (x exchanged), 2 dSB (signs exchanged), 3 NMFA (states exchanged)
@@ -80,6 +81,7 @@ struct PlainPersist {
   uint64_t seed;
 };
 constexpr int kPersistRows = 16;
+constexpr size_t kPersistAlign = 1024;
 constexpr int kPersistMaxJp = 2048;
 // Number of CTAs (G R) of the persistent launch, or 0 when this shape does not qualify.
 int plain_persist_ctas(int n, int R, int jp);

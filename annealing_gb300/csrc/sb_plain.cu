@@ -859,9 +859,10 @@ __global__ void __launch_bounds__(kPersistThreads, 1) plain_persist_kernel(Plain
   constexpr int kLine = 16;                                       // words per line
   unsigned long long *wr = a.words + (size_t)r * G * kLine;      // parity 0 of replica r
   const size_t par = (size_t)a.R * G * kLine;                     // parity stride
-  // dSB: the replica's words side by side
-  const int gp = (G + 31) & ~31;
-  auto signs = [&](int t) { return reinterpret_cast<uint32_t *>(a.words) + ((size_t)(t & 1) * a.R + r) * gp; };
+  // dSB: the replica's words side by side, both parities in one aligned block (a.words is aligned to the largest, 1 KB):
+  // with a 4 KB boundary between the parities the two lie on different dies, and a step took 3.3 us in place of 1.4
+  const int gp = (G + 31) & ~31, half = gp <= 32 ? 32 : gp <= 64 ? 64 : 128;
+  auto signs = [&](int t) { return reinterpret_cast<uint32_t *>(a.words) + (size_t)r * 2 * half + (t & 1) * half; };
   // rows past n publish x = 0 (sign -1), as the per-step kernel reads padding spins
   auto publish = [&](int t) {  // x(t) or its signs, with tag t + 1
     const unsigned long long tag = (unsigned long long)(uint32_t)(t + 1) << 32;
