@@ -410,6 +410,11 @@ int run_chunks(int dt, int n) { return kp_for(dt, n) / (dt == kTcFp4 ? 256 : 128
 // 16.8. (E2M1 shapes beyond nine chunks take FP8.) BF16 couplings as 16 hi + lo in E4M3, resident up to 512 spins,
 // against the kernel on BF16 operands: (88, 599) 1.71 / 7.90, (300, 1000) 2.53 / 9.39, (1000, 300) 4.07 / 11.7,
 // (2000, 1024) 12.6 / 17.1, (4096, 290) 23.7 / 26.4, (8192, 64) 29.3 / 41.5, (16384, 32) 79.5 / 91.6.
+// Two items of a CTA stream the same J rows one after the other, where the other kernel's 128-replica unit reads them
+// once: with couplings that L2 does not hold beside the rest that costs more than the exchange saves. FP8 (7700, 256),
+// 61 MB, 30.2 / 30.8, (8000, 256), 65 MB, 32.2 / 31.4, (10240, 128), 105 MB, 45.9 / 37.7, (16384, 128) 91.6 / 61.0; 16 hi + lo
+// (6500, 256), 85 MB, 43.8 / 44.9, (6800, 256), 96 MB, 47.3 / 46.8, (8192, 256), 134 MB, 63.1 / 54.0, (16384, 128) 165 / 114.
+constexpr int64_t two_item_bytes(int dt) { return dt == kTcBf16 ? 90000000 : 63000000; }
 bool run_shape(int dt, int n, int R, int sms, int *nr, int *per_cta) {
   if (dt == kTcFp4 && run_chunks(dt, n) > kResChunks) return false;
   const int mt = (n + kBM - 1) / kBM, t32 = (R + 31) / 32, t64 = (R + 63) / 64;
@@ -418,7 +423,7 @@ bool run_shape(int dt, int n, int R, int sms, int *nr, int *per_cta) {
     *nr = 32;
   } else if (mt * t64 <= sms) {
     *nr = 64;
-  } else if (mt * ((t64 + 1) / 2) <= sms) {
+  } else if (mt * ((t64 + 1) / 2) <= sms && (int64_t)mt * kBM * run_chunks(dt, n) * kChunkBytes <= two_item_bytes(dt)) {
     *nr = 64;
     *per_cta = 2;
   } else {

@@ -89,7 +89,9 @@ def run_kernel_takes(dtype, n, R, sms):
     """Whether an untraced dSB solve runs in the multi-step kernel (run_shape in csrc/sb_tc.cu)."""
     if dtype not in ("fp4e2m1", "fp8e4m3", "bf16") or (dtype == "fp4e2m1" and n > 9 * 256):
         return False
-    return -(-n // 128) * (-(-R // 64) + 1 >> 1) <= sms
+    tiles, t64 = -(-n // 128), -(-R // 64)
+    operand_bytes = tiles * 128 * (-(-n // 128)) * 128 * (2 if dtype == "bf16" else 1)
+    return tiles * t64 <= sms or (tiles * (t64 + 1 >> 1) <= sms and operand_bytes <= (90e6 if dtype == "bf16" else 63e6))
 
 
 def tensor_rate(dtype):
