@@ -697,6 +697,20 @@ bool reserve(T *&p, size_t &cap, size_t count) {
 }
 }  // namespace
 
+// An instance needs a slot for each of its items. With more items than SMs a CTA takes two of them, which stream couplings
+// one after the other that a 128-replica tile of grouped_kernel reads once. Where that tile's items have an SM each and L2
+// does not hold the couplings beside the rest, the launch per step is faster: us per step, waves / 128-replica tiles,
+// E2M3 n = 9700 R = 192 (71 MB) 33.3 / 34.0, n = 10240 R = 80 (79 MB) 35.1 / 28.1, n = 12000 R = 128 (108 MB) 45.4 / 37.3,
+// n = 16384 69.7 / 50.8; FP8 n = 9700 R = 256 (95 MB) 33.4 / 35.9, n = 10240 R = 128 (105 MB) 40.4 / 33.6, n = 16384
+// 80.0 / 59.5; E2M1 n = 16384 R = 128 (134 MB) 30.5 / 37.5, n = 17500 R = 80 (154 MB) 40.8 / 37.5, n = 19400 52.7 / 45.5.
+bool Grouped::wave_takes(int n, int R, int nr, int op, int sms) {
+  const int64_t mt = (n + kBM - 1) / kBM, items = mt * ((R + nr - 1) / nr);
+  if (items > (int64_t)run_slots(nr) * sms) return false;
+  if (nr != 64 || R <= 64 || items <= sms || mt * ((R + 127) / 128) > sms) return true;
+  const int64_t spins = mt * kBM, bytes = op == kGopE2m1 ? spins * ((n + 255) / 256 * 128) : op == kGopE2m3 ? spins * spins / 4 * 3 : spins * spins;
+  return bytes <= (op == kGopE2m1 ? 145000000 : op == kGopE2m3 ? 75000000 : 100000000);
+}
+
 // Deals the resident instances into waves, largest first: as many as fit the CTAs' slots and kWaveBytes
 // of couplings (at least one instance). Like-sized instances share a wave, so its CTAs carry like work.
 sb_status Grouped::build_waves(std::string &err) {
@@ -713,7 +727,7 @@ sb_status Grouped::build_waves(std::string &err) {
     GHost &g = insts[i];
     const int mt = g.Np / kBM, rt = g.Rp / nr, kc = grouped_kchunks(g.Kp, g.op);
     const size_t words = (size_t)2 * 4 * mt * nr;  // of one replica tile
-    g.wave = (int64_t)mt * rt <= most;
+    g.wave = wave_takes(g.n, g.R, nr, g.op, sms);
     if (!g.wave) {
       for (int m = 0; m < mt; ++m)
         for (int r = 0; r < rt; ++r) rest.push_back(GItem{i, m * kBM, r * nr, kc});

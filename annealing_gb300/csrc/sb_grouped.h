@@ -104,6 +104,8 @@ class Grouped {
   cudaError_t run_steps(int tick0, int count, bool use_graph);
   // SB steps of instance g that one launch of run_steps(., count, .) advances
   static int steps_per_launch(const GHost &g, int count);
+  // Whether an instance's steps run in a wave for a replica tile of nr, on a device of `sms` SMs.
+  static bool wave_takes(int n, int R, int nr, int op, int sms);
   // whether some instance does not fit a wave (valid after sync_tables)
   bool has_rest() const { return n_rest > 0; }
   // The initial state of every resident instance, seeded with seed + its tag (after sync_tables).

@@ -64,11 +64,14 @@ struct Req {
   int best_r = 0, ok = 0;
 };
 
-int tile_for(int R) { return R <= 32 ? 32 : 64; }
+// Replica tile of a request; 128 where it takes a launch per step.
+int tile_for(int n, int R, int sms) {
+  return R <= 32 ? 32 : R <= 64 || sbk::Grouped::wave_takes(n, R, 64, kServeOperand, sms) ? 64 : 128;
+}
 }  // namespace
 
 struct Server {
-  int device = 0;
+  int device = 0, sms = 1;
   cudaStream_t st = nullptr;
   int64_t budget = 0, used = 0;
   int max_inflight = 64;
@@ -415,6 +418,7 @@ sb_status server_create(Server **out, int device, int64_t hbm_budget, int max_in
   s->budget = hbm_budget;
   s->max_inflight = max_inflight;
   cudaSetDevice(device);
+  cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, device);
   bool streams_ok = cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking) == cudaSuccess;
   for (int w = 0; w < Server::kPreparers; ++w)
     streams_ok = streams_ok && cudaStreamCreateWithFlags(&s->pst[w], cudaStreamNonBlocking) == cudaSuccess;
@@ -480,7 +484,7 @@ sb_status server_submit(Server *s, const sb_problem *p, const sb_params *prm, ui
   r->prm = *prm;
   r->submitted = Clock::now();
   const bool grouped = sbk::grouped_supports(p, prm) && prm->trace == 0 && prm->trace_all == 0;
-  r->nr = grouped ? tile_for(prm->replicas) : 0;
+  r->nr = grouped ? tile_for(p->n, prm->replicas, s->sms) : 0;
   r->bytes = grouped ? sbk::grouped_instance_bytes(p->n, prm->replicas, prm->steps, r->nr, kServeOperand)
                      : sb_plan_footprint(p, prm);
   std::lock_guard<std::mutex> lk(s->mu);

@@ -22,3 +22,27 @@ def test_single_instances(n, jmax):
     np.testing.assert_array_equal(out[0].final_y, out[1].final_y[:40])
     np.testing.assert_array_equal(out[0].replica_energies, out[1].replica_energies[:40])
     assert out[1].energy_check_ok
+
+
+@pytest.mark.parametrize("n,R,jmax,wave", [(9700, 100, 9, True), (10112, 100, 9, False), (10112, 100, 1, True),
+                                           (10112, 64, 9, True)])
+def test_batches_and_served(n, R, jmax, wave):
+    """E2M3 couplings of more than 75 MB with 65 to 128 replicas take a launch per step, the others a wave."""
+    prob = sb.Problem.random(n, 0.3, jmax, 0, seed=n)
+    prm = sb.Params.default(sb.DSB, steps=6, replicas=R, seed=1, field_mode=sb.FIELD_TC)
+    ctx = sb.Context(0)
+    batch = ctx.batch([prob], prm, want_state=True)
+    try:
+        a = batch.run(seed=1)[0]
+        b = ctx.solve(prob, prm, want_state=True)
+        c = ctx.poll(ctx.submit(prob, prm), n, prm, wait_ms=-1)
+    finally:
+        batch.close()
+        ctx.close()
+    assert a.steps_per_launch == (6 if wave else 1)
+    if jmax > 4:
+        assert c.steps_per_launch == a.steps_per_launch
+    np.testing.assert_array_equal(a.final_x, b.final_x)
+    for r in (a, c):
+        np.testing.assert_array_equal(r.replica_energies, b.replica_energies)
+        assert r.energy_check_ok

@@ -24,6 +24,7 @@ static std::atomic<int> recorded{0};  // the runtime's last error
 // ---- CUDA: device memory is host memory ----
 extern "C" {
 cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+cudaError_t cudaDeviceGetAttribute(int *v, cudaDeviceAttr, int) { *v = 1; return cudaSuccess; }
 cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cudaStream_t) { memcpy(d, s, n); return cudaSuccess; }
 cudaError_t cudaMemsetAsync(void *d, int v, size_t n, cudaStream_t) { memset(d, v, n); return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
@@ -49,6 +50,7 @@ namespace sbk {
 bool grouped_supports(const sb_problem *, const sb_params *) { return true; }
 int64_t grouped_instance_bytes(int, int, int, int, int) { return 1; }
 Grouped::~Grouped() {}
+bool Grouped::wave_takes(int, int, int, int, int) { return true; }
 int Grouped::steps_per_launch(const GHost &, int) { return 1; }
 sb_status Grouped::prepare(GHost &g, const sb_problem *p, const sb_params *prm, uint64_t, int tag, int, cudaStream_t, Staging &,
                            std::string &, int) {
