@@ -14,7 +14,8 @@ def _problem(n, jmax, seed):
 
 @pytest.mark.parametrize("profile", [0, 1])
 def test_batch(profile):
-    """Two operand types; 4096 replicas of 700 spins are more items than a wave holds."""
+    """Two operand types; 4096 replicas of 700 spins are more items than a wave holds, and the
+    tile that is timed as the faster one for that bucket may have no waves at all."""
     ctx = sb.Context(0)
     try:
         for ns, R, waves in (((300, 500, 200), 64, (True, True, True)), ((700, 200), 4096, (False, True))):
@@ -25,7 +26,11 @@ def test_batch(profile):
             buckets = len({r.field_dtype for r in res})
             assert buckets == (2 if 500 in ns else 1)
             for r, w in zip(res, waves):
-                assert r.energy_check_ok and r.steps_per_launch == (STEPS if w and not profile else 1)
+                assert r.energy_check_ok
+                if all(waves) or not w or profile:
+                    assert r.steps_per_launch == (STEPS if w and not profile else 1)
+                else:
+                    assert r.steps_per_launch in (1, STEPS)
                 if all(waves) and not profile:
                     assert r.kernel_launches < 10 * buckets  # states, a wave, signs, energies, results
                 else:
