@@ -713,6 +713,10 @@ bool Grouped::wave_takes(int n, int R, int nr, int op, int sms) {
 
 // Deals the resident instances into waves, largest first: as many as fit the CTAs' slots and kWaveBytes
 // of couplings (at least one instance). Like-sized instances share a wave, so its CTAs carry like work.
+// A wave is a table's clearing, a cooperative launch and, before the energies, the V buffers from x: 10 to 15 us beside a
+// launch per step, of whose steps each costs 2 to 5 us more (large instances 4 to 10). Device us of whole runs, launch per
+// step / wave: n = 128, R = 64, E2M1 2 steps 37 / 49, 4 steps 48 / 53, 6 steps 58 / 56; n = 2000, R = 64, E2M1 4 steps 58 / 66,
+// 6 steps 73 / 72; three of n = 4000, R = 32, E2M3 4 steps 83 / 76; n = 8000, R = 32, E2M3 3 steps 98 / 98, 4 steps 118 / 101.
 sb_status Grouped::build_waves(std::string &err) {
   waves.clear();
   const int sms = device_sms(), most = run_slots(nr) * sms;
@@ -723,12 +727,14 @@ sb_status Grouped::build_waves(std::string &err) {
   std::vector<GItem> rest;
   int64_t bytes = 0;
   size_t ll = 0;
+  wave_from = !by_size.empty() && insts[by_size[0]].n > 2048 ? 4 : 5;
   for (int i : by_size) {
     GHost &g = insts[i];
     const int mt = g.Np / kBM, rt = g.Rp / nr, kc = grouped_kchunks(g.Kp, g.op);
     const size_t words = (size_t)2 * 4 * mt * nr;  // of one replica tile
-    g.wave = wave_takes(g.n, g.R, nr, g.op, sms);
-    if (!g.wave) {
+    const bool takes = wave_takes(g.n, g.R, nr, g.op, sms);
+    g.wave_from = takes ? wave_from : 0;
+    if (!takes) {
       for (int m = 0; m < mt; ++m)
         for (int r = 0; r < rt; ++r) rest.push_back(GItem{i, m * kBM, r * nr, kc});
       continue;
@@ -831,11 +837,11 @@ cudaError_t Grouped::launch_items(const GItem *items_ptr, int count, int tick, i
   return cudaLaunchKernel(k, dim3(grid), dim3(kTcThreads), args, smem, st);
 }
 
-int Grouped::steps_per_launch(const GHost &g, int count) { return g.wave && count > 1 ? std::min(count, kWaveSteps) : 1; }
+int Grouped::steps_per_launch(const GHost &g, int count) { return g.wave_from > 0 && count >= g.wave_from ? std::min(count, kWaveSteps) : 1; }
 
 cudaError_t Grouped::run_steps(int tick0, int count, bool use_graph) {
   if (count <= 0) return cudaSuccess;
-  if (count > 1 && !waves.empty()) {
+  if (count >= wave_from && !waves.empty()) {
     for (const Wave &w : waves)
       if (cudaError_t e = run_wave(w, tick0, count); e != cudaSuccess) return e;
     for (int s = 0; s < count && n_rest > 0; ++s)
@@ -849,6 +855,7 @@ cudaError_t Grouped::run_steps(int tick0, int count, bool use_graph) {
     }
     return cudaSuccess;
   }
+  if (cudaError_t e = refresh_v(tick0); e != cudaSuccess) return e;  // before the capture: a graph holds steps alone
   if (!graph || graph_tick0 != tick0 || graph_count != count) {
     if (graph) cudaGraphExecDestroy(graph);
     graph = nullptr;

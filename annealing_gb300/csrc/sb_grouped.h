@@ -63,7 +63,7 @@ struct GHost {
   float *x = nullptr, *y = nullptr, *h = nullptr, *pumps = nullptr;
   double *energy = nullptr;
   size_t out = 0;  // offset of its results in results()
-  bool wave = false;            // its steps run in a wave (valid after sync_tables)
+  int wave_from = 0;            // runs of this many steps or more advance it in a wave, 0: none does (valid after sync_tables)
   GInst desc;
 };
 
@@ -98,9 +98,9 @@ class Grouped {
   void clear();
   // Re-uploads the instance / item tables after add / remove (synchronous).
   sb_status sync_tables(std::string &err);
-  // Steps ticks [tick0, tick0 + count) for every resident instance. Two steps or more run wave by wave,
-  // a wave's steps in one launch (sb_run.cuh); a single step, and instances with more items than
-  // a wave holds, take one launch per step (a CUDA graph of them when use_graph).
+  // Steps ticks [tick0, tick0 + count) for every resident instance. Runs of four or five steps and more go wave by
+  // wave, a wave's steps in one launch (sb_run.cuh); shorter ones, and instances that wave_takes refuses,
+  // take one launch per step (a CUDA graph of them when use_graph).
   cudaError_t run_steps(int tick0, int count, bool use_graph);
   // SB steps of instance g that one launch of run_steps(., count, .) advances
   static int steps_per_launch(const GHost &g, int count);
@@ -162,6 +162,7 @@ class Grouped {
   GItem *d_rest = nullptr;           // items of the instances that fit no wave
   unsigned long long *d_ll = nullptr;  // exchange words of one wave
   int n_run = 0, n_rest = 0;
+  int wave_from = 5;                   // steps from which on a run goes wave by wave
   size_t cap_run = 0, cap_rest = 0, cap_ll = 0;
   uint8_t *d_out = nullptr;            // results of the resident instances, packed
   size_t cap_out = 0, out_bytes = 0;
