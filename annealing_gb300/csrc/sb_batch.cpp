@@ -24,8 +24,8 @@
 #include "sb_internal.h"
 
 // One operand bucket of a batch: the instances whose couplings share an operand type (packed E2M1
-// when every coupling is an integer |J| <= 4, else packed E2M3), advanced by their own grouped
-// launch per step with their own autotuned replica tile and item order.
+// when every coupling is an integer |J| <= 4, else packed E2M3), advanced by their own waves or grouped
+// launches per step, with their own autotuned form where these are in question.
 struct sb_bucket {
   sbk::Grouped *g = nullptr;
   std::vector<int> members;  // batch index of each resident instance, in residence order
@@ -45,7 +45,7 @@ struct sb_batch {
 namespace {
 
 std::mutex g_tune_mu;
-std::map<std::string, std::pair<int, int>> g_tune_cache;
+std::map<std::string, sbk::Grouped::Form> g_tune_cache;
 
 // instance k of the batch starts from seed + k, whichever bucket holds it
 sb_status init_all(sb_bucket &bk, uint64_t seed, std::string &err) {
@@ -55,37 +55,37 @@ sb_status init_all(sb_bucket &bk, uint64_t seed, std::string &err) {
   return SB_ERR_CUDA;
 }
 
-// Instances too large for a wave take one launch per step: times a few steps of each (replica tile, item
-// order) candidate on the bucket itself and keeps the fastest; the choice is cached by (replica count, total work bucket, batch size bucket, operands).
+// A bucket whose instances all run in waves keeps its form: 64 replicas halve the couplings' L2 traffic of 32
+// (N = 4096, R = 64: 11.2 against 18.2 us per step) and leave two items per CTA where 128 leave one. Two kinds of bucket
+// time a few steps of each candidate on themselves and keep the fastest: those with instances too large for a wave,
+// and those with more than 64 replicas whose waves give a CTA two items that stream the couplings one after the other,
+// where 128-replica tiles read them once. us per step with 200 replicas, waves / launch per step: 8 of n = 5000 E2M3
+// 144 / 80, E2M1 80 / 60; 4 of n = 6000 E2M3 84 / 57; 3 of n = 8000 E2M3 83 / 69, E2M1 46 / 44; 5 of n = 2000..4000 E2M3
+// 25 / 28, E2M1 16 / 21; up to n = 2048 waves are the faster ones throughout (12 of n = 2000 E2M3 27 / 32).
+// The choice is cached by (replica count, total work bucket, batch size bucket, operands; where waves are in question also
+// the counts of instances and waves).
 sb_status autotune(sb_batch *b, sb_bucket &bk, std::string &err) {
   sbk::Grouped &g = *bk.g;
-  // a bucket whose instances all run in waves keeps its tile: 64 replicas halve the couplings' L2 traffic
-  // of 32 (N = 4096, R = 64: 11.2 against 18.2 us per step) and leave two items per CTA where 128 leave one
-  if (sb_status s = g.sync_tables(err); s != SB_OK || !g.has_rest()) return s;
+  if (sb_status s = g.sync_tables(err); s != SB_OK || !g.tunable()) return s;
   const std::string key = g.tune_key();
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = g_tune_cache.find(key);
-    if (it != g_tune_cache.end()) {
-      sb_status s = g.retile(it->second.first, err);
-      g.set_order(it->second.second);
-      return s;
-    }
+    if (it != g_tune_cache.end()) return g.reform(it->second, err);
   }
-  const auto cands = sbk::Grouped::candidates(b->prm.replicas);
-  std::pair<int, int> best = cands.front();
+  const auto cands = g.candidates(b->prm.replicas);
+  sbk::Grouped::Form best = cands.front();
   float best_ms = 1e30f;
   if (cands.size() > 1 && b->prm.steps >= 4) {
     cudaStream_t st = b->ctx->stream;
     for (const auto &c : cands) {
-      sb_status s = g.retile(c.first, err);
+      sb_status s = g.reform(c, err);
       if (s != SB_OK) return s;
-      g.set_order(c.second);
       if ((s = g.sync_tables(err)) != SB_OK) return s;
       if ((s = init_all(bk, b->prm.seed, err)) != SB_OK) return s;
-      if (g.run_steps(0, 1, false) != cudaSuccess) continue;
+      if (g.run_steps(0, 4, false) != cudaSuccess) continue;
       cudaEventRecord(b->ev0, st);
-      if (g.run_steps(1, std::min(b->prm.steps - 1, 16), false) != cudaSuccess) continue;
+      if (g.run_steps(0, std::min(b->prm.steps, 16), false) != cudaSuccess) continue;
       cudaEventRecord(b->ev1, st);
       if (cudaEventSynchronize(b->ev1) != cudaSuccess) continue;
       float ms = 0;
@@ -96,11 +96,11 @@ sb_status autotune(sb_batch *b, sb_bucket &bk, std::string &err) {
       }
     }
   }
-  sb_status s = g.retile(best.first, err);
-  g.set_order(best.second);
-  std::lock_guard<std::mutex> lk(g_tune_mu);
-  g_tune_cache[key] = best;
-  return s;
+  if (best_ms < 1e30f) {  // a choice that nothing timed is not one for the next bucket
+    std::lock_guard<std::mutex> lk(g_tune_mu);
+    g_tune_cache[key] = best;
+  }
+  return g.reform(best, err);
 }
 
 void destroy(sb_batch *b) {

@@ -727,12 +727,13 @@ sb_status Grouped::build_waves(std::string &err) {
   std::vector<GItem> rest;
   int64_t bytes = 0;
   size_t ll = 0;
+  two_rounds = false;
   wave_from = !by_size.empty() && insts[by_size[0]].n > 2048 ? 4 : 5;
   for (int i : by_size) {
     GHost &g = insts[i];
     const int mt = g.Np / kBM, rt = g.Rp / nr, kc = grouped_kchunks(g.Kp, g.op);
     const size_t words = (size_t)2 * 4 * mt * nr;  // of one replica tile
-    const bool takes = wave_takes(g.n, g.R, nr, g.op, sms);
+    const bool takes = waves_on && wave_takes(g.n, g.R, nr, g.op, sms);
     g.wave_from = takes ? wave_from : 0;
     if (!takes) {
       for (int m = 0; m < mt; ++m)
@@ -750,6 +751,7 @@ sb_status Grouped::build_waves(std::string &err) {
     w.count += mt * rt;
     w.ll += rt * words;
     w.res = w.res && w.count <= sms;
+    two_rounds = two_rounds || (nr == 64 && g.R > 64 && g.n > 2048 && w.count > sms);
     bytes += ab;
     ll = std::max(ll, w.ll);
   }
@@ -954,18 +956,31 @@ std::string Grouped::tune_key() const {
   int b = 0;
   while ((int64_t(1) << b) < chunks) ++b;
   return std::to_string(rmax) + ":" + std::to_string(b) + ":" + std::to_string(insts.size() > 64 ? 2 : insts.size() > 8 ? 1 : 0) +
-         (op == kGopE2m1 ? ":e2m1" : (op == kGopE2m3 ? ":e2m3" : ":e4m3"));
+         (op == kGopE2m1 ? ":e2m1" : (op == kGopE2m3 ? ":e2m3" : ":e4m3")) +
+         (two_rounds ? ":" + std::to_string(insts.size()) + ":" + std::to_string(waves.size()) : "");
 }
 
-std::vector<std::pair<int, int>> Grouped::candidates(int R) {
-  std::vector<std::pair<int, int>> c;
+std::vector<Grouped::Form> Grouped::candidates(int R) const {
+  std::vector<Form> c;
   std::vector<int> nrs;
   if (R <= 32) nrs = {32};
   else if (R <= 64) nrs = {64, 32};
   else nrs = {128, 64};
   for (int v : nrs)
-    for (int o : {0, 1}) c.push_back({v, o});
+    for (int o : {0, 1}) c.push_back({v, o, n_rest > 0});
+  if (!two_rounds) return c;
+  if (n_rest > 0)
+    for (int o : {0, 1}) c.push_back({64, o, false});
+  else
+    c.insert(c.begin(), Form{nr, order, true});
   return c;
+}
+
+sb_status Grouped::reform(const Form &f, std::string &err) {
+  if (f.order != order || f.waves != waves_on) dirty = true;
+  order = f.order;
+  waves_on = f.waves;
+  return retile(f.nr, err);
 }
 
 }  // namespace sbk

@@ -106,8 +106,6 @@ class Grouped {
   static int steps_per_launch(const GHost &g, int count);
   // Whether an instance's steps run in a wave for a replica tile of nr, on a device of `sms` SMs.
   static bool wave_takes(int n, int R, int nr, int op, int sms);
-  // whether some instance does not fit a wave (valid after sync_tables)
-  bool has_rest() const { return n_rest > 0; }
   // The initial state of every resident instance, seeded with seed + its tag (after sync_tables).
   cudaError_t init_states(uint64_t seed);
   // Energies of every resident instance's current spins (instances must be at step t = tick - t0).
@@ -123,14 +121,18 @@ class Grouped {
       if (insts[i].tag == tag) return (int)i;
     return -1;
   }
+  // What autotuning chooses from: a replica tile, an order of the items, and whether the instances that fit one
+  // take waves.
+  struct Form {
+    int nr, order;
+    bool waves;
+  };
+  // Whether timing may show another form than the one at hand to be the faster (after sync_tables), and the forms to time.
+  bool tunable() const { return n_rest > 0 || two_rounds; }
+  std::vector<Form> candidates(int R) const;
   std::string tune_key() const;
-  static std::vector<std::pair<int, int>> candidates(int R);
-  void set_order(int o) {
-    if (o != order) {
-      order = o;
-      dirty = true;
-    }
-  }
+  // Takes a form (the state must be re-initialised).
+  sb_status reform(const Form &f, std::string &err);
 
   cudaStream_t st;
   int nr, order;
@@ -153,6 +155,8 @@ class Grouped {
     size_t ll;         // 8-byte words of its sign exchange
     bool res;          // J rows resident in shared memory
   };
+  bool waves_on = true;
+  bool two_rounds = false;  // a wave of streamed couplings has more 64-replica items of more than 64 replicas than SMs
   sb_status build_waves(std::string &err);
   cudaError_t run_wave(const Wave &w, int tick0, int count);
   // V(tick) from x for every instance of a wave: the multi-step launches exchange signs of their own
