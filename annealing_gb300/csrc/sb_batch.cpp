@@ -62,12 +62,12 @@ sb_status init_all(sb_bucket &bk, uint64_t seed, std::string &err) {
 // where 128-replica tiles read them once. us per step with 200 replicas, waves / launch per step: 8 of n = 5000 E2M3
 // 144 / 80, E2M1 80 / 60; 4 of n = 6000 E2M3 84 / 57; 3 of n = 8000 E2M3 83 / 69, E2M1 46 / 44; 5 of n = 2000..4000 E2M3
 // 25 / 28, E2M1 16 / 21; up to n = 2048 waves are the faster ones throughout (12 of n = 2000 E2M3 27 / 32).
-// The choice is cached by (replica count, total work bucket, batch size bucket, operands; where waves are in question also
-// the counts of instances and waves).
+// The choice is cached by (replica count, total work bucket, batch size bucket, operands, fewer than 64 steps; where waves are in
+// question also the counts of instances and waves).
 sb_status autotune(sb_batch *b, sb_bucket &bk, std::string &err) {
   sbk::Grouped &g = *bk.g;
   if (sb_status s = g.sync_tables(err); s != SB_OK || !g.tunable()) return s;
-  const std::string key = g.tune_key();
+  const std::string key = g.tune_key() + (b->prm.steps < 64 ? ":short" : "");  // where a wave's launch counts
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = g_tune_cache.find(key);
@@ -76,20 +76,23 @@ sb_status autotune(sb_batch *b, sb_bucket &bk, std::string &err) {
   const auto cands = g.candidates(b->prm.replicas);
   sbk::Grouped::Form best = cands.front();
   float best_ms = 1e30f;
-  if (cands.size() > 1 && b->prm.steps >= 4) {
+  const int steps = b->prm.steps, timed = std::min(steps, g.has_rest() ? 16 : 8);
+  if (cands.size() > 1 && steps >= 4) {
     cudaStream_t st = b->ctx->stream;
     for (const auto &c : cands) {
       sb_status s = g.reform(c, err);
       if (s != SB_OK) return s;
       if ((s = g.sync_tables(err)) != SB_OK) return s;
       if ((s = init_all(bk, b->prm.seed, err)) != SB_OK) return s;
-      if (g.run_steps(0, 4, false) != cudaSuccess) continue;
+      if (g.run_steps(0, c.waves ? 4 : 1, false) != cudaSuccess) continue;
       cudaEventRecord(b->ev0, st);
-      if (g.run_steps(0, std::min(b->prm.steps, 16), false) != cudaSuccess) continue;
+      if (g.run_steps(0, timed, false) != cudaSuccess) continue;
       cudaEventRecord(b->ev1, st);
       if (cudaEventSynchronize(b->ev1) != cudaSuccess) continue;
       float ms = 0;
       cudaEventElapsedTime(&ms, b->ev0, b->ev1);
+      const float beside = 0.012f * g.wave_count();  // ms of a wave's launch and exchange words, once in a run
+      ms = (ms - beside) / timed * steps + beside;
       if (ms < best_ms) {
         best_ms = ms;
         best = c;

@@ -966,13 +966,11 @@ std::vector<Grouped::Form> Grouped::candidates(int R) const {
   if (R <= 32) nrs = {32};
   else if (R <= 64) nrs = {64, 32};
   else nrs = {128, 64};
+  if (n_rest == 0) return {{nr, order, true}, {128, 0, false}, {128, 1, false}};
   for (int v : nrs)
-    for (int o : {0, 1}) c.push_back({v, o, n_rest > 0});
-  if (!two_rounds) return c;
-  if (n_rest > 0)
+    for (int o : {0, 1}) c.push_back({v, o, true});
+  if (two_rounds)
     for (int o : {0, 1}) c.push_back({64, o, false});
-  else
-    c.insert(c.begin(), Form{nr, order, true});
   return c;
 }
 

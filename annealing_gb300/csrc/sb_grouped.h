@@ -121,6 +121,9 @@ class Grouped {
       if (insts[i].tag == tag) return (int)i;
     return -1;
   }
+  // whether some instance does not fit a wave (valid after sync_tables)
+  bool has_rest() const { return n_rest > 0; }
+  int wave_count() const { return (int)waves.size(); }
   // What autotuning chooses from: a replica tile, an order of the items, and whether the instances that fit one
   // take waves.
   struct Form {
