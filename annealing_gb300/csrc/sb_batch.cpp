@@ -60,8 +60,8 @@ sb_status init_all(sb_bucket &bk, uint64_t seed, std::string &err) {
 // time a few steps of each candidate on themselves and keep the fastest: those with instances too large for a wave,
 // and those with more than 64 replicas whose waves give a CTA two items that stream the couplings one after the other,
 // where 128-replica tiles read them once. us per step with 200 replicas, waves / launch per step: 8 of n = 5000 E2M3
-// 144 / 80, E2M1 80 / 60; 4 of n = 6000 E2M3 84 / 57; 3 of n = 8000 E2M3 83 / 69, E2M1 46 / 44; 5 of n = 2000..4000 E2M3
-// 25 / 28, E2M1 16 / 21; up to n = 2048 waves are the faster ones throughout (12 of n = 2000 E2M3 27 / 32).
+// 92 / 80, E2M1 53 / 60; 4 of n = 6000 E2M3 64 / 57, E2M1 37 / 40; 3 of n = 8000 E2M3 83 / 69, E2M1 46 / 45; 5 of
+// n = 2000..4000 E2M3 24 / 28, E2M1 16 / 21; up to n = 2048 waves are the faster ones throughout (12 of n = 2000 E2M3 27 / 33).
 // The choice is cached by (replica count, total work bucket, batch size bucket, operands, fewer than 64 steps; where waves are in
 // question also the counts of instances and waves).
 sb_status autotune(sb_batch *b, sb_bucket &bk, std::string &err) {

@@ -711,8 +711,12 @@ bool Grouped::wave_takes(int n, int R, int nr, int op, int sms) {
   return bytes <= (op == kGopE2m1 ? 145000000 : op == kGopE2m3 ? 75000000 : 100000000);
 }
 
-// Deals the resident instances into waves, largest first: as many as fit the CTAs' slots and kWaveBytes
-// of couplings (at least one instance). Like-sized instances share a wave, so its CTAs carry like work.
+// Deals the resident instances into waves, largest first: as many as fit the CTAs' slots and kWaveBytes of couplings.
+// Like-sized instances share a wave, so its CTAs carry like work. The replica tiles of an instance do not depend on one
+// another, so where that saves a wave, one that does not fit what is left of a wave goes on in the next. Dealt whole, an
+// instance of n = 5000, R = 200 makes a wave of 160 items, a second round of 8, where 7 of its tiles are 280 items. us per
+// step, whole / split: 8 of them E2M3 144 / 92, E2M1 80 / 53; 4 of n = 6000, R = 200 E2M3 84 / 64; 8 of n = 3000, R = 400
+// E2M3 93 / 61; 12 of n = 2000, R = 400 E2M3 54 / 43; but with as many waves 10 of n = 1000, R = 400 E2M3 12.0 / 12.6.
 // A wave is a table's clearing, a cooperative launch and, before the energies, the V buffers from x: 10 to 15 us beside a
 // launch per step, of whose steps each costs 2 to 5 us more (large instances 4 to 10). Device us of whole runs, launch per
 // step / wave: n = 128, R = 64, E2M1 2 steps 37 / 49, 4 steps 48 / 53, 6 steps 58 / 56; n = 2000, R = 64, E2M1 4 steps 58 / 66,
@@ -725,36 +729,51 @@ sb_status Grouped::build_waves(std::string &err) {
   std::stable_sort(by_size.begin(), by_size.end(), [&](int a, int b) { return insts[a].Kp > insts[b].Kp; });
   std::vector<RunItem> run;
   std::vector<GItem> rest;
-  int64_t bytes = 0;
   size_t ll = 0;
-  two_rounds = false;
   wave_from = !by_size.empty() && insts[by_size[0]].n > 2048 ? 4 : 5;
+  // one dealing, whole instances or (split) their replica tiles
+  auto deal = [&](bool split) {
+    waves.clear();
+    run.clear();
+    ll = 0;
+    two_rounds = false;
+    int64_t bytes = 0;
+    for (int i : by_size) {
+      GHost &g = insts[i];
+      if (g.wave_from == 0) continue;
+      const int mt = g.Np / kBM, rt = g.Rp / nr, kc = grouped_kchunks(g.Kp, g.op), unit = split ? 1 : rt;
+      const size_t words = (size_t)2 * 4 * mt * nr;  // of one replica tile
+      const int64_t ab = (int64_t)g.Np * g.kbytes;
+      g.waves = 0;
+      for (int r = 0; r < rt;) {
+        if (waves.empty() || waves.back().count + mt * unit > most || (waves.back().count > 0 && bytes + ab > kWaveBytes)) {
+          waves.push_back(Wave{(int)run.size(), 0, 0, kc <= kResChunks});
+          bytes = 0;
+        }
+        Wave &w = waves.back();
+        const int tiles = std::min((most - w.count) / mt, rt - r);
+        for (int m = 0; m < mt; ++m)
+          for (int t = 0; t < tiles; ++t) run.push_back(RunItem{i, m * kBM, (r + t) * nr, kc, mt, (uint32_t)(w.ll + t * words)});
+        r += tiles;
+        w.count += mt * tiles;
+        w.ll += tiles * words;
+        w.res = w.res && w.count <= sms;
+        two_rounds = two_rounds || (nr == 64 && g.R > 64 && g.n > 2048 && w.count > sms);
+        bytes += ab;
+        ++g.waves;
+        ll = std::max(ll, w.ll);
+      }
+    }
+    return waves.size();
+  };
   for (int i : by_size) {
     GHost &g = insts[i];
-    const int mt = g.Np / kBM, rt = g.Rp / nr, kc = grouped_kchunks(g.Kp, g.op);
-    const size_t words = (size_t)2 * 4 * mt * nr;  // of one replica tile
     const bool takes = waves_on && wave_takes(g.n, g.R, nr, g.op, sms);
     g.wave_from = takes ? wave_from : 0;
-    if (!takes) {
-      for (int m = 0; m < mt; ++m)
-        for (int r = 0; r < rt; ++r) rest.push_back(GItem{i, m * kBM, r * nr, kc});
-      continue;
-    }
-    const int64_t ab = (int64_t)g.Np * g.kbytes;
-    if (waves.empty() || waves.back().count + mt * rt > most || bytes + ab > kWaveBytes) {
-      waves.push_back(Wave{(int)run.size(), 0, 0, kc <= kResChunks});
-      bytes = 0;
-    }
-    Wave &w = waves.back();
-    for (int m = 0; m < mt; ++m)
-      for (int r = 0; r < rt; ++r) run.push_back(RunItem{i, m * kBM, r * nr, kc, mt, (uint32_t)(w.ll + r * words)});
-    w.count += mt * rt;
-    w.ll += rt * words;
-    w.res = w.res && w.count <= sms;
-    two_rounds = two_rounds || (nr == 64 && g.R > 64 && g.n > 2048 && w.count > sms);
-    bytes += ab;
-    ll = std::max(ll, w.ll);
+    for (int m = 0; m < g.Np && !takes; m += kBM)
+      for (int r = 0; r < g.Rp; r += nr) rest.push_back(GItem{i, m, r, grouped_kchunks(g.Kp, g.op)});
   }
+  if (const size_t tiles = deal(true); deal(false) > tiles) deal(true);
   n_run = (int)run.size();
   n_rest = (int)rest.size();
   if (!reserve(d_run, cap_run, run.size()) || !reserve(d_rest, cap_rest, rest.size()) || !reserve(d_ll, cap_ll, ll)) {

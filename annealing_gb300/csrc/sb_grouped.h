@@ -64,6 +64,7 @@ struct GHost {
   double *energy = nullptr;
   size_t out = 0;  // offset of its results in results()
   int wave_from = 0;            // runs of this many steps or more advance it in a wave, 0: none does (valid after sync_tables)
+  int waves = 1;                // waves that its tiles are in
   GInst desc;
 };
 

@@ -377,8 +377,9 @@ void Server::run() {
         stats.grouped_launches += kv.second->launches - before;
         for (Req *r : resident)
           if (r->nr == kv.first && nt > 0) {
-            const int per = sbk::Grouped::steps_per_launch(kv.second->insts[kv.second->find((int)r->ticket)], nt);
-            r->launches += (nt + per - 1) / per;
+            const sbk::GHost &g = kv.second->insts[kv.second->find((int)r->ticket)];
+            const int per = sbk::Grouped::steps_per_launch(g, nt);
+            r->launches += (int64_t)(nt + per - 1) / per * (per > 1 ? g.waves : 1);
             r->steps_per_launch = std::max(r->steps_per_launch, per);
           }
         if (e != cudaSuccess) {

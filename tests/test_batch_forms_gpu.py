@@ -51,3 +51,34 @@ def test_untimed_choice_is_not_kept():
         assert all(r.steps_per_launch == 1 and r.energy_check_ok for r in out)  # 80 us per step where waves take 144
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("sizes,R,jmax", [
+    ((1900,) * 7, 400, 9),          # 15 items a tile, 7 tiles an instance, 20 tiles a wave
+    ((1000, 1000, 990), 1300, 1),   # 21 tiles of 8 items, 38 tiles a wave: the second instance is in both
+])
+def test_instances_split_over_waves(sizes, R, jmax):
+    probs = [sb.Problem.random(n, 0.3, jmax, 0, seed=n + k) for k, n in enumerate(sizes)]
+    prm = sb.Params.default(sb.DSB, steps=20, replicas=R, seed=1, field_mode=sb.FIELD_TC)
+    ctx = sb.Context(0)
+    try:
+        batch = ctx.batch(probs, prm, want_state=True)
+        res = batch.run(seed=1)
+        batch.close()
+        assert all(r.steps_per_launch == 20 for r in res)
+        tickets = []
+        for k, prob in enumerate(probs):
+            prm.seed, prm.replicas = 1 + k, R
+            tickets.append(ctx.submit(prob, prm))
+        for k, (prob, ticket) in enumerate(zip(probs, tickets)):
+            prm.seed, prm.replicas = 1 + k, min(R, 600)
+            one = ctx.solve(prob, prm, want_state=True)
+            prm.replicas = R
+            served = ctx.poll(ticket, prob.n, prm, wait_ms=-1)
+            np.testing.assert_array_equal(res[k].final_x[:600], one.final_x)
+            np.testing.assert_array_equal(res[k].final_y[:600], one.final_y)
+            np.testing.assert_array_equal(res[k].replica_energies[:600], one.replica_energies)
+            np.testing.assert_array_equal(served.replica_energies, res[k].replica_energies)
+            assert res[k].energy_check_ok and served.energy_check_ok
+    finally:
+        ctx.close()

@@ -39,7 +39,9 @@ def test_batches_and_served(n, R, jmax, wave):
     finally:
         batch.close()
         ctx.close()
-    assert a.steps_per_launch == (6 if wave else 1)
+    assert a.steps_per_launch == 1 or wave
+    if (n, jmax) != (10112, 1):  # its 158 items are two rounds, and waves are taken there if a trial finds them faster
+        assert a.steps_per_launch == (6 if wave else 1)
     if jmax > 4:
         assert c.steps_per_launch == a.steps_per_launch
     np.testing.assert_array_equal(a.final_x, b.final_x)
