@@ -316,9 +316,11 @@ int64_t sb_plan_footprint(const sb_problem *p, const sb_params *params);
  * grouped tensor-core launches (dSB, integer |J| <= 16). Instances whose couplings are integers
  * |J| <= 4 run on packed E2M1 operands (half the bytes), the others on packed E2M3
  * (params->operand_dtype SB_OPERAND_FP8 / SB_OPERAND_FP6 / SB_OPERAND_FP4 forces one type). Each operand
- * bucket runs in waves of instances whose couplings share L2, all steps of a wave in one launch; an
- * instance with more work items than a wave holds takes one grouped launch per step, the replica tile
- * and work order then chosen by timing the candidates on the bucket itself (cached per shape).
+ * bucket runs in waves of instances whose couplings share L2, all steps of a wave in one launch. An
+ * instance that no wave takes (more work items than one holds, or more than 64 replicas of couplings
+ * beyond L2) and runs of up to four steps take one grouped launch per step. Where either form may be
+ * the faster, it is chosen with the replica tile and work order by timing a few steps of the
+ * candidates on the bucket itself when the batch is created (cached per shape).
  * params is shared; instance k uses seed
  * seed + k; results[k] is filled as sb_solve would fill it (arrays sized for instance k). The
  * problems must stay alive until sb_batch_destroy. */
